@@ -1085,13 +1085,12 @@ def main():
                  else "fallback 6.65 TB/s")
     phases = prof["phases"]
     dom = max(phases.items(), key=lambda kv: kv[1][0])
-    kernels = {"ldl_solve": "k_ldl_solve_warp<double, 1> (single-warp LDL solve + refinement)",
-               "ldl_solve2": "k_ldl_solve_warp<double, 2> (single-warp LDL solve of the "
+    kernels = {"ldl_solve": "k_sl_solve<double, 1> (block-per-instance LDL solve + refinement)",
+               "ldl_solve2": "k_sl_solve<double, 2> (block-per-instance LDL solve of the "
                              "constant and affine right-hand sides + refinement)",
-               "ldl_factor": "k_ldl_factor_stream (streamed LDL factorisation, 4 warps per "
-                             "instance)"}
-    summaries = {"ldl_solve": "ldl_solve_mpc4096.md", "ldl_solve2": "ldl_solve2_mpc4096.md",
-                 "ldl_factor": "ldl_factor_stream_mpc4096.md"}
+               "ldl_factor": "k_sl_factor<double, double> (block-per-instance LDL "
+                             "factorisation)"}
+    summaries = {}  # profiles/ summaries of these kernels' DRAM traffic
 
     def roofline(name):
         ms, calls = phases[name]

@@ -29,6 +29,7 @@
 #include "equilibrate.cuh"
 #include "sn_exec.cuh"
 #include "setup.hpp"
+#include "sliced.hpp"
 
 namespace clgpu {
 
@@ -1011,17 +1012,17 @@ extern "C" int clgpu_default_settings(clgpu_settings *s) {
 // Builds every device structure of a batch from prepared instances.
 // Runs f(i) for i in [0, n) on nth host threads (blocks of 16 indices).
 template <class F>
-static void par_for(int n, int nth, F f) {
-  if (nth <= 1 || n < 64) {
+static void par_for(int n, int nth, F f, int grain = 16) {
+  if (nth <= 1 || n < 4 * grain) {
     for (int i = 0; i < n; ++i) f(i);
     return;
   }
   std::atomic<int> next{0};
   std::vector<std::thread> th;
-  for (int t = 0; t < nth; ++t)
+  for (int t = 0; t < std::min(nth, n / grain); ++t)
     th.emplace_back([&]() {
-      for (int i0; (i0 = next.fetch_add(16)) < n;)
-        for (int i = i0; i < std::min(n, i0 + 16); ++i) f(i);
+      for (int i0; (i0 = next.fetch_add(grain)) < n;)
+        for (int i = i0; i < std::min(n, i0 + grain); ++i) f(i);
     });
   for (auto &t : th) t.join();
 }
@@ -1037,236 +1038,33 @@ static std::vector<long long> prefix(const std::vector<T> &counts) {
 // Concatenates the prepared instances into the batch layout and uploads it.
 // Every per-instance copy runs on nth host threads: offsets first (prefix
 // sums over instances), then each instance fills its own disjoint slices.
-// First-fit-decreasing packing of instances into blocks of `slots` warps:
-// items in decreasing order of need (stable), each placed in the first block
-// with a free slot and room for it; a block's needs sum to at most cap.
-// pinst / poff receive per slot the instance (-1: idle) and its byte offset in
-// the block's shared memory.  Returns the number of blocks.
-template <typename Need>
-static int ffd_pack(std::vector<int> items, Need need, long long cap, int slots,
-                    std::vector<int> &pinst, std::vector<int> &poff) {
-  std::stable_sort(items.begin(), items.end(), [&](int a, int b) { return need(a) > need(b); });
-  std::vector<long long> used;
-  std::vector<int> cnt;
-  pinst.clear();
-  poff.clear();
-  size_t first_open = 0;
-  for (int i : items) {
-    const long long s_i = need(i);
-    size_t b = first_open;
-    while (b < used.size() && (cnt[b] == slots || used[b] + s_i > cap)) ++b;
-    if (b == used.size()) {
-      used.push_back(0);
-      cnt.push_back(0);
-      for (int w = 0; w < slots; ++w) {
-        pinst.push_back(-1);
-        poff.push_back(0);
-      }
-    }
-    pinst[(size_t)slots * b + cnt[b]] = i;
-    poff[(size_t)slots * b + cnt[b]] = (int)used[b];
-    used[b] += s_i;
-    ++cnt[b];
-    while (first_open < used.size() &&
-           (cnt[first_open] == slots || used[first_open] + need(items.back()) > cap))
-      ++first_open;
-  }
-  return (int)used.size();
-}
-
-// KKT position of every L entry (i, j), i > j, in the instance's permuted
-// full CSR (rows sorted, pattern symmetric), offset by kb; -1 when K has no
-// such entry.  Walking the rows r in order meets the entries (c, r) of each
-// row c in increasing r, so tpos[t] (the position of entry t's transpose) is
-// one pass with a cursor per row; row j scattered into a stamped map then
-// gives (j, i), and tpos its transpose (i, j).  Linear in nnz(K) + nnz(L).
-struct FactorOpScratch {
-  std::vector<int4> lev;
-  std::vector<int> nodes, cnt, segs, rowpos, rowstamp, tpos, cur;
-  std::vector<int> wch[kFactorWarps];
-  int stamp = 0;
-  void fit(int n, int nk) {
-    if ((int)rowpos.size() < n) {
-      rowpos.resize(n);
-      rowstamp.assign(n, 0);
-      cur.resize(n);
-      stamp = 0;
-    }
-    if ((int)tpos.size() < nk) tpos.resize(nk);
-  }
-};
-
-static void l_kkt_positions(const Prepared &p, long long kb, int *Lkpos, FactorOpScratch &sc) {
-  const int Ni = p.N;
-  sc.fit(Ni, (int)p.Kj.size());
-  int *rowpos = sc.rowpos.data(), *rowstamp = sc.rowstamp.data();
-  int *tpos = sc.tpos.data(), *cur = sc.cur.data();
-  for (int r = 0; r < Ni; ++r) cur[r] = p.Kp[r];
-  for (int r = 0; r < Ni; ++r)
-    for (int t = p.Kp[r]; t < p.Kp[r + 1]; ++t) tpos[t] = cur[p.Kj[t]]++;
-  for (int j = 0; j < Ni; ++j) {
-    const int st = ++sc.stamp;
-    for (int t = p.Kp[j]; t < p.Kp[j + 1]; ++t) {
-      rowpos[p.Kj[t]] = t;
-      rowstamp[p.Kj[t]] = st;
-    }
-    for (int q = p.Lp[j]; q < p.Lp[j + 1]; ++q) {
-      const int r = p.Li[q];
-      Lkpos[q] = rowstamp[r] == st ? (int)(kb + tpos[rowpos[r]]) : -1;
-    }
-  }
-}
-
-// Number of ops of the instance's streamed factorisation: one per (j, k)
-// pair of its row structure and per entry of L(:,k) below row j, and one
-// pivot per column.
-static long long factor_op_count(const Prepared &p) {
-  long long t = p.N;
-  for (size_t r = 0; r < p.Rk.size(); ++r) t += p.Lp[p.Rk[r] + 1] - p.Rpos[r];
-  return t;
-}
-
-// The streamed factorisation's ops of one instance, written to op (exactly
-// factor_op_count(p) of them), level by level:
-//  - the level's updates grouped by target (a segment per target), targets
-//    increasing: first the diagonal targets j (update d_j -= U(j,k)^2 / d_k,
-//    {j, Ni + pjk, Ni + pjk, k}), then the column targets Ni + q (update
-//    L(i,j) -= L(i,k) U(j,k), {Ni + q, Ni + pp, Ni + pjk, k}); a segment keeps
-//    its ops in generation order (the pairs (j, k) in row-structure order);
-//  - split into kFactorWarps parts of about equal length at segment starts,
-//    each op's .w or'd with min(position in segment, kPosMax) << 16 and the
-//    last-of-segment bit, each part cut into chunk words;
-//  - then the level's pivots (t = j, a = sign + 1) in kFactorWarps contiguous
-//    parts.
-// Each op is packed into 8 bytes (fop_pack).
-// The column ranges of L follow the node order, so sorting the level's nodes
-// and bucketing each column by q (counting sort) lists the groups in target
-// order without a comparison sort.  Returns false when the structure of
-// L(:,k) below j is not inside L(:,j) (not reached for a valid symbolic
-// factorisation) or a part's chunk count leaves its 16-bit field.
-static bool build_factor_ops(const Prepared &p, uint2 *op, int *flcnt, std::vector<int> &chk,
-                             std::array<int, kFactorWarps + 1> &woff, FactorOpScratch &sc) {
-  constexpr int W = kFactorWarps;
-  const int Ni = p.N;
-  const int nl = (int)p.lvl_ptr.size() - 1;
-  const int *lp = p.lvl_ptr.data();
-  sc.fit(Ni, 0);
-  int *rowpos = sc.rowpos.data(), *rowstamp = sc.rowstamp.data();
-  auto &lev = sc.lev;
-  auto &nodes = sc.nodes;
-  auto &cnt = sc.cnt;
-  auto &segs = sc.segs;
-  for (int w = 0; w < W; ++w) sc.wch[w].clear();
-  long long nops = 0;
-  bool bad = false;
-  auto put_chunks = [&](int w, long long c0, long long c1, bool pivot) {
-    int n = 0;
-    for (long long c = c0; c < c1; c += kChunk, ++n) {
-      const int cn = (int)std::min<long long>(kChunk, c1 - c);
-      const int steps =
-          pivot ? 0 : chunk_scan_steps<2>(cn, [&](int e) { return fop_pos(op[c + e]); });
-      sc.wch[w].push_back((int)(c | ((long long)steps << kStepShift) |
-                                ((long long)(cn - 1) << kCntShift) |
-                                (pivot ? (long long)1 << 31 : 0LL)));
-    }
-    return n;
+// Launch groups of one kind: instances (sorted by decreasing need of shared
+// memory) that fit 4, 2 or 1 blocks per SM; a group's launches are sized for
+// its largest member.  Finer groups lose: groups run one after the other, and
+// at 4096 MPC instances two more of them took the two-side solves from 10.5 to
+// 14.0 ms.
+static SlGroups sl_groups(const std::vector<int> &items, const std::vector<long long> &need,
+                          const std::vector<long long> &need2) {
+  SlGroups g{};
+  static constexpr long long cap[3] = {227 * 1024, 113 * 1024, 56 * 1024};
+  auto band = [&](int i) {
+    int c = 0;
+    while (c < 2 && std::max(need[i], need2[i]) <= cap[c + 1]) ++c;
+    return c;
   };
-  for (int l = 0; l < nl && !bad; ++l) {
-    nodes.assign(p.lvl_nodes.begin() + lp[l], p.lvl_nodes.begin() + lp[l + 1]);
-    std::sort(nodes.begin(), nodes.end());
-    size_t nlev = 0;
-    for (int j : nodes)
-      for (int r = p.Rp[j]; r < p.Rp[j + 1]; ++r) nlev += p.Lp[p.Rk[r] + 1] - p.Rpos[r];
-    if (lev.size() < nlev) lev.resize(nlev);
-    segs.clear();
-    int f = 0;
-    for (int j : nodes) {
-      if (p.Rp[j + 1] > p.Rp[j]) segs.push_back(f);
-      for (int r = p.Rp[j]; r < p.Rp[j + 1]; ++r) {
-        const int pjk = p.Rpos[r];
-        lev[f++] = make_int4(j, Ni + pjk, Ni + pjk, p.Rk[r]);
-      }
+  for (size_t t = 0; t < items.size();) {
+    size_t u = t;
+    SlGroup gr{(int)t, 0, 0, 0};
+    while (u < items.size() && band(items[u]) == band(items[t])) {
+      gr.smem = std::max(gr.smem, (int)need[items[u]]);
+      gr.smem2 = std::max(gr.smem2, (int)need2[items[u]]);
+      ++u;
     }
-    for (int j : nodes) {
-      if (p.Rp[j + 1] == p.Rp[j]) continue;
-      const int q0 = p.Lp[j], qe = p.Lp[j + 1], len = qe - q0;
-      if ((int)cnt.size() < len + 1) cnt.resize(len + 1);
-      std::fill(cnt.begin(), cnt.begin() + len + 1, 0);
-      const int st = ++sc.stamp;
-      for (int q = q0; q < qe; ++q) {
-        rowpos[p.Li[q]] = q - q0;
-        rowstamp[p.Li[q]] = st;
-      }
-      for (int r = p.Rp[j]; r < p.Rp[j + 1] && !bad; ++r) {
-        const int k = p.Rk[r];
-        for (int pp = p.Rpos[r] + 1; pp < p.Lp[k + 1]; ++pp) {
-          const int row = p.Li[pp];
-          if (rowstamp[row] != st) {
-            bad = true;
-            break;
-          }
-          cnt[rowpos[row] + 1]++;
-        }
-      }
-      if (bad) break;
-      for (int a = 0; a < len; ++a) {
-        if (cnt[a + 1]) segs.push_back(f + cnt[a]);
-        cnt[a + 1] += cnt[a];
-      }
-      for (int r = p.Rp[j]; r < p.Rp[j + 1]; ++r) {
-        const int k = p.Rk[r], pjk = p.Rpos[r];
-        for (int pp = pjk + 1; pp < p.Lp[k + 1]; ++pp) {
-          const int a = rowpos[p.Li[pp]];
-          lev[f + cnt[a]++] = make_int4(Ni + q0 + a, Ni + pp, Ni + pjk, k);
-        }
-      }
-      f += cnt[len - 1];  // bucket ends after placement
-    }
-    if (bad) break;
-    const int nseg = (int)segs.size();
-    segs.push_back(f);
-    int sb[W + 1];
-    sb[0] = 0;
-    sb[W] = nseg;
-    for (int w = 1; w < W; ++w) {
-      const int ideal = (int)((size_t)f * w / W);
-      const int g = (int)(std::lower_bound(segs.begin(), segs.end(), ideal) - segs.begin());
-      sb[w] = std::min(nseg, std::max(sb[w - 1], g));
-    }
-    int nop[W], npv[W];
-    for (int w = 0; w < W; ++w) {
-      const long long start = nops;
-      for (int g = sb[w]; g < sb[w + 1]; ++g) {
-        const int s0 = segs[g], s1 = segs[g + 1];
-        for (int t = s0; t < s1; ++t) {
-          const int4 o4 = lev[t];
-          op[nops++] = fop_pack(o4.x, o4.y, o4.z, o4.w, std::min(t - s0, kPosMax),
-                                t == s1 - 1 ? 1 : 0);
-        }
-      }
-      nop[w] = put_chunks(w, start, nops, false);
-    }
-    const int np = lp[l + 1] - lp[l];
-    for (int w = 0; w < W; ++w) {
-      const long long start = nops;
-      for (int t = lp[l] + np * w / W; t < lp[l] + np * (w + 1) / W; ++t) {
-        const int j = p.lvl_nodes[t];
-        op[nops++] = fop_pack(j, (int)p.Dsign[j] + 1, 0, 0, 0, 0);
-      }
-      npv[w] = put_chunks(w, start, nops, true);
-    }
-    for (int w = 0; w < W; ++w) {
-      if (nop[w] > 0xffff || npv[w] > 0xffff) bad = true;
-      flcnt[(size_t)l * W + w] = nop[w] | (npv[w] << 16);
-    }
+    gr.count = (int)(u - t);
+    g.g[g.n++] = gr;
+    t = u;
   }
-  chk.clear();
-  woff[0] = 0;
-  for (int w = 0; w < W; ++w) {
-    chk.insert(chk.end(), sc.wch[w].begin(), sc.wch[w].end());
-    woff[w + 1] = (int)chk.size();
-  }
-  return !bad;
+  return g;
 }
 
 static int build_batch(clgpu_solver *h, std::vector<Prepared> &prep, int nth) {
@@ -1526,14 +1324,34 @@ static int build_batch(clgpu_solver *h, std::vector<Prepared> &prep, int nth) {
   // ---------------- KKT arrays (concatenate with global positions)
   std::vector<int> N(B), voff(B + 1, 0), poff(B, 0), nlev(B);
   std::vector<long long> kcnt(B), lcnt(B), lvcnt(B);
+  // kernel class: one block with everything in shared memory (1) when the
+  // factor fits it, else the block kernels with global scratch (2), or the
+  // supernodal path (3)
+  std::vector<int> cls(B);
+  std::vector<SlicedPlan> plan(B);
+  par_for(B, nth, [&](int i) {
+    cls[i] = prep[i].supernodal ? 3 : (sl_fits(prep[i]) ? 1 : 2);
+    if (cls[i] == 1 && !sl_build(prep[i], h->mixed ? 4 : 2, plan[i])) {
+      cls[i] = 2;
+      plan[i] = SlicedPlan();
+    }
+  }, B < 256 ? 2 : 16);
+  mark("sliced layouts");
+  bool has_large = false;
   for (int i = 0; i < B; ++i) {
     N[i] = prep[i].N;
     voff[i + 1] = voff[i] + N[i];
     poff[i] = voff[i] + i;
-    kcnt[i] = (long long)prep[i].Kj.size();
-    lcnt[i] = (long long)prep[i].Li.size();
-    lvcnt[i] = (long long)prep[i].lvl_ptr.size();
+    // a class-1 instance stores K in slices (padding included) and has no
+    // scalar factor structures on the device
+    // (the others are padded so that every class-1 page stays 16-byte aligned)
+    kcnt[i] = cls[i] == 1 ? (long long)plan[i].kdst.size()
+                          : ((long long)prep[i].Kj.size() + 3) & ~3LL;
+    lcnt[i] = cls[i] == 1 ? 0 : (long long)prep[i].Li.size();
+    lvcnt[i] = cls[i] == 1 ? 0 : (long long)prep[i].lvl_ptr.size();
     nlev[i] = (int)prep[i].lvl_ptr.size() - 1;
+    has_large |= cls[i] == 2;
+    h->any_sn |= cls[i] == 3;
   }
   const auto kof = prefix(kcnt), lof = prefix(lcnt), lvof = prefix(lvcnt);
   const long long knz = kof[B], lnz = lof[B];
@@ -1541,34 +1359,28 @@ static int build_batch(clgpu_solver *h, std::vector<Prepared> &prep, int nth) {
   std::vector<int> lvl_off(B);
   for (int i = 0; i < B; ++i) lvl_off[i] = (int)lvof[i];
   const int VT = voff[B], PT = voff[B] + B;
-  hvec<int> Kp(PT), Kj((size_t)knz), Kdiag(VT), Lp(PT), Li((size_t)lnz), Rp(PT), Rk((size_t)lnz),
-      Rpos((size_t)lnz), gsrc(VT), lvl_ptr(lvof[B]), lvl_nodes(VT);
+  // CSR structures only where some instance reads them
+  const bool csr = has_large || h->any_sn;
+  hvec<int> Kp(csr ? PT : 0), Kj(csr ? (size_t)knz : 0), Kdiag(csr ? VT : 0),
+      Lp(csr ? PT : 0), Li((size_t)lnz), Rp(csr ? PT : 0), Rk((size_t)lnz), Rpos((size_t)lnz),
+      gsrc(VT), lvl_ptr(lvof[B]), lvl_nodes(csr ? VT : 0);
   hvec<double> Kx((size_t)knz);
-  hvec<signed char> Dsign(VT);
-  const int tsize = 8;  // work vectors are FP64 in both precision forms
-  int max_small = 0;
-  bool has_small = false, has_large = false;
-  // kernel class: single warp when the work vector fits the shared-memory
-  // budget and the streams fit the chunk-word offsets
-  std::vector<int> cls(B);
-  for (int i = 0; i < B; ++i) {
-    const bool fits = (long long)N[i] * tsize <= 48 * 1024 &&
-                      (long long)prep[i].Li.size() <= (long long)kStartMask &&
-                      (long long)prep[i].Kj.size() <= (long long)kStartMask;
-    cls[i] = prep[i].supernodal ? 3 : (fits ? 1 : 2);
-    if (cls[i] == 3) {
-      h->any_sn = true;
-    } else if (fits) {
-      has_small = true;
-      max_small = std::max(max_small, N[i]);
-    } else {
-      has_large = true;
-    }
-  }
+  hvec<signed char> Dsign(csr ? VT : 0);
   par_for(B, nth, [&](int i) {
     auto &p = prep[i];
     const int n = p.n, m = p.m;
     const long long kb = kof[i], lb = lof[i];
+    if (cls[i] == 1) {
+      const SlicedPlan &sp = plan[i];
+      std::fill(Kx.begin() + kb, Kx.begin() + kb + kcnt[i], 0.0);
+      for (size_t k = 0; k < p.Kx.size(); ++k) Kx[kb + sp.kslot[k]] = p.Kx[k];
+      for (int r = 0; r < N[i]; ++r) {
+        const int o = p.perm[r];
+        gsrc[voff[i] + r] =
+            o < n ? xoff[i] + o : (o < n + m ? -grow[i][o - n] - 2 : -1);
+      }
+      return;
+    }
     for (int r = 0; r <= N[i]; ++r) {
       Kp[poff[i] + r] = (int)(kb + p.Kp[r]);
       Lp[poff[i] + r] = (int)(lb + p.Lp[r]);
@@ -1576,6 +1388,7 @@ static int build_batch(clgpu_solver *h, std::vector<Prepared> &prep, int nth) {
     }
     std::copy(p.Kj.begin(), p.Kj.end(), Kj.begin() + kb);
     std::copy(p.Kx.begin(), p.Kx.end(), Kx.begin() + kb);
+    std::fill(Kx.begin() + kb + p.Kx.size(), Kx.begin() + kb + kcnt[i], 0.0);
     std::copy(p.Li.begin(), p.Li.end(), Li.begin() + lb);
     std::copy(p.Rk.begin(), p.Rk.end(), Rk.begin() + lb);
     for (size_t k = 0; k < p.Rpos.size(); ++k) Rpos[lb + k] = (int)(lb + p.Rpos[k]);
@@ -1618,8 +1431,9 @@ static int build_batch(clgpu_solver *h, std::vector<Prepared> &prep, int nth) {
       pow_pos(o_pow[B]), psdo(opsd[B]), psd_pos(2 * o_pse[B]);
   par_for(B, nth, [&](int i) {
     auto &p = prep[i];
-    const int kb = Kp[poff[i]];
-    auto addk = [&](int v) { return v < 0 ? -1 : v + kb; };
+    const int kb = (int)kof[i];
+    const int *ks = cls[i] == 1 ? plan[i].kslot.data() : nullptr;
+    auto addk = [&](int v) { return v < 0 ? -1 : (ks ? ks[v] : v) + kb; };
     for (long long t = 0; t < c_nn[i]; ++t) nn_pos[o_nn[i] + t] = addk(p.nn_pos[t]);
     long long sc_g = osoc[i], de = o_sde[i];
     size_t sc = 0;
@@ -1675,17 +1489,19 @@ static int build_batch(clgpu_solver *h, std::vector<Prepared> &prep, int nth) {
     par_for(B, nth, [&](int i) {
       const auto &p = prep[i];
       const int pb = (int)poffs[i], kb = (int)kof[i];
+      const int *ks = cls[i] == 1 ? plan[i].kslot.data() : nullptr;
       auto g = [](int v, int base) { return v < 0 ? -1 : v + base; };
+      auto gk = [&](int v) { return v < 0 ? -1 : (ks ? ks[v] : v) + kb; };
       for (long long t = 0; t < pu[i]; ++t) {
         const int *m4 = p.pmap.data() + 4 * t;
-        pmap[opu[i] + t] = make_int4(g(m4[0], pb), g(m4[1], pb), g(m4[2], kb), g(m4[3], kb));
+        pmap[opu[i] + t] = make_int4(g(m4[0], pb), g(m4[1], pb), gk(m4[2]), gk(m4[3]));
         const int r = p.pxy[2 * t], c = p.pxy[2 * t + 1];
         pxy[opu[i] + t] = r < 0 ? make_int2(-1, -1) : make_int2(xoff[i] + r, xoff[i] + c);
       }
       for (int j = 0; j < p.n; ++j)
         for (int k = p.A.p[j]; k < p.A.p[j + 1]; ++k) {
           const long long t = aoffs[i] + k;
-          amap[t] = make_int4((int)t, acsr[t], g(p.amapk[2 * k], kb), g(p.amapk[2 * k + 1], kb));
+          amap[t] = make_int4((int)t, acsr[t], gk(p.amapk[2 * k]), gk(p.amapk[2 * k + 1]));
           axy[t] = make_int2(Atj[t], xoff[i] + j);
         }
     });
@@ -1738,12 +1554,12 @@ static int build_batch(clgpu_solver *h, std::vector<Prepared> &prep, int nth) {
   kk.lvl_ptr = A.upload(lvl_ptr);
   kk.lvl_nodes = A.upload(lvl_nodes);
   mark("kkt upload");
-  // ---------------- substitution schedules (block instances) and streams
-  // (single-warp instances)
+  // ---------------- substitution schedules (block instances)
   kk.fsched = kk.bsched = nullptr;
   if (has_large) {
     std::vector<int4> fsched(VT), bsched(VT);
     par_for(B, nth, [&](int i) {
+      if (cls[i] != 2) return;
       const int *lp = lvl_ptr.data() + lvl_off[i];
       const int *nodes = lvl_nodes.data() + voff[i];
       for (int l = 0; l < nlev[i]; ++l)
@@ -1757,208 +1573,115 @@ static int build_batch(clgpu_solver *h, std::vector<Prepared> &prep, int nth) {
     kk.fsched = A.upload(fsched);
     kk.bsched = A.upload(bsched);
   }
-  hvec<int2> fent((size_t)lnz), bent((size_t)lnz), kent((size_t)knz);
-  hvec<int> fpos((size_t)lnz), bpos((size_t)lnz), flev(lvl_ptr.size()), blev(lvl_ptr.size());
-  std::vector<int> nchf(B, 0), nchb(B, 0), nchk(B, 0);
-  // encode segment positions: .x = seg | min(pos, kSPosMax) << 16 | last << kSLastBit
-  auto encode = [](int2 *e, long long n) {
-    long long q = 0;
-    while (q < n) {
-      long long r = q;
-      while (r + 1 < n && e[r + 1].x == e[q].x) ++r;
-      for (long long t = q; t <= r; ++t) {
-        const int pos = (int)std::min<long long>(t - q, kSPosMax);
-        e[t].x = (e[t].x & 0xffff) | (pos << 16) | ((t == r ? 1 : 0) << kSLastBit);
-      }
-      q = r + 1;
-    }
-  };
-  auto nchunks = [](const int *lev, int nl) {
-    int n = 0;
-    for (int l = 0; l < nl; ++l) n += (lev[l + 1] - lev[l] + kSChunk - 1) / kSChunk;
-    return n;
-  };
-  par_for(B, nth, [&](int i) {
-    const auto &p = prep[i];
-    const int nl = nlev[i];
-    const int *lp = p.lvl_ptr.data();
-    const long long base = Lp[poff[i]];
-    long long f = base;
-    for (int l = 0; l < nl; ++l) {
-      flev[lvl_off[i] + l] = (int)f;
-      for (int t = lp[l]; t < lp[l + 1]; ++t) {
-        const int node = p.lvl_nodes[t];
-        for (int r = p.Rp[node]; r < p.Rp[node + 1]; ++r) {
-          fent[f] = make_int2(node, p.Rk[r]);
-          fpos[f] = (int)(base + p.Rpos[r]);
-          ++f;
-        }
-      }
-    }
-    flev[lvl_off[i] + nl] = (int)f;
-    long long g = base;
-    for (int l = nl - 1, t2 = 0; l >= 0; --l, ++t2) {
-      blev[lvl_off[i] + t2] = (int)g;
-      for (int t = lp[l]; t < lp[l + 1]; ++t) {
-        const int node = p.lvl_nodes[t];
-        for (int q = p.Lp[node]; q < p.Lp[node + 1]; ++q) {
-          bent[g] = make_int2(node, p.Li[q]);
-          bpos[g] = (int)(base + q);
-          ++g;
-        }
-      }
-    }
-    blev[lvl_off[i] + nl] = (int)g;
-    const long long kbase = Kp[poff[i]];
-    for (int r = 0; r < N[i]; ++r)
-      for (int q = p.Kp[r]; q < p.Kp[r + 1]; ++q) kent[kbase + q] = make_int2(r, p.Kj[q]);
-    if (cls[i] == 1) {
-      encode(fent.data() + base, f - base);
-      encode(bent.data() + base, g - base);
-      encode(kent.data() + kbase, (long long)p.Kj.size());
-      nchf[i] = nchunks(flev.data() + lvl_off[i], nl);
-      nchb[i] = nchunks(blev.data() + lvl_off[i], nl);
-      nchk[i] = ((int)p.Kj.size() + kSChunk - 1) / kSChunk;
-    }
-  });
-  mark("  streams: entries");
-  // chunk tables: start relative to the stream base | scan steps <<
-  // kStepShift | (count - 1) << kCntShift
-  const auto ofch = prefix(nchf), obch = prefix(nchb), okch = prefix(nchk);
-  hvec<int> fch(ofch[B]), bch(obch[B]), kch(okch[B]);
-  std::vector<int> fch_off(B + 1), bch_off(B + 1), kch_off(B + 1);
-  for (int i = 0; i <= B; ++i) {
-    fch_off[i] = (int)ofch[i];
-    bch_off[i] = (int)obch[i];
-    kch_off[i] = (int)okch[i];
-  }
-  par_for(B, nth, [&](int i) {
-    auto put = [](int *out, const int *lev, int nl, long long base, const int2 *ent) {
-      for (int l = 0; l < nl; ++l)
-        for (long long c = lev[l]; c < lev[l + 1]; c += kSChunk) {
-          const int cnt = (int)std::min<long long>(kSChunk, lev[l + 1] - c);
-          const int steps = chunk_scan_steps<kSK>(
-              cnt, [&](int e) { return (ent[c + e].x >> 16) & kSPosMax; });
-          *out++ = (int)((c - base) | ((long long)steps << kStepShift) |
-                         ((long long)(cnt - 1) << kCntShift));
-        }
-    };
-    if (cls[i] != 1) return;
-    const long long base = Lp[poff[i]], kbase = Kp[poff[i]];
-    put(fch.data() + ofch[i], flev.data() + lvl_off[i], nlev[i], base, fent.data());
-    put(bch.data() + obch[i], blev.data() + lvl_off[i], nlev[i], base, bent.data());
-    const int klev[2] = {(int)kbase, (int)(kbase + prep[i].Kj.size())};
-    put(kch.data() + okch[i], klev, 1, kbase, kent.data());
-  });
-  // setup statistics (verbose): scan steps per chunk of each stream kind
-  auto step_stats = [&](const char *name, const int *w, size_t n, bool factor) {
-    if (!h->st.verbose) return;
-    long long hist[8] = {0, 0, 0, 0, 0, 0, 0, 0}, nc = 0, ne = 0;
-    for (size_t c = 0; c < n; ++c) {
-      if (factor && ((unsigned)w[c] >> 31)) continue;  // pivot chunks take no scan
-      ++hist[((unsigned)w[c] >> kStepShift) & 7u];
-      ++nc;
-      ne += (((unsigned)w[c] >> kCntShift) & (factor ? 63u : 127u)) + 1;
-    }
-    double mean = 0;
-    for (int q = 0; q < 8; ++q) mean += q * (double)hist[q];
-    std::fprintf(stderr,
-                 "clgpu setup: %-6s chunks %lld, entries/chunk %.1f, scan steps mean %.2f "
-                 "[%lld %lld %lld %lld %lld %lld]\n",
-                 name, nc, nc ? (double)ne / nc : 0.0, nc ? mean / nc : 0.0, hist[0], hist[1],
-                 hist[2], hist[3], hist[4], hist[5]);
-  };
-  step_stats("fwd", fch.data(), fch.size(), false);
-  step_stats("bwd", bch.data(), bch.size(), false);
-  step_stats("resid", kch.data(), kch.size(), false);
-  mark("  streams: chunks + upload");
-  // streamed factorisation: op streams, pivots and chunk tables, split over
-  // the kFactorWarps warps of the instance's block level by level
+  // ---------------- sliced layouts of the class-1 instances, concatenated
   {
-    constexpr long long kFactorSmemBytes = 96 * 1024;
-    constexpr int W = kFactorWarps;
-    const long long ring_bytes = (long long)W * kFRingSlots * kChunk * (long long)sizeof(uint2);
-    std::vector<int> fs(B, 0);
-    std::vector<long long> nch(B, 0);
-    std::vector<std::vector<int>> ich(B);
-    std::vector<std::array<int, W + 1>> iwoff(B);
-    hvec<int> flcnt((size_t)lvof[B] * W);
-    hvec<int> Lkpos((size_t)lnz);
-    // instances on the streamed factorisation, their op counts, and the
-    // streams written in place at their final offsets
-    std::vector<long long> ocnt(B, 0);
-    par_for(B, nth, [&](int i) {
-      const auto &p = prep[i];
-      // (the op words address at most kFopMaxPos work-vector positions)
-      if (cls[i] != 1 || (N[i] + (long long)p.Li.size()) * 8 + ring_bytes > kFactorSmemBytes ||
-          N[i] + (long long)p.Li.size() > kFopMaxPos)
-        return;
-      fs[i] = 1;
-      ocnt[i] = factor_op_count(p);
-    });
-    const auto oop = prefix(ocnt);
-    if (oop[B] > 2000000000LL) return -4;
-    hvec<uint2> fop(std::max<long long>(oop[B], 1));
-    par_for(B, nth, [&](int i) {
-      thread_local FactorOpScratch sc;
-      const auto &p = prep[i];
-      l_kkt_positions(p, kof[i], Lkpos.data() + lof[i], sc);
-      if (!fs[i]) return;
-      bool ok = build_factor_ops(p, fop.data() + oop[i], flcnt.data() + (size_t)lvl_off[i] * W,
-                                 ich[i], iwoff[i], sc);
-      // an op stream longer than the chunk words address, or a structure
-      // mismatch, falls back to the level-scheduled single-warp factorisation
-      if (ocnt[i] > (long long)kStartMask) ok = false;
-      if (!ok) {
-        fs[i] = 0;
-        ich[i].clear();
-        for (int w = 0; w <= W; ++w) iwoff[i][w] = 0;
-      }
-      nch[i] = (long long)ich[i].size();
-    });
-    const auto och = prefix(nch);
-    if (och[B] > 2000000000LL) return -4;
-    hvec<int> foch(std::max<long long>(och[B], 1));
-    std::vector<int> fop_base(B), fwoff((size_t)B * (W + 1));
-    bool any_fs = false;
+    std::vector<long long> cpage(B), clane(B), cvp(B), cop(B), cecol(B);
     for (int i = 0; i < B; ++i) {
-      fop_base[i] = (int)oop[i];
-      for (int w = 0; w <= W; ++w) fwoff[(size_t)i * (W + 1) + w] = (int)(och[i] + iwoff[i][w]);
-      if (fs[i]) any_fs = true;
+      const SlicedPlan &sp = plan[i];
+      cpage[i] = (long long)sp.used.size();
+      clane[i] = (long long)(sp.ent.size() / 4);
+      cvp[i] = (long long)(sp.lpos.size() / kSlRun);
+      cop[i] = (long long)(sp.ops.size() / kSlOpWords);
+      cecol[i] = (long long)sp.ecol.size();
     }
+    const auto opage = prefix(cpage), olane = prefix(clane), ovp = prefix(cvp), oop = prefix(cop), oecol = prefix(cecol);
+    if (olane[B] * 4 > 2000000000LL || oop[B] * kSlOpWords > 2000000000LL) return -4;
+    std::vector<SlInst> sl(B);
+    hvec<uint16_t> kdst((size_t)knz), lpos(ovp[B] * kSlRun), leaf(VT), ecols(oecol[B]);
+    hvec<uint32_t> ent(olane[B] * 4), ops(oop[B] * kSlOpWords);
+    hvec<int> kdiag(VT);
+    hvec<uint8_t> used(opage[B]);
+    hvec<signed char> sign(VT);
     par_for(B, nth, [&](int i) {
-      std::copy(ich[i].begin(), ich[i].end(), foch.begin() + och[i]);
-    });
-    step_stats("factor", foch.data(), foch.size(), true);
-    mark("  factor ops: build");
-    kk.fstream = A.upload(fs);
-    kk.fop_base = A.upload(fop_base);
-    kk.foch = A.upload(foch);
-    kk.fwoff = A.upload(fwoff);
-    kk.flcnt = A.upload(flcnt);
-    kk.fop = A.upload(fop);
-    kk.Lkpos = A.upload(Lkpos);
-    mark("  factor ops: upload");
-    kk.has_fstream = any_fs ? 1 : 0;
-    kk.has_small_legacy = 0;
-    for (int i = 0; i < B; ++i)
-      if (cls[i] == 1 && !fs[i]) kk.has_small_legacy = 1;
-    // launch list: streamed instances by decreasing shared-memory need (the
-    // largest start first); one block each, sized for the largest
-    {
-      auto need = [&](int i) {
-        return ((((long long)N[i] + (long long)prep[i].Li.size()) * 8 + 15) & ~15LL) +
-               ring_bytes;
+      SlInst &d = sl[i];
+      d = SlInst{};
+      if (cls[i] != 1) return;
+      SlicedPlan &sp = plan[i];
+      d.N = sp.N;
+      d.nl = sp.nl;
+      d.nk = (int)sp.kslot.size();
+      d.voff = voff[i];
+      d.stage0 = (int)opage[i];
+      d.nf = sp.nstage[0];
+      d.nb = sp.nstage[1];
+      d.nr = sp.nstage[2];
+      d.lane0 = (int)olane[i];
+      d.vlane0 = (int)ovp[i];
+      d.nvlane = (int)cvp[i];
+      d.kx0 = (int)kof[i];
+      d.nkx = (int)sp.kdst.size();
+      d.opage0 = (int)oop[i];
+      d.nops = (int)sp.ops.size();
+      d.nleaf = (int)sp.leaf.size();
+      d.ncarry = sp.ncarry;
+      d.nopcarry = sp.nopcarry;
+      d.ecol0 = (int)oecol[i];
+      for (int w = 0; w < kSlWarps; ++w)
+        d.w[w] = {sp.op.first[w], sp.op.count[w], sp.op.skip[w]};
+      auto put = [](auto &dst, long long at, const auto &src, size_t n) {
+        std::copy(src.begin(), src.begin() + n, dst.begin() + at);
       };
-      std::vector<int> items;
-      for (int i = 0; i < B; ++i)
-        if (fs[i]) items.push_back(i);
-      std::stable_sort(items.begin(), items.end(),
-                       [&](int a, int b) { return need(a) > need(b); });
-      kk.fs_count = (int)items.size();
-      kk.fs_smem = items.empty() ? 0 : (int)need(items[0]);
-      kk.fs_inst = A.upload(items);
+      put(kdst, kof[i], sp.kdst, sp.kdst.size());
+      put(lpos, ovp[i] * kSlRun, sp.lpos, sp.lpos.size());
+      put(used, opage[i], sp.used, sp.used.size());
+      put(leaf, voff[i], sp.leaf, sp.leaf.size());
+      put(sign, voff[i], sp.sign, sp.sign.size());
+      for (int r = 0; r < sp.N; ++r) kdiag[voff[i] + r] = sp.kslot[prep[i].Kdiag[r]];
+      put(ecols, oecol[i], sp.ecol, sp.ecol.size());
+      put(ent, olane[i] * 4, sp.ent, sp.ent.size());
+      put(ops, oop[i] * kSlOpWords, sp.ops, sp.ops.size());
+      sp = SlicedPlan();  // freed here, by all threads
+    });
+    if (h->st.verbose) {
+      long long nl = 0, nk = 0;
+      for (const SlInst &d : sl) {
+        nl += d.nl;
+        nk += d.nk;
+      }
+      std::fprintf(stderr,
+                   "clgpu setup: sliced L entries %lld in %lld slots (both passes), K %lld in "
+                   "%lld, op words %lld\n",
+                   nl, ovp[B] * kSlRun, nk, knz, oop[B] * kSlOpWords);
     }
+    kk.sl = A.upload(sl);
+    kk.sl_kdst = A.upload(kdst);
+    kk.sl_kdiag = A.upload(kdiag);
+    kk.sl_used = A.upload(used);
+    kk.sl_ent = A.upload(ent);
+    kk.sl_ops = A.upload(ops);
+    kk.sl_lpos = A.upload(lpos);
+    kk.sl_leaf = A.upload(leaf);
+    kk.sl_sign = A.upload(sign);
+    kk.sl_ecol = A.upload(ecols);
+    const size_t nval = (size_t)(ovp[B] * kSlRun);
+    kk.sl_val = h->mixed ? (void *)A.alloc<float>(nval, false) : A.alloc<double>(nval, false);
+    // launch order: the largest need of shared memory first
+    std::vector<long long> s1(B, 0), s2(B, 0), f1(B, 0), f2(B, 0);
+    std::vector<int> items;
+    for (int i = 0; i < B; ++i)
+      if (cls[i] == 1) {
+        items.push_back(i);
+        const SlInst &d = sl[i];
+        const long long ring = (long long)kSlRing * kSlStage * (8 * kSlRun + 16) +
+                               (((long long)cpage[i] + 15) & ~15LL);
+        const long long slots = 2LL * N[i] + 1 + d.ncarry;
+        s1[i] = ring + 8 * slots;
+        s2[i] = ring + 16 * slots;
+        const long long tab = (long long)kSlWarps * kSlOpRing * 512 + ((N[i] + 15) & ~15LL);
+        f1[i] = tab + 8LL * (N[i] + d.nl + 1 + d.nopcarry);
+        f2[i] = tab + 4LL * (N[i] + d.nl + 1 + d.nopcarry);
+      }
+    auto order = [&](const std::vector<long long> &need) {
+      std::vector<int> v = items;
+      std::stable_sort(v.begin(), v.end(), [&](int a, int b) { return need[a] > need[b]; });
+      return v;
+    };
+    const auto so = order(s1), fo = order(f1);
+    kk.sl_solve_inst = A.upload(so);
+    kk.sl_factor_inst = A.upload(fo);
+    kk.sl_solve = sl_groups(so, s1, s2);
+    kk.sl_factor = sl_groups(fo, f1, f2);
+    mark("sliced upload");
   }
   kk.cls = A.upload(cls);
   // ---------------- supernodal instances: plan and numeric storage
@@ -1972,82 +1695,37 @@ static int build_batch(clgpu_solver *h, std::vector<Prepared> &prep, int nth) {
         vlo = std::min(vlo, voff[i]);
         vhi = std::max(vhi, voff[i + 1]);
       }
-    SnPlan plan;
+    SnPlan snp;
     std::string err;
-    if (!sn_build_plan(sin, plan, &err)) return -4;
+    if (!sn_build_plan(sin, snp, &err)) return -4;
     std::vector<int> vinst(vhi - vlo, -1);
     for (int i = 0; i < B; ++i)
       if (cls[i] == 3)
         for (int v = voff[i]; v < voff[i + 1]; ++v) vinst[v - vlo] = i;
     h->sn.reset(new SnExec());
-    if (!sn_exec_create(plan, h->mixed, B, vlo, vhi - vlo, vinst, A, *h->sn)) return -5;
+    if (!sn_exec_create(snp, h->mixed, B, vlo, vhi - vlo, vinst, A, *h->sn)) return -5;
     kk.sn = h->sn.get();
     mark("supernodal plan");
   }
-  // pack single-warp solves into blocks of kSolveWarps warps: each warp needs
-  // its work vector (N FP64 values) and its ring (entries + FP64 values);
-  // bins sized so kSolveBlocksPerSM blocks fit an SM's shared memory
-  // (two-side solves: two work vectors per warp)
-  for (int nr = 1; nr <= 2; ++nr) {
-    auto need = [&](int i) {
-      return nr * (((long long)N[i] * 8 + 15) & ~15LL) +
-             (long long)kSRingSlots * kSChunk * (long long)(sizeof(int2) + sizeof(double));
-    };
-    std::vector<int> items, pinst, poffv;
-    for (int i = 0; i < B; ++i)
-      if (cls[i] == 1) items.push_back(i);
-    long long cap = ((228LL * 1024) / kSolveBlocksPerSM - 1024) & ~15LL;
-    for (int i : items) cap = std::max(cap, need(i));
-    const int nb = ffd_pack(items, need, cap, kSolveWarps, pinst, poffv);
-    if (nr == 1) {
-      kk.spack_blocks = nb;
-      kk.spack_inst = A.upload(pinst);
-      kk.spack_off = A.upload(poffv);
-      kk.spack_smem = (int)cap;
-    } else {
-      kk.spack2_blocks = nb;
-      kk.spack2_inst = A.upload(pinst);
-      kk.spack2_off = A.upload(poffv);
-      kk.spack2_smem = (int)cap;
-    }
-  }
-  kk.fch = A.upload(fch);
-  kk.bch = A.upload(bch);
-  kk.kch = A.upload(kch);
-  kk.fch_off = A.upload(fch_off);
-  kk.bch_off = A.upload(bch_off);
-  kk.kch_off = A.upload(kch_off);
-  kk.fent = A.upload(fent);
-  kk.bent = A.upload(bent);
-  kk.fpos = A.upload(fpos);
-  kk.bpos = A.upload(bpos);
-  kk.flev = A.upload(flev);
-  kk.blev = A.upload(blev);
-  kk.kent = A.upload(kent);
+  // scalar factor of the block kernels
+  const size_t lv = has_large ? (size_t)lnz : 0;
   if (h->mixed) {
-    kk.LxF = A.alloc<float>((size_t)lnz);
-    kk.LxB = A.alloc<float>((size_t)lnz);
-    kk.LxR = has_large ? A.alloc<float>((size_t)lnz) : nullptr;
-    kk.Lx = A.alloc<float>((size_t)lnz);
-    kk.D = A.alloc<float>(VT);
+    kk.LxR = A.alloc<float>(lv);
+    kk.Lx = A.alloc<float>(lv);
+    kk.D = A.alloc<float>(has_large ? VT : 0);
     kk.Dinv = A.alloc<float>(VT);
-    kk.Lacc = A.alloc<double>((size_t)lnz);
-    kk.Dacc = A.alloc<double>(VT);
+    kk.Lacc = A.alloc<double>(lv);
+    kk.Dacc = A.alloc<double>(has_large ? VT : 0);
   } else {
-    kk.LxF = A.alloc<double>((size_t)lnz);
-    kk.LxB = A.alloc<double>((size_t)lnz);
-    kk.LxR = has_large ? A.alloc<double>((size_t)lnz) : nullptr;
-    kk.Lx = A.alloc<double>((size_t)lnz);
-    kk.D = A.alloc<double>(VT);
+    kk.LxR = A.alloc<double>(lv);
+    kk.Lx = A.alloc<double>(lv);
+    kk.D = A.alloc<double>(has_large ? VT : 0);
     kk.Dinv = A.alloc<double>(VT);
     kk.Lacc = nullptr;
     kk.Dacc = nullptr;
   }
-  mark("schedules + streams");
-  kk.yf = A.alloc<double>(VT);
-  kk.w = A.alloc<double>(VT);
-  kk.max_small_N = max_small;
-  kk.has_small = has_small;
+  kk.yf = A.alloc<double>(has_large ? VT : 0);
+  kk.w = A.alloc<double>(has_large ? VT : 0);
   kk.has_large = has_large;
   kk.b = A.alloc<double>(VT);
   kk.x = A.alloc<double>(VT);
@@ -2055,7 +1733,7 @@ static int build_batch(clgpu_solver *h, std::vector<Prepared> &prep, int nth) {
   kk.b2 = A.alloc<double>(VT);
   kk.x2 = A.alloc<double>(VT);
   kk.e2 = A.alloc<double>(VT);
-  kk.dx = A.alloc<double>(VT);
+  kk.dx = A.alloc<double>(has_large ? VT : 0);
   // ---------------- vectors and scalars
   Dev &dv = h->dv;
   dv.B = B;
@@ -2226,22 +1904,19 @@ static int build_batch(clgpu_solver *h, std::vector<Prepared> &prep, int nth) {
   return 0;
 }
 
-// Host replay of one instance's streamed-factorisation op stream (the
-// records, chunk words and level counts build_batch uploads) on a
-// quasi-definite matrix with the instance's KKT pattern, against a dense
-// LDL^T of the same permuted matrix.  The replay follows the kernel's
-// schedule: per level, every warp part's update chunks (a segment's sum is
-// subtracted from its target at the segment's last record, carried across
-// chunk boundaries), then every part's pivot chunks (V[j] becomes 1/d_j);
-// at the end L(i,j) = U(i,j) / d_j.  *resid receives the largest difference
-// of L and D entries relative to the largest |D|.  Returns 0, -2 when the
-// instance cannot be prepared, -3 when it does not take the streamed path,
-// -4 when it is too large for the dense reference (N > 2000), or a negative
-// structure code.
+// Host replay of one instance's sliced layouts (sliced.hpp: the op stream,
+// the substitution pages and the residual slices that build_batch uploads) on
+// a quasi-definite matrix with the instance's KKT pattern, in the kernels'
+// schedule (ldl_sliced.cu).  The factor is compared with a dense LDL^T of the
+// same permuted matrix, then a solve with it through the pages is checked by
+// its residual through the slices.  *resid receives the largest difference of
+// the L and D entries relative to the largest |D|, or that residual if it is
+// larger.  Returns 0, -2 when the instance cannot be prepared, -3 when it does
+// not take this path, -4 when it is too large for the dense reference (N >
+// 2000), or a negative structure code.
 extern "C" int clgpu_debug_factor_stream(const clgpu_problem *pb, const clgpu_settings *st,
                                          double *resid) {
   using namespace clgpu;
-  constexpr int W = kFactorWarps;
   if (!pb) return -1;
   SetupOptions opt;
   if (st) {
@@ -2252,16 +1927,10 @@ extern "C" int clgpu_debug_factor_stream(const clgpu_problem *pb, const clgpu_se
   Prepared p;
   if (!prepare_instance(*pb, opt, p)) return -2;
   const int N = p.N, nli = (int)p.Li.size();
-  if (p.supernodal || N + nli > kFopMaxPos) return -3;
+  if (!sl_fits(p)) return -3;
   if (N > 2000) return -4;
-  FactorOpScratch sc;
-  std::vector<int> Lkpos(nli);
-  l_kkt_positions(p, 0, Lkpos.data(), sc);
-  const int nl = (int)p.lvl_ptr.size() - 1;
-  std::vector<uint2> ops(factor_op_count(p));
-  std::vector<int> flcnt((size_t)nl * W), chk;
-  std::array<int, W + 1> woff;
-  if (!build_factor_ops(p, ops.data(), flcnt.data(), chk, woff, sc)) return -5;
+  SlicedPlan sp;
+  if (!sl_build(p, 2, sp)) return -5;
   // the quasi-definite test matrix of clgpu_debug_check_instance
   const int knz = (int)p.Kj.size();
   std::vector<double> Kx(knz, 0.0);
@@ -2271,54 +1940,79 @@ extern "C" int clgpu_debug_factor_stream(const clgpu_problem *pb, const clgpu_se
       if (c != r) Kx[q] = 0.01 * std::sin(1.0 + r + 7.0 * c) * std::sin(1.0 + c + 7.0 * r);
     }
   for (int r = 0; r < N; ++r) Kx[p.Kdiag[r]] = p.Dsign[r] * 2.0;
-  // replay
-  std::vector<double> V(N + nli, 0.0), D(N, 0.0);
-  for (int j = 0; j < N; ++j) V[j] = Kx[p.Kdiag[j]];
-  for (int q = 0; q < nli; ++q) V[N + q] = Lkpos[q] >= 0 ? Kx[Lkpos[q]] : 0.0;
-  int cur[W];
-  for (int w = 0; w < W; ++w) cur[w] = woff[w];
-  auto chunk = [&](int w, bool pivot_expected, double &acc) {
-    if (cur[w] >= woff[w + 1]) return -6;
-    const unsigned word = (unsigned)chk[cur[w]++];
-    const bool pivot = (word >> 31) != 0;
-    if (pivot != pivot_expected) return -7;
-    const int p0 = (int)(word & kStartMask), cnt = (int)((word >> kCntShift) & 63u) + 1;
-    if (p0 + cnt > (int)ops.size()) return -8;
-    for (int e = 0; e < cnt; ++e) {
-      const uint2 o = ops[p0 + e];
-      const int t = fop_t(o), a = fop_a(o);
-      if (t >= N + nli || a >= N + nli) return -9;
-      if (pivot) {
-        const int sgn = a - 1;
-        if (t >= N || (sgn != 1 && sgn != -1) || sgn != p.Dsign[t]) return -10;
-        D[t] = V[t];
-        V[t] = 1.0 / V[t];
-      } else {
-        const int b = fop_b(o), k = fop_k(o);
-        if (b >= N + nli || k >= N) return -11;
-        if (fop_pos(o) == 0) acc = 0.0;
-        acc += V[a] * V[b] * V[k];
-        if (fop_last(o)) V[t] -= acc;
-      }
+  // replay: the values through their stored slots, then warp by warp up to each
+  // level's end, the level's pivots, and so on
+  const int zero = N + nli;
+  std::vector<double> kv(sp.kdst.size(), 0.0), V(zero + 1 + sp.nopcarry, 0.0), D(N, 0.0);
+  for (int k = 0; k < knz; ++k) kv[sp.kslot[k]] = Kx[k];
+  for (size_t t = 0; t < kv.size(); ++t)
+    if (sp.kdst[t] != kSlNone) {
+      if (sp.kdst[t] >= zero) return -6;
+      V[sp.kdst[t]] = kv[t];
     }
-    return 0;
+  // lane sums -> the parts' sums, as the kernels' scan adds them
+  auto scan = [](double (&x)[32], auto reach, auto prev, int steps) {
+    for (int h = 0; h < steps; ++h) {
+      double was[32];
+      std::copy(x, x + 32, was);
+      for (int t = 0; t < 32; ++t)
+        if ((1 << h) <= reach(t)) x[t] = t >= 1 << h ? was[t] + was[t - (1 << h)] : NAN;
+    }
+    double was[32];
+    std::copy(x, x + 32, was);
+    for (int t = 0; t < 32; ++t)
+      if (prev(t)) x[t] = t ? was[t] + was[t - 1] : NAN;
   };
-  for (int l = 0; l < nl; ++l) {
-    for (int w = 0; w < W; ++w) {
-      double acc = 0.0;
-      const int nop = flcnt[(size_t)l * W + w] & 0xffff;
-      for (int c = 0; c < nop; ++c)
-        if (int rc = chunk(w, false, acc)) return rc;
-    }
-    for (int w = 0; w < W; ++w) {
-      double acc = 0.0;
-      const int npv = (flcnt[(size_t)l * W + w] >> 16) & 0xffff;
-      for (int c = 0; c < npv; ++c)
-        if (int rc = chunk(w, true, acc)) return rc;
+  int taken = 0;
+  auto pivot = [&](int j) {
+    D[j] = V[j];
+    if ((D[j] < 0) != (sp.sign[j] < 0)) return false;
+    V[j] = 1.0 / D[j];
+    ++taken;
+    return true;
+  };
+  for (int j : sp.leaf)
+    if (j >= N || D[j] != 0.0 || !pivot(j)) return -7;
+  int at[kSlWarps], wait[kSlWarps];
+  for (int w = 0; w < kSlWarps; ++w) {
+    at[w] = sp.op.first[w];
+    wait[w] = sp.op.skip[w];
+  }
+  for (int ev = 1; ev <= sp.olevels; ++ev) {
+    for (int w = 0; w < kSlWarps; ++w) {
+      for (; wait[w] == 0; ++at[w]) {
+        if (at[w] >= sp.op.first[w] + sp.op.count[w]) return -8;
+        const uint32_t *pg = sp.ops.data() + (size_t)at[w] * kSlOpWords;
+        auto f = [&](int t, int bit, int width) {
+          return (int)sl_op_field(pg + 4 * t, bit, width);
+        };
+        double x[32];
+        for (int t = 0; t < 32; ++t) {
+          for (int b = 0; b < 8; ++b)
+            if (f(t, 14 * b, 14) >= (int)V.size()) return -9;
+          x[t] = V[f(t, 98, 14)];
+          for (int c = 0; c < kSlOpRun; ++c)
+            x[t] += V[f(t, 42 * c, 14)] * V[f(t, 42 * c + 14, 14)] * V[f(t, 42 * c + 28, 14)];
+          if (f(t, 118, 10) != f(0, 118, 10)) return -10;
+        }
+        scan(x, [&](int t) { return f(t, 112, 5); }, [&](int t) { return f(t, 117, 1) != 0; },
+             f(0, 118, 3));
+        for (int t = 0; t < 32; ++t) {
+          const int to = f(t, 84, 14);
+          if (to < zero)
+            V[to] -= x[t];
+          else if (to > zero)
+            V[to] = x[t];
+          if (to < N && (D[to] != 0.0 || !pivot(to))) return -11;
+        }
+        wait[w] = f(0, 121, 7);
+      }
+      --wait[w];
     }
   }
-  for (int w = 0; w < W; ++w)
-    if (cur[w] != woff[w + 1]) return -12;  // every chunk replayed
+  for (int w = 0; w < kSlWarps; ++w)
+    if (wait[w] != 0 || at[w] != sp.op.first[w] + sp.op.count[w]) return -12;
+  if (taken != N || V[zero] != 0.0) return -13;
   // dense LDL^T of the same permuted matrix
   std::vector<double> Ad((size_t)N * N, 0.0), Ld((size_t)N * N, 0.0), Dd(N, 0.0);
   for (int r = 0; r < N; ++r)
@@ -2335,10 +2029,76 @@ extern "C" int clgpu_debug_factor_stream(const clgpu_problem *pb, const clgpu_se
   }
   double dmax = 0.0, err = 0.0;
   for (int j = 0; j < N; ++j) dmax = std::max(dmax, std::fabs(Dd[j]));
+  double *M = V.data() + N;
   for (int j = 0; j < N; ++j) {
     err = std::max(err, std::fabs(D[j] - Dd[j]));
-    for (int q = p.Lp[j]; q < p.Lp[j + 1]; ++q)
-      err = std::max(err, std::fabs(V[N + q] * V[j] - Ld[(size_t)p.Li[q] * N + j]));
+    for (int q = p.Lp[j]; q < p.Lp[j + 1]; ++q) {
+      if (sp.ecol[q] != j) return -13;
+      M[q] *= V[j];
+      err = std::max(err, std::fabs(M[q] - Ld[(size_t)p.Li[q] * N + j]));
+    }
+  }
+  // a solve: y = L^-T D^-1 L^-1 rhs through the pages, rhs - K y through the
+  // residual's (the slot N gathers as zero)
+  std::vector<double> y(N + 1 + sp.ncarry, 0.0), rhs(N), ky(N);
+  for (int i = 0; i < N; ++i) y[i] = rhs[i] = std::sin(1.0 + 3.0 * i);
+  const int nli_ = nli;
+  size_t stage = 0, lane0 = 0, vlane = 0, klane = 0;
+  auto pass = [&](int ps, auto value) {
+    for (int st = 0; st < sp.nstage[ps]; ++st, ++stage) {
+      if (stage >= sp.used.size()) return -14;
+      const int used = sp.used[stage];
+      if (used < 1 || used > kSlStage || (lane0 + used) * 4 > sp.ent.size()) return -15;
+      for (int l0 = 0; l0 < used; l0 += 32) {
+        uint32_t e[kSlPage];  // lanes beyond the used ones repeat the last
+        for (int t = 0; t < 32; ++t)
+          std::copy_n(sp.ent.data() + 4 * (lane0 + std::min(l0 + t, used - 1)), 4, e + 4 * t);
+        double x[32];
+        const unsigned ctl = e[3] >> 16;
+        for (int t = 0; t < 32; ++t) {
+          const unsigned ini = e[4 * t + 2] >> 16;
+          if (e[4 * t + 3] >> 16 != ctl || ini >= y.size() || e[4 * t] >> 16 >= y.size())
+            return -15;
+          x[t] = ctl & 8u ? y[ini] : 0.0;
+          for (int c = 0; c < kSlRun; ++c) {
+            const unsigned id = e[4 * t + c] & 0xffff;
+            if (id % 8 || id / 8 >= y.size()) return -15;
+            x[t] += value(used, c, std::min(l0 + t, used - 1)) * y[id / 8];
+          }
+        }
+        scan(x, [&](int t) { return (int)((e[4 * t + 1] >> 16) & 31u); },
+             [&](int t) { return ctl & 16u && (e[4 * t + 1] >> 21) & 1u; }, (int)(ctl & 7u));
+        for (int t = 0; t < std::min(32, used - l0); ++t) {
+          const int to = (int)(e[4 * t] >> 16);
+          if (to > N)
+            y[to] = x[t];
+          else if (to < N)
+            (ps == 2 ? ky : y)[to] = ps == 2 ? x[t] : y[to] - x[t];
+        }
+      }
+      lane0 += used;
+      (ps == 2 ? klane : vlane) += used;
+    }
+    return 0;
+  };
+  auto lval = [&](int used, int c, int t) {
+    if ((vlane + used) * kSlRun > sp.lpos.size()) return (double)NAN;
+    const uint16_t lp = sp.lpos[vlane * kSlRun + sl_at(c, t, 2, used)];
+    return lp == kSlNone ? 0.0 : (lp < nli ? M[lp] : (double)NAN);
+  };
+  if (int rc = pass(0, lval)) return rc;
+  for (int j = 0; j < N; ++j) y[j] /= D[j];
+  if (int rc = pass(1, lval)) return rc;
+  if (y[N] != 0.0) return -17;
+  if (int rc = pass(2, [&](int used, int c, int t) {
+        return (klane + used) * kSlRun > kv.size()
+                   ? (double)NAN
+                   : kv[klane * kSlRun + sl_at(c, t, 2, used)];
+      }))
+    return rc;
+  for (int i = 0; i < N; ++i) {
+    const double d = std::fabs(rhs[i] - ky[i]);
+    err = std::max(err, std::isfinite(d) ? d * dmax : HUGE_VAL);
   }
   if (resid) *resid = err / std::max(dmax, 1e-300);
   return 0;

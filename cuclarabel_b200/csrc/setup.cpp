@@ -420,12 +420,11 @@ static void csc_transpose(const HostCSC &A, HostCSC &T) {
     }
 }
 
-// entries of the single-warp kernels' encoded streams addressable by a
-// chunk word (ldl.cuh kStartMask)
+// entries of the largest factor or matrix the scalar paths take
 constexpr long long kStreamMaxEntries = (1LL << 22) - 1;
 
 // dense columns: a factor column longer than this belongs to a dense front
-// (the supernodal path factors it with tensor-core tiles; the single-warp
+// (the supernodal path factors it with tensor-core tiles; the scalar
 // kernels are built for sparse columns)
 constexpr int kScalarMaxColumn = 512;
 
@@ -777,10 +776,10 @@ bool prepare_instance(const clgpu_problem &pb, const SetupOptions &opt, Prepared
         adjncy[cur[en.r]++] = en.c;
         adjncy[cur[en.c]++] = en.r;
       }
-    // instances whose work vector exceeds the single-warp kernels' budget
-    // (48 KB of FP64), whose factor or matrix exceeds the range of their
-    // stream chunk words, or whose factor has dense columns (> 512 entries)
-    // take the supernodal factorisation
+    // instances whose work vector exceeds the block kernels' budget
+    // (48 KB of FP64), whose factor or matrix has more than kStreamMaxEntries
+    // entries, or whose factor has dense columns (> 512 entries) take the
+    // supernodal factorisation
     out.supernodal = (long long)N * 8 > 48 * 1024 || (long long)xadj[N] + N > kStreamMaxEntries;
     if (!out.supernodal) {
       out.perm = nd_order_csr(N, xadj, adjncy);
@@ -1246,7 +1245,7 @@ extern "C" int clgpu_debug_check_instance(const clgpu_problem *pb, const clgpu_s
         if (lvl[p.Rk[r]] >= lvl[j]) return -26;  // dependency must be on a lower level
   }
   std::vector<double> w(N, 0.0), Lx(lnz, 0.0), D(N, 0.0);
-  const int narrow_below = 16;  // NT/2 for the single-warp kernel
+  const int narrow_below = 16;  // levels below this are narrow
   for (int l = 0; l < nlev; ++l) {
     const int a = p.lvl_ptr[l], bnd = p.lvl_ptr[l + 1];
     for (int t = a; t < bnd; ++t) {

@@ -48,7 +48,7 @@ struct Prepared {
   std::vector<signed char> Dsign;  // permuted
   std::vector<int> Lp, Li, Rp, Rk, Rpos;
   std::vector<int> lvl_ptr, lvl_nodes;  // elimination-tree levels (leaves first)
-  // Large instances (work vector beyond the single-warp kernels' budget)
+  // Large instances (work vector beyond the block kernels' budget)
   // take the supernodal factorisation: AMD ordering, supernodal symbolic
   // structure in sym, and no scalar structures (Lp, Rp zero, Li, Rk, Rpos
   // and the levels empty).

@@ -5,7 +5,7 @@
 // every IPM iteration (:37-46) and a solve (:50-59), in FP64 or, for
 // :cudssmixed, in FP32 (directldl_mixed_cudss.jl:24-78).  cuDSS is not
 // available here; this is the project's own sparse direct solver for the
-// instances too large for the single-warp kernels.
+// instances too large for the block-per-instance kernels.
 //
 // Host side (supernodal.cpp): approximate minimum degree ordering
 // (amd.cpp), elimination tree and postorder, column counts, fundamental

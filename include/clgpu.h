@@ -193,12 +193,12 @@ int clgpu_solver_get_phase_times(const clgpu_solver *h, double *ms,
                                  long long *calls);
 /* algorithmic bytes of the last profiled solve, bytes[3]: bytes[0] all LDL
  * factorisations, bytes[1] all one-side LDL solves, bytes[2] all two-side
- * solves, with refinement (each stream pass reads its entries, values and
- * chunk words once per side; vectors once per use).  Divided by the phase
+ * solves, with refinement (each pass over the factor or K reads its values
+ * and indices once; vectors once per use).  Divided by the phase
  * times this gives the achieved bandwidth.  No reference counterpart. */
 int clgpu_solver_get_phase_bytes(const clgpu_solver *h, double *bytes);
 /* Supernodal factorisation of the large instances (those whose KKT work
- * vector exceeds the single-warp kernels' 48 KB), per launch kind, summed
+ * vector exceeds the block kernels' 48 KB), per launch kind, summed
  * over the solves since profiling was switched on: device ms (each launch
  * bracketed by CUDA events), algorithmic flops and launches, CLGPU_SN_KINDS
  * entries each (any pointer may be NULL).  Kinds: 0 small fronts, 1 front
@@ -457,18 +457,18 @@ int clgpu_debug_check_instance(const clgpu_problem *prob,
                                const clgpu_settings *settings, double *resid);
 /* Host-only view of the factorisation path setup picks for one instance
  * (diagnostic, no reference counterpart): *supernodal = 1 for the
- * supernodal (dense-front) LDL^T, 0 for the single-warp kernels, and the
+ * supernodal (dense-front) LDL^T, 0 for the block-per-instance kernels, and the
  * factor's strictly-lower entries.  Needs no GPU. */
 int clgpu_debug_instance_path(const clgpu_problem *prob, const clgpu_settings *settings,
                               int *supernodal, long long *factor_entries);
-/* Host replay of one instance's streamed-factorisation op stream (the 8-byte
- * records, chunk words and per-level counts that setup uploads for
- * k_ldl_factor_stream) on a quasi-definite matrix with the instance's KKT
- * pattern, compared with a dense LDL^T of the same permuted matrix
- * (diagnostic, no reference counterpart): *resid = largest difference of
- * the L and D entries relative to the largest |D|.  Returns 0, or -3 when
- * the instance does not take the streamed path, -4 when N > 2000, other
- * negative codes for structure errors.  Needs no GPU. */
+/* Host replay of the layouts that setup uploads for one instance's
+ * block-per-instance LDL^T (op pages, substitution and residual stages) on a
+ * quasi-definite matrix with the instance's KKT pattern, in the kernels'
+ * schedule (diagnostic, no reference counterpart): *resid = the largest
+ * difference of the L and D entries from a dense LDL^T of the same permuted
+ * matrix, relative to the largest |D|, or the residual of a solve if that is
+ * larger.  Returns 0, or -3 when the instance does not take this path, -4
+ * when N > 2000, other negative codes for structure errors.  Needs no GPU. */
 int clgpu_debug_factor_stream(const clgpu_problem *prob, const clgpu_settings *settings,
                               double *resid);
 /* Counters of the process-wide page-locked host pool that setup arrays,

@@ -1,0 +1,70 @@
+"""The block-per-instance LDL^T (csrc/ldl_sliced.cu) where its layouts have
+edges: sums that span several chunks of their stream (rows and columns of more
+than 128 and 256 terms), levels of one short page and of many pages, an
+instance without off-diagonal factor entries, and pivots without dynamic
+regularisation."""
+import ctypes
+
+import numpy as np
+import pytest
+import scipy.sparse as sp
+
+from cuclarabel_b200 import (BatchSolver, NonnegativeConeT, Solver, ZeroConeT, _lib, problems)
+from cuclarabel_b200.api import Settings, _prep_problem
+from helpers import ITER_TOL, OBJ_RTOL, rel_err
+
+
+def budget(n, seed=0):
+    """min x'Px/2 + q'x, sum x = 1, x >= 0: one row of n entries."""
+    r = np.random.default_rng(seed)
+    A = sp.vstack([sp.csc_matrix(np.ones((1, n))), -sp.identity(n)], format="csc")
+    return (sp.diags(r.uniform(0.5, 2, n), format="csc"), r.standard_normal(n), A,
+            np.concatenate([[1.0], np.zeros(n)]), [ZeroConeT(1), NonnegativeConeT(n)])
+
+
+CASES = {
+    "one_variable": lambda: (sp.csc_matrix([[2.0]]), np.array([-1.0]), sp.csc_matrix([[1.0]]),
+                             np.array([0.3]), [NonnegativeConeT(1)]),
+    "budget_127": lambda: budget(127),
+    "budget_128": lambda: budget(128),
+    "budget_300": lambda: budget(300),
+    "psd_3": lambda: problems.psd_lp(3, 1, seed=2),
+    "psd_8": lambda: problems.psd_lp(8, 3, seed=2),
+    "mpc_small": lambda: problems.mpc_qp(5, n=20),
+    "mpc_large": lambda: problems.mpc_qp(6, n=400),
+}
+
+
+@pytest.mark.parametrize("name", CASES)
+def test_layouts_replay_on_the_host(name):
+    cp, keep, n, m = _prep_problem(*CASES[name]())
+    st = Settings().to_c()
+    r = ctypes.c_double()
+    rc = _lib.load().clgpu_debug_factor_stream(ctypes.byref(cp), ctypes.byref(st),
+                                               ctypes.byref(r))
+    assert rc == 0 and r.value < 1e-12, (rc, r.value)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dyn", [True, False])
+@pytest.mark.parametrize("name", CASES)
+def test_solves_match_the_oracle(cuda_device, name, dyn):
+    import oracle
+    pb = CASES[name]()
+    sol = Solver(*pb, dynamic_regularization_enable=dyn).solve()
+    ref = oracle.solve(*pb)
+    assert sol.status.name == ref["status_name"] == "SOLVED"
+    assert rel_err(sol.obj_val, ref["obj_val"]) < OBJ_RTOL
+    assert abs(sol.iterations - ref["iterations"]) <= ITER_TOL
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("method", ["cudss", "cudssmixed", "mixed_f64elim"])
+def test_mixed_sizes_give_the_bits_of_each_alone(cuda_device, method):
+    """Instances of very different shared-memory needs in one batch (so in
+    several launches) return exactly what each returns alone."""
+    pbs = [c() for c in CASES.values()]
+    opts = dict(direct_solve_method=method, max_iter=4)
+    for pb, s in zip(pbs, BatchSolver(pbs, **opts).solve()):
+        a = BatchSolver([pb], **opts).solve()[0]
+        assert np.array_equal(a.x, s.x) and np.array_equal(a.s, s.s) and np.array_equal(a.z, s.z)
