@@ -68,3 +68,33 @@ def test_mixed_sizes_give_the_bits_of_each_alone(cuda_device, method):
     for pb, s in zip(pbs, BatchSolver(pbs, **opts).solve()):
         a = BatchSolver([pb], **opts).solve()[0]
         assert np.array_equal(a.x, s.x) and np.array_equal(a.s, s.s) and np.array_equal(a.z, s.z)
+
+
+def _entries(pb):
+    cp, keep, n, m = _prep_problem(*pb)
+    st = Settings().to_c()
+    sn, ent = ctypes.c_int(), ctypes.c_longlong()
+    assert _lib.load().clgpu_debug_instance_path(ctypes.byref(cp), ctypes.byref(st),
+                                                 ctypes.byref(sn), ctypes.byref(ent)) == 0
+    return sn.value, ent.value
+
+
+@pytest.mark.parametrize("assets", [20, 50, 200])
+def test_coupled_problems_are_ordered_by_minimum_degree(assets):
+    """A budget row over all assets: dissection would leave 2 to 13 times K's
+    entries, minimum degree stays below them (7 N bounds K here)."""
+    P, q, A, b, cones = problems.portfolio(3, assets, 5)
+    sn, ent = _entries((P, q, A, b, cones))
+    assert sn == 0 and ent < 2 * A.nnz + len(q) + len(b)
+
+
+@pytest.mark.parametrize("seed", [0, 1881, 2335, 3584])
+def test_banded_problems_keep_dissection(seed):
+    """The control family (its densest factor and deepest tree among them):
+    minimum degree has less fill there but trees three to eight times as
+    deep, so a shallow tree with more entries shows dissection."""
+    pb = problems.mpc_qp(seed)
+    cp, keep, n, m = _prep_problem(*pb)
+    sn, ent = _entries(pb)
+    nnz = 2 * pb[2].nnz + n + m  # K without the cones' blocks
+    assert sn == 0 and ent > 0.5 * nnz
