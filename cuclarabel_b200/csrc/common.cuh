@@ -76,6 +76,7 @@ struct ConeSet {
   double *exp_Hd, *exp_Hs, *exp_grad, *exp_z;  // 9,9,3,3 per cone
   double *pow_Hd, *pow_Hs, *pow_grad, *pow_z;
   double *psd_R, *psd_Rinv, *psd_lam;  // nmax^2, nmax^2, nmax per cone
+  double *psd_eig;  // step length scratch, nmax (nmax + 1) per cone
   // per-instance flags
   const int *inst_active;  // [B] nonzero -> instance takes part
   const int *inst_sym;     // [B] 1 if every cone of the instance is symmetric

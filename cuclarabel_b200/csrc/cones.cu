@@ -881,6 +881,175 @@ __global__ void k_psd_update_scaling(ConeSet cs, const double *__restrict__ s,
   for (int r = p.lane; r < n; r += p.g.G) lam[r] = S[r];
 }
 
+// The same for sides up to kPsdPairSide, four lanes per cone and eight cones
+// per warp.  A lane takes a whole rotation of the Jacobi sweep: the pairs (p, q)
+// with the same p + q touch different columns, and every earlier pair of the
+// row-cyclic order that shares a column with (p, q) has a smaller p + q, so
+// running them side by side gives the row-cyclic sweep's own result, in 2 n - 3
+// steps.  (One cone per 16 lanes, one pair at a time, spent its time in the
+// exchanges of three 16-lane sums per pair and repeated each rotation's
+// division and square roots on all lanes: 79 k warp instructions per 10 x 10
+// cone, 3.87 ms for 40 000; now 0.65 ms.)  Matrices are interleaved over
+// the warp's cones, so lanes of one step read neighbouring words.
+constexpr int kPsdPairSide = 16, kPsdPairWarps = 2;
+__global__ void __launch_bounds__(32 * kPsdPairWarps)
+    k_psd_update_pairs(ConeSet cs, const double *__restrict__ s, const double *__restrict__ z,
+                       int *scale_ok) {
+  extern __shared__ double sm_psd[];
+  const int nm = cs.psd_nmax, nn = nm * nm, nb = nm * (nm | 1);
+  const int lane = threadIdx.x & 31, c8 = lane & 7, q4 = lane >> 3;
+  double *M = sm_psd + (size_t)(threadIdx.x >> 5) * 8 * (2 * nb + 2 * nm) + c8;
+  double *V = M + 8 * nb, *S = V + 8 * nb;
+  int *perm = reinterpret_cast<int *>(S - c8 + 8 * nm) + c8;
+  const int c = (blockIdx.x * kPsdPairWarps + (threadIdx.x >> 5)) * 8 + c8;
+  int n = 0, off = 0, inst = -1;
+  if (c < cs.n_psd) {
+    inst = cs.psd_inst[c];
+    off = cs.psd_off[c];
+    if (active_inst(cs, inst)) n = cs.psd_n[c];
+  }
+  const int ld = n | 1;  // odd: the four lanes of a cone meet different banks
+  // s, z into the lower triangles of M and V, and their Cholesky factors (one
+  // lane per matrix)
+  for (int j = q4; j < n; j += 4) {
+    const double is2 = 0.70710678118654752440;
+    const double *sp = s + off + j * (j + 1) / 2, *zp = z + off + j * (j + 1) / 2;
+    for (int i = 0; i <= j; ++i) {
+      const double f = i == j ? 1.0 : is2;
+      M[8 * (j + ld * i)] = sp[i] * f;
+      V[8 * (j + ld * i)] = zp[i] * f;
+    }
+  }
+  __syncwarp();
+  bool ok = true;
+  if (q4 < 2) {
+    double *A = q4 == 0 ? M : V;
+    for (int j = 0; j < n; ++j) {
+      double d = A[8 * (j + ld * j)];
+      for (int k = 0; k < j; ++k) d -= A[8 * (j + ld * k)] * A[8 * (j + ld * k)];
+      if (!(d > 0)) ok = false;
+      d = ok ? sqrt(d) : 1.0;
+      for (int i = j + 1; i < n; ++i) {
+        double t = A[8 * (i + ld * j)];
+        for (int k = 0; k < j; ++k) t -= A[8 * (i + ld * k)] * A[8 * (j + ld * k)];
+        A[8 * (i + ld * j)] = t / d;
+      }
+      A[8 * (j + ld * j)] = d;
+    }
+  }
+  const unsigned bad = __ballot_sync(0xffffffffu, !ok);
+  if (bad & (0x01010101u << c8)) {
+    if (q4 == 0 && n > 0) scale_ok[inst] = 0;
+    n = 0;  // this cone is done
+  }
+  int nw = n;
+  for (int o = 4; o > 0; o >>= 1) nw = max(nw, __shfl_xor_sync(0xffffffffu, nw, o));
+  // L1 kept in R's place, L2 transposed in Rinv's (row i of L1 and row j of L2
+  // are read back by the lane that overwrites them); M = L2' L1, column by
+  // column in place of L1's
+  double *R = cs.psd_R + (size_t)min(c, cs.n_psd - 1) * nn;
+  double *Ri = cs.psd_Rinv + (size_t)min(c, cs.n_psd - 1) * nn;
+  double row[kPsdPairSide];
+  for (int j = q4; j < n; j += 4) {
+#pragma unroll
+    for (int k = 0; k < kPsdPairSide; ++k) {
+      row[k] = k >= j && k < n ? M[8 * (k + ld * j)] : 0.0;
+      if (k >= j && k < n) {
+        R[k + n * j] = row[k];
+        Ri[j + n * k] = V[8 * (k + ld * j)];
+      }
+    }
+    for (int i = 0; i < n; ++i) {
+      double t = 0;
+#pragma unroll
+      for (int k = 0; k < kPsdPairSide; ++k)
+        if (k >= i && k >= j && k < n) t += V[8 * (k + ld * i)] * row[k];
+      M[8 * (i + ld * j)] = t;
+    }
+  }
+  __syncwarp();
+  for (int j = q4; j < n; j += 4)
+    for (int i = 0; i < n; ++i) V[8 * (i + ld * j)] = i == j ? 1.0 : 0.0;
+  __syncwarp();
+  for (int sweep = 0; sweep < 60; ++sweep) {
+    bool rotated = false;
+    for (int t = 1; t <= 2 * nw - 3; ++t) {
+      for (int p = max(0, t - n + 1) + q4; 2 * p < t && p < n; p += 4) {
+        double *Mp = M + 8 * ld * p, *Mq = M + 8 * ld * (t - p);
+        double a = 0, b = 0, gd = 0;
+        for (int r = 0; r < n; ++r) {
+          const double mp = Mp[8 * r], mq = Mq[8 * r];
+          a += mp * mp;
+          b += mq * mq;
+          gd += mp * mq;
+        }
+        // columns orthogonal to 1e-14 of their norms (see warp_svd)
+        if (fabs(gd) <= 1e-14 * sqrt(a * b) || gd == 0) continue;
+        rotated = true;
+        const double zeta = (b - a) / (2 * gd);
+        const double tt = (zeta >= 0 ? 1.0 : -1.0) / (fabs(zeta) + sqrt(1 + zeta * zeta));
+        const double co = 1 / sqrt(1 + tt * tt), sn = co * tt;
+        double *Vp = V + 8 * ld * p, *Vq = V + 8 * ld * (t - p);
+        for (int r = 0; r < n; ++r) {
+          const double mp = Mp[8 * r], mq = Mq[8 * r], vp = Vp[8 * r], vq = Vq[8 * r];
+          Mp[8 * r] = co * mp - sn * mq;
+          Mq[8 * r] = sn * mp + co * mq;
+          Vp[8 * r] = co * vp - sn * vq;
+          Vq[8 * r] = sn * vp + co * vq;
+        }
+      }
+      __syncwarp();
+    }
+    if (!__any_sync(0xffffffffu, rotated)) break;
+  }
+  // singular values in descending order, the columns of U
+  for (int j = q4; j < n; j += 4) {
+    double t = 0;
+    for (int k = 0; k < n; ++k) t += M[8 * (k + ld * j)] * M[8 * (k + ld * j)];
+    t = sqrt(t);
+    S[8 * j] = t;
+    for (int k = 0; k < n; ++k) M[8 * (k + ld * j)] = t > 0 ? M[8 * (k + ld * j)] / t : 0.0;
+  }
+  __syncwarp();
+  if (q4 == 0) {
+    for (int i = 0; i < n; ++i) perm[8 * i] = i;
+    for (int i = 0; i < n; ++i)
+      for (int j = i + 1; j < n; ++j) {
+        const int pi = perm[8 * i], pj = perm[8 * j];
+        if (S[8 * pj] > S[8 * pi]) {
+          perm[8 * i] = pj;
+          perm[8 * j] = pi;
+        }
+      }
+  }
+  __syncwarp();
+  // R = L1 V Lis (row i), Rinv = Lis U' L2' (column j = row j of L2)
+  double *lam = cs.psd_lam + (size_t)min(c, cs.n_psd - 1) * nm;
+  for (int i = q4; i < n; i += 4) {
+#pragma unroll
+    for (int k = 0; k < kPsdPairSide; ++k) row[k] = k <= i ? R[i + n * k] : 0.0;
+    for (int j = 0; j < n; ++j) {
+      const int pj = perm[8 * j];
+      double t = 0;
+#pragma unroll
+      for (int k = 0; k < kPsdPairSide; ++k)
+        if (k <= i) t += row[k] * V[8 * (k + ld * pj)];
+      R[i + n * j] = t * (1.0 / sqrt(S[8 * pj]));
+    }
+#pragma unroll
+    for (int k = 0; k < kPsdPairSide; ++k) row[k] = k <= i ? Ri[k + n * i] : 0.0;
+    for (int j = 0; j < n; ++j) {
+      const int pj = perm[8 * j];
+      double t = 0;
+#pragma unroll
+      for (int k = 0; k < kPsdPairSide; ++k)
+        if (k <= i) t += M[8 * (k + ld * pj)] * row[k];
+      Ri[j + n * i] = (1.0 / sqrt(S[8 * pj])) * t;
+    }
+    lam[i] = S[8 * perm[8 * i]];
+  }
+}
+
 // y = a*op(Rx)... helper: Y = Rx' X Rx (trans=false) or Rx X Rx' (trans=true)
 __device__ void psd_wmul(int n, const double *Rx, bool trans, const double *X, double *Y,
                          double *T, const PsdGrp &g) {
@@ -1468,6 +1637,134 @@ __global__ void k_psd_step(ConeSet cs, const double *__restrict__ dz,
     res = fmin(res, a);
   }
   if (p.lane == 0) atomic_min_nonneg_filtered(alpha + p.inst, res);
+}
+// The two halves of it for sides up to kPsdPairSide: the matrices Lis (W dz)
+// Lis and Lis (W^{-T} ds) Lis into cs.psd_eig (packed lower triangles, two per
+// cone), then their smallest eigenvalues, one thread per matrix: Householder
+// tridiagonalisation (Martin, Reinsch and Wilkinson 1968), then Laguerre's
+// method for the one eigenvalue that is wanted.  A thread works alone on some
+// 8 k instructions; the cyclic Jacobi of a 16-lane group it replaces took 45
+// rotations per sweep with three barriers each (2.89 ms for 40 000 10 x 10
+// cones; now 0.33 ms in the two kernels).
+__global__ void k_psd_step_matrices(ConeSet cs, const double *__restrict__ dz,
+                                    const double *__restrict__ ds) {
+  PsdCtx p = psd_ctx(cs);
+  if (!p.valid) return;
+  int n = p.n, nm = cs.psd_nmax, nn = nm * nm;
+  double *X = psd_smem(nm, 3), *Y = X + nn, *T = Y + nn;
+  const double *R = cs.psd_R + (size_t)p.c * nn, *Ri = cs.psd_Rinv + (size_t)p.c * nn;
+  const double *lam = cs.psd_lam + (size_t)p.c * nm;
+  const double li = p.lane < n ? 1.0 / sqrt(lam[p.lane]) : 0.0;
+  for (int side = 0; side < 2; ++side) {
+    svec_to_mat(n, (side == 0 ? dz : ds) + p.off, X, p.g);
+    p.g.sync();
+    if (side == 0)
+      psd_wmul(n, R, false, X, Y, T, p.g);  // W dz = R' dZ R
+    else
+      psd_wmul(n, Ri, true, X, Y, T, p.g);  // W^{-T} ds = Ri dS Ri'
+    // the symmetric part (the reference's svec round trip), scaled
+    double *out = cs.psd_eig + (size_t)(2 * p.c + side) * (nm * (nm + 1) / 2);
+    for (int j = 0; j < n; ++j) {
+      const double lj = __shfl_sync(p.g.mask, li, j, p.g.G);
+      const int i = p.lane;
+      if (i >= j && i < n) {
+        const double is2 = 0.70710678118654752440;
+        const double v = i == j ? Y[i + n * j] : ((Y[i + n * j] + Y[j + n * i]) * is2) * is2;
+        out[i * (i + 1) / 2 + j] = v * (li * lj);
+      }
+    }
+    p.g.sync();
+  }
+}
+constexpr int kPsdEigThreads = 32;
+__global__ void __launch_bounds__(kPsdEigThreads) k_psd_step_eig(ConeSet cs, double *alpha) {
+  extern __shared__ double sm_psd[];
+  constexpr int W = kPsdEigThreads + 1;  // odd: the copy in below is free of conflicts
+  const int nm = cs.psd_nmax, tm = nm * (nm + 1) / 2, tid = threadIdx.x;
+  double *A = sm_psd + tid, *d = A + W * tm, *e = d + W * nm;  // element k at [W k]
+  const int first = blockIdx.x * kPsdEigThreads, m = min(kPsdEigThreads, 2 * cs.n_psd - first);
+  const double *src = cs.psd_eig + (size_t)first * tm;
+  for (int i = tid; i < m * tm; i += kPsdEigThreads) sm_psd[W * (i % tm) + i / tm] = src[i];
+  __syncwarp();
+  if (tid >= m) return;
+  const int c = (first + tid) >> 1, inst = cs.psd_inst[c];
+  if (!active_inst(cs, inst)) return;
+  const int n = cs.psd_n[c];
+  // tridiagonal form: diagonal d, subdiagonal e[1 .. n - 1]
+  for (int i = n - 1; i > 0; --i) {
+    double *Ai = A + W * (i * (i + 1) / 2);
+    const int l = i - 1;
+    double h = 0;
+    for (int k = 0; k < l; ++k) h += Ai[W * k] * Ai[W * k];
+    const double f = Ai[W * l];
+    if (h == 0) {  // already tridiagonal here
+      e[W * i] = f;
+      continue;
+    }
+    h += f * f;
+    const double g = f >= 0 ? -sqrt(h) : sqrt(h);
+    e[W * i] = g;
+    h -= f * g;
+    Ai[W * l] = f - g;
+    const double hi = 1.0 / h;
+    double ff = 0;
+    for (int j = 0; j <= l; ++j) {
+      const double *Aj = A + W * (j * (j + 1) / 2);
+      double t = 0;
+      for (int k = 0; k <= j; ++k) t += Aj[W * k] * Ai[W * k];
+      for (int k = j + 1; k <= l; ++k) t += A[W * (k * (k + 1) / 2 + j)] * Ai[W * k];
+      t *= hi;
+      d[W * j] = t;
+      ff += t * Ai[W * j];
+    }
+    const double hh = 0.5 * ff * hi;
+    for (int j = 0; j <= l; ++j) {
+      double *Aj = A + W * (j * (j + 1) / 2);
+      const double fj = Ai[W * j], gj = d[W * j] - hh * fj;
+      d[W * j] = gj;
+      for (int k = 0; k <= j; ++k) Aj[W * k] -= fj * d[W * k] + gj * Ai[W * k];
+    }
+  }
+  for (int i = 0; i < n; ++i) d[W * i] = A[W * (i * (i + 1) / 2 + i)];
+  double gmin = d[0];
+  if (n > 1) {
+    // Laguerre's iteration on det(T - x I) from Gershgorin's lower bound: the
+    // roots are real, so x rises to the smallest one monotonically.  With the
+    // pivots q of T - x I, G = sum 1 / (lambda - x) is the sum of the g = -q'/q
+    // and H = sum 1 / (lambda - x)^2 that of the h = g'; no term is negative.
+    // A pivot that is not positive: x has arrived, to the rounding of T.
+    double x = CUDART_INF, norm = 0;
+    for (int i = 0; i < n; ++i) {
+      const double r =
+          (i > 0 ? fabs(e[W * i]) : 0.0) + (i + 1 < n ? fabs(e[W * (i + 1)]) : 0.0);
+      x = fmin(x, d[W * i] - r);
+      if (!(fabs(d[W * i]) + r <= norm)) norm = fabs(d[W * i]) + r;
+      if (!isfinite(norm)) return;  // no eigenvalue to limit the step by
+    }
+    x -= kDEps * norm;
+    for (int it = 0; it < 100; ++it) {
+      double G = 0, H = 0, qi = 0, g = 0, h = 0;
+      bool pos = true;
+      for (int i = 0; i < n && pos; ++i) {
+        const double t = i > 0 ? e[W * i] * e[W * i] * qi : 0.0;
+        const double q = d[W * i] - x - t;
+        pos = q > 0;
+        qi = 1.0 / q;
+        const double g2 = g * g + h;
+        g = (1.0 + t * g) * qi;
+        h = g * g + t * g2 * qi;
+        G += g;
+        H += h;
+      }
+      if (!pos) break;
+      const double nx = x + n / (G + sqrt(fmax((n - 1) * (n * H - G * G), 0.0)));
+      if (!(nx - x > 0.25 * kDEps * norm)) break;
+      x = nx;
+    }
+    gmin = x;
+  }
+  const double amax = alpha[inst];
+  if (gmin < 0) atomic_min_nonneg_filtered(alpha + inst, fmin(1.0 / (-gmin), amax));
 }
 // coneops_nonsymmetric_common.jl:5-34 backtracking, per cone
 template <class Ops>
@@ -2293,6 +2590,15 @@ static inline void psd_launch_dims(const ConeSet &cs, int nmats, int &nb, int &n
     }                                                                                  \
   } while (0)
 
+// sides up to kPsdPairSide take the pair-per-lane scaling and the
+// thread-per-matrix step length: at 16 their matrices still leave three blocks
+// per SM and a row fits in registers; above, the group kernels' 32 lanes are
+// filled by one column (side 8, 96 cones: scaling 231 us by groups, 92 by
+// pairs, step 217 against 46; side 10, 40 000 cones: 3866 against 655 and 2892
+// against 329)
+static inline bool psd_small(const ConeSet &cs) {
+  return cs.n_psd > 0 && cs.psd_nmax <= kPsdPairSide;
+}
 static NonsymArgs<ExpOps> exp_args(const ConeSet &cs) {
   return NonsymArgs<ExpOps>{cs.n_exp, cs.exp_begin, cs.exp_inst, nullptr,
                             cs.exp_Hd, cs.exp_Hs, cs.exp_grad, cs.exp_z};
@@ -2314,7 +2620,18 @@ void cones_update_scaling(const ConeSet &cs, const double *s, const double *z,
   if (cs.n_pow)
     k_nonsym_update_scaling<PowOps><<<blocks_for(cs.n_pow, 128), 128, 0, st>>>(
         cs, pow_args(cs), s, z, mu, scaling);
-  LAUNCH_PSD(k_psd_update_scaling, 7, cs, s, z, scale_ok);
+  if (psd_small(cs)) {
+    const size_t sm = (size_t)kPsdPairWarps * 8 * (2 * cs.psd_nmax * (cs.psd_nmax | 1) +
+                                                   2 * cs.psd_nmax) * sizeof(double);
+    static const bool attr = cudaFuncSetAttribute(k_psd_update_pairs,
+                                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                  96 * 1024) == cudaSuccess;
+    (void)attr;
+    k_psd_update_pairs<<<blocks_for(cs.n_psd, 8 * kPsdPairWarps), 32 * kPsdPairWarps, sm, st>>>(
+        cs, s, z, scale_ok);
+  } else {
+    LAUNCH_PSD(k_psd_update_scaling, 7, cs, s, z, scale_ok);
+  }
 }
 
 void cones_refresh_kkt(const ConeSet &cs, const KKTMapDev &map, double *kv,
@@ -2404,7 +2721,15 @@ void cones_step_length_sym(const ConeSet &cs, const double *dz, const double *ds
     k_nn_step<<<blocks_for(cs.n_nn, nn_block(cs) * (cs.B == 1 ? kNNRows : 1)), nn_block(cs), 0,
                 st>>>(cs, dz, ds, z, s, alpha);
   LAUNCH_SOC_SHAPED(kSocStep, k_soc_tile_step, 4, k_soc_step, dz, ds, z, s, alpha);
-  LAUNCH_PSD(k_psd_step, 4, cs, dz, ds, alpha);
+  if (psd_small(cs)) {
+    LAUNCH_PSD(k_psd_step_matrices, 3, cs, dz, ds);
+    const size_t sm = (size_t)(kPsdEigThreads + 1) * (cs.psd_nmax * (cs.psd_nmax + 1) / 2 +
+                                                2 * cs.psd_nmax) * sizeof(double);
+    k_psd_step_eig<<<blocks_for(2 * cs.n_psd, kPsdEigThreads), kPsdEigThreads, sm, st>>>(cs,
+                                                                                      alpha);
+  } else {
+    LAUNCH_PSD(k_psd_step, 4, cs, dz, ds, alpha);
+  }
 }
 
 void cones_step_length_asym(const ConeSet &cs, const double *dz, const double *ds,

@@ -184,6 +184,7 @@ extern "C" int clgpu_cones_create(int ncones, const int *types, const int *dims,
   cs.psd_R = A.alloc<double>(nn2 * cs.n_psd);
   cs.psd_Rinv = A.alloc<double>(nn2 * cs.n_psd);
   cs.psd_lam = A.alloc<double>((size_t)psd_max * cs.n_psd);
+  cs.psd_eig = A.alloc<double>((size_t)psd_max * (psd_max + 1) * cs.n_psd);
   cs.cone_tmp = A.alloc<double>((size_t)cs.n_soc + cs.n_exp + cs.n_pow + cs.n_psd);
   cs.cone_tmp2 = A.alloc<double>((size_t)cs.n_soc + cs.n_exp + cs.n_pow + cs.n_psd);
   {

@@ -1346,6 +1346,7 @@ static int build_batch(clgpu_solver *h, std::vector<Prepared> &prep, int nth) {
   cs.psd_R = A.alloc<double>(nn2 * cs.n_psd);
   cs.psd_Rinv = A.alloc<double>(nn2 * cs.n_psd);
   cs.psd_lam = A.alloc<double>((size_t)cs.psd_nmax * cs.n_psd);
+  cs.psd_eig = A.alloc<double>((size_t)cs.psd_nmax * (cs.psd_nmax + 1) * cs.n_psd);
   cs.cone_tmp = A.alloc<double>((size_t)cs.n_soc + cs.n_exp + cs.n_pow + cs.n_psd);
   cs.cone_tmp2 = A.alloc<double>((size_t)cs.n_soc + cs.n_exp + cs.n_pow + cs.n_psd);
   mark("data + cones");

@@ -1,0 +1,102 @@
+"""PSD scaling and step length on both sides of the side limit (16) of the
+kernels that give a lane a rotation and a thread a matrix: sides at the edges,
+cone counts that do not fill a warp (8) or a block, and matrices with repeated
+or zero eigenvalues, against the oracle.  Tolerances are those of
+test_gpu_cones.py: FP64 arithmetic with condition numbers below about 1e2."""
+import ctypes
+
+import numpy as np
+import pytest
+
+import oracle
+from test_gpu_cones import GPUCones, close
+
+pytestmark = pytest.mark.gpu
+
+SIDES = {"one": [1], "two": [2] * 3, "three": [3] * 9, "ten": [10] * 17, "fifteen": [15] * 5,
+         "sixteen": [16] * 35, "seventeen": [17] * 3, "mixed": [1, 16, 7, 2, 15, 10, 8, 3, 5] * 4,
+         "mixed_large": [1, 16, 17, 2, 9]}
+
+
+def interior(rng, n):
+    A = rng.standard_normal((n, n))
+    M = 0.5 * np.eye(n) + A @ A.T / n
+    return np.array([M[i, j] if i == j else M[i, j] * np.sqrt(2)
+                     for j in range(n) for i in range(j + 1)])
+
+
+def svec_eye(sides, value):
+    return np.concatenate([[value if i == j else 0.0 for j in range(n) for i in range(j + 1)]
+                           for n in sides])
+
+
+@pytest.mark.parametrize("name", list(SIDES))
+def test_psd_sides(cuda_device, name):
+    sides = SIDES[name]
+    specs = [(5, n, 0.0) for n in sides]
+    rng = np.random.default_rng(len(sides))
+    s = np.concatenate([interior(rng, n) for n in sides])
+    z = np.concatenate([interior(rng, n) for n in sides])
+    C, G = oracle.Cones(specs), GPUCones(specs)
+    d_s, d_z = G.dev(s), G.dev(z)
+    assert C.update_scaling(s, z, 1.0, 0) == 0
+    assert G.L.clgpu_update_scaling(G.h, d_s.data_ptr(), d_z.data_ptr(), 1.0, 0, None) == 0
+    hs = G.empty(G.hs_len)
+    assert G.L.clgpu_get_Hs(G.h, hs.data_ptr(), None) == 0
+    assert close(hs.cpu().numpy()[:C.hs_len], C.get_Hs(), 1e-11)
+    out = G.empty(C.numel)
+    stz, sts = rng.standard_normal(C.numel) * 0.1, rng.standard_normal(C.numel) * 0.1
+    d_stz, d_sts = G.dev(stz), G.dev(sts)
+    assert G.L.clgpu_combined_ds_shift(G.h, out.data_ptr(), d_stz.data_ptr(),
+                                       d_sts.data_ptr(), d_z.data_ptr(), 0.37, None) == 0
+    assert close(out.cpu().numpy(), C.combined_ds_shift(stz, sts, z, 0.37), 1e-10)
+    steps = [(rng.standard_normal(C.numel) * k, rng.standard_normal(C.numel) * k)
+             for k in (0.5, 2.0, 1e-3)]
+    steps.append((-2.0 * s, svec_eye(sides, 0.5)))  # direction along s: clustered eigenvalues
+    steps.append((np.zeros(C.numel), -3.0 * z))
+    steps.append((np.zeros(C.numel), np.zeros(C.numel)))
+    for dz, ds in steps:
+        ref = C.step_length(dz, ds, z, s, 1.0)
+        a = ctypes.c_double()
+        d_dz, d_ds = G.dev(dz), G.dev(ds)
+        assert G.L.clgpu_step_length(G.h, d_dz.data_ptr(), d_ds.data_ptr(), d_z.data_ptr(),
+                                     d_s.data_ptr(), 1.0, 0.99, 0.8, 1e-4, ctypes.byref(a),
+                                     None) == 0
+        assert abs(a.value - ref) <= 1e-10 * max(1.0, ref), (a.value, ref)
+
+
+@pytest.mark.parametrize("n", [1, 8, 16])
+def test_psd_repeated_eigenvalues(cuda_device, n):
+    """s = z = I: the scaling is the identity and every eigenvalue of the step's
+    matrix is the same, or all but one are."""
+    specs = [(5, n, 0.0)] * 3
+    s = svec_eye([n] * 3, 1.0)
+    C, G = oracle.Cones(specs), GPUCones(specs)
+    d_s = G.dev(s)
+    assert C.update_scaling(s, s, 1.0, 0) == 0
+    assert G.L.clgpu_update_scaling(G.h, d_s.data_ptr(), d_s.data_ptr(), 1.0, 0, None) == 0
+    v = np.ones(n) / np.sqrt(n)
+    rank1 = -4.0 * np.outer(v, v)
+    m = n * (n + 1) // 2
+    low = np.array([rank1[i, j] * (1.0 if i == j else np.sqrt(2))
+                    for j in range(n) for i in range(j + 1)])
+    for ds in (-4.0 * s, np.concatenate([low, 0 * low, -low]), np.concatenate([-s[:2 * m], low])):
+        a = ctypes.c_double()
+        d_ds = G.dev(ds)
+        assert G.L.clgpu_step_length(G.h, d_ds.data_ptr(), d_ds.data_ptr(), d_s.data_ptr(),
+                                     d_s.data_ptr(), 1.0, 0.99, 0.8, 1e-4, ctypes.byref(a),
+                                     None) == 0
+        ref = C.step_length(ds, ds, s, s, 1.0)
+        assert abs(a.value - ref) <= 1e-12 * n, (a.value, ref)
+
+
+def test_psd_scaling_failure_small_side(cuda_device):
+    specs = [(5, 4, 0.0)] * 9
+    s = svec_eye([4] * 9, 1.0)
+    bad = s.copy()
+    bad[7 * 10] = -1.0
+    G = GPUCones(specs)
+    d_s, d_b = G.dev(s), G.dev(bad)
+    assert G.L.clgpu_update_scaling(G.h, d_s.data_ptr(), d_s.data_ptr(), 1.0, 0, None) == 0
+    assert G.L.clgpu_update_scaling(G.h, d_b.data_ptr(), d_s.data_ptr(), 1.0, 0, None) != 0
+    assert G.L.clgpu_update_scaling(G.h, d_s.data_ptr(), d_b.data_ptr(), 1.0, 0, None) != 0
