@@ -604,7 +604,7 @@ __device__ __forceinline__ void svec_to_mat(int n, const double *x, double *M, c
   const double is2 = 0.70710678118654752440;  // 1/sqrt(2)
   int t = n * (n + 1) / 2;
   for (int k = g.lane; k < t; k += g.G) {
-    int col = (int)((sqrt(8.0 * k + 1.0) - 1.0) * 0.5);
+    int col = (int)((sqrtf(8.0f * k + 1.0f) - 1.0f) * 0.5f);
     while ((col + 1) * (col + 2) / 2 <= k) ++col;
     while (col * (col + 1) / 2 > k) --col;
     int row = k - col * (col + 1) / 2;
@@ -621,7 +621,7 @@ __device__ __forceinline__ void mat_to_svec(int n, const double *M, double *x, c
   const double is2 = 0.70710678118654752440;
   int t = n * (n + 1) / 2;
   for (int k = g.lane; k < t; k += g.G) {
-    int col = (int)((sqrt(8.0 * k + 1.0) - 1.0) * 0.5);
+    int col = (int)((sqrtf(8.0f * k + 1.0f) - 1.0f) * 0.5f);
     while ((col + 1) * (col + 2) / 2 <= k) ++col;
     while (col * (col + 1) / 2 > k) --col;
     int row = k - col * (col + 1) / 2;
@@ -889,14 +889,14 @@ __global__ void k_psd_update_scaling(ConeSet cs, const double *__restrict__ s,
 // steps.  (One cone per 16 lanes, one pair at a time, spent its time in the
 // exchanges of three 16-lane sums per pair and repeated each rotation's
 // division and square roots on all lanes: 79 k warp instructions per 10 x 10
-// cone, 3.87 ms for 40 000; now 0.65 ms.)  Matrices are interleaved over
+// cone, 3.87 ms for 40 000; now 0.60 ms.)  Matrices are interleaved over
 // the warp's cones, so lanes of one step read neighbouring words.
 constexpr int kPsdPairSide = 16, kPsdPairWarps = 2;
 __global__ void __launch_bounds__(32 * kPsdPairWarps)
     k_psd_update_pairs(ConeSet cs, const double *__restrict__ s, const double *__restrict__ z,
                        int *scale_ok) {
   extern __shared__ double sm_psd[];
-  const int nm = cs.psd_nmax, nn = nm * nm, nb = nm * (nm | 1);
+  const int nm = cs.psd_nmax, nn = nm * nm, nb = nm * (nm + 1 + (nm & 1));
   const int lane = threadIdx.x & 31, c8 = lane & 7, q4 = lane >> 3;
   double *M = sm_psd + (size_t)(threadIdx.x >> 5) * 8 * (2 * nb + 2 * nm) + c8;
   double *V = M + 8 * nb, *S = V + 8 * nb;
@@ -908,7 +908,11 @@ __global__ void __launch_bounds__(32 * kPsdPairWarps)
     off = cs.psd_off[c];
     if (active_inst(cs, inst)) n = cs.psd_n[c];
   }
-  const int ld = n | 1;  // odd: the four lanes of a cone meet different banks
+  // odd, so that the four lanes of a cone meet different banks, and with room
+  // for the row of zeros
+  const int ld = n + 1 + (n & 1);
+  if (n & 1)
+    for (int j = q4; j < n; j += 4) M[8 * (n + ld * j)] = V[8 * (n + ld * j)] = 0.0;
   // s, z into the lower triangles of M and V, and their Cholesky factors (one
   // lane per matrix)
   for (int j = q4; j < n; j += 4) {
@@ -976,27 +980,41 @@ __global__ void __launch_bounds__(32 * kPsdPairWarps)
     for (int t = 1; t <= 2 * nw - 3; ++t) {
       for (int p = max(0, t - n + 1) + q4; 2 * p < t && p < n; p += 4) {
         double *Mp = M + 8 * ld * p, *Mq = M + 8 * ld * (t - p);
-        double a = 0, b = 0, gd = 0;
-        for (int r = 0; r < n; ++r) {
-          const double mp = Mp[8 * r], mq = Mq[8 * r];
-          a += mp * mp;
-          b += mq * mq;
-          gd += mp * mq;
-        }
+        double mp[kPsdPairSide], mq[kPsdPairSide], a = 0, b = 0, gd = 0;
+#pragma unroll
+        for (int r = 0; r < kPsdPairSide; r += 2)
+          if (r < n) {  // (a row of zeros follows an odd n)
+            mp[r] = Mp[8 * r];
+            mq[r] = Mq[8 * r];
+            mp[r + 1] = Mp[8 * r + 8];
+            mq[r + 1] = Mq[8 * r + 8];
+            a += mp[r] * mp[r];
+            b += mq[r] * mq[r];
+            gd += mp[r] * mq[r];
+            a += mp[r + 1] * mp[r + 1];
+            b += mq[r + 1] * mq[r + 1];
+            gd += mp[r + 1] * mq[r + 1];
+          }
         // columns orthogonal to 1e-14 of their norms (see warp_svd)
         if (fabs(gd) <= 1e-14 * sqrt(a * b) || gd == 0) continue;
         rotated = true;
         const double zeta = (b - a) / (2 * gd);
         const double tt = (zeta >= 0 ? 1.0 : -1.0) / (fabs(zeta) + sqrt(1 + zeta * zeta));
-        const double co = 1 / sqrt(1 + tt * tt), sn = co * tt;
+        const double co = rsqrt(1 + tt * tt), sn = co * tt;
         double *Vp = V + 8 * ld * p, *Vq = V + 8 * ld * (t - p);
-        for (int r = 0; r < n; ++r) {
-          const double mp = Mp[8 * r], mq = Mq[8 * r], vp = Vp[8 * r], vq = Vq[8 * r];
-          Mp[8 * r] = co * mp - sn * mq;
-          Mq[8 * r] = sn * mp + co * mq;
-          Vp[8 * r] = co * vp - sn * vq;
-          Vq[8 * r] = sn * vp + co * vq;
-        }
+#pragma unroll
+        for (int r = 0; r < kPsdPairSide; r += 2)
+          if (r < n) {
+            const double v0 = Vp[8 * r], w0 = Vq[8 * r], v1 = Vp[8 * r + 8], w1 = Vq[8 * r + 8];
+            Mp[8 * r] = co * mp[r] - sn * mq[r];
+            Mq[8 * r] = sn * mp[r] + co * mq[r];
+            Mp[8 * r + 8] = co * mp[r + 1] - sn * mq[r + 1];
+            Mq[8 * r + 8] = sn * mp[r + 1] + co * mq[r + 1];
+            Vp[8 * r] = co * v0 - sn * w0;
+            Vq[8 * r] = sn * v0 + co * w0;
+            Vp[8 * r + 8] = co * v1 - sn * w1;
+            Vq[8 * r + 8] = sn * v1 + co * w1;
+          }
       }
       __syncwarp();
     }
@@ -1088,7 +1106,7 @@ __device__ __forceinline__ double skron_entry(const double *A, int n, int i, int
   return Ajl * Ajl;
 }
 __device__ __forceinline__ void tri_coord(int k, int &row, int &col) {
-  col = (int)((sqrt(8.0 * k + 1.0) - 1.0) * 0.5);
+  col = (int)((sqrtf(8.0f * k + 1.0f) - 1.0f) * 0.5f);  // a guess, made exact below
   while ((col + 1) * (col + 2) / 2 <= k) ++col;
   while (col * (col + 1) / 2 > k) --col;
   row = k - col * (col + 1) / 2;
@@ -1645,37 +1663,7 @@ __global__ void k_psd_step(ConeSet cs, const double *__restrict__ dz,
 // method for the one eigenvalue that is wanted.  A thread works alone on some
 // 8 k instructions; the cyclic Jacobi of a 16-lane group it replaces took 45
 // rotations per sweep with three barriers each (2.89 ms for 40 000 10 x 10
-// cones; now 0.33 ms in the two kernels).
-__global__ void k_psd_step_matrices(ConeSet cs, const double *__restrict__ dz,
-                                    const double *__restrict__ ds) {
-  PsdCtx p = psd_ctx(cs);
-  if (!p.valid) return;
-  int n = p.n, nm = cs.psd_nmax, nn = nm * nm;
-  double *X = psd_smem(nm, 3), *Y = X + nn, *T = Y + nn;
-  const double *R = cs.psd_R + (size_t)p.c * nn, *Ri = cs.psd_Rinv + (size_t)p.c * nn;
-  const double *lam = cs.psd_lam + (size_t)p.c * nm;
-  const double li = p.lane < n ? 1.0 / sqrt(lam[p.lane]) : 0.0;
-  for (int side = 0; side < 2; ++side) {
-    svec_to_mat(n, (side == 0 ? dz : ds) + p.off, X, p.g);
-    p.g.sync();
-    if (side == 0)
-      psd_wmul(n, R, false, X, Y, T, p.g);  // W dz = R' dZ R
-    else
-      psd_wmul(n, Ri, true, X, Y, T, p.g);  // W^{-T} ds = Ri dS Ri'
-    // the symmetric part (the reference's svec round trip), scaled
-    double *out = cs.psd_eig + (size_t)(2 * p.c + side) * (nm * (nm + 1) / 2);
-    for (int j = 0; j < n; ++j) {
-      const double lj = __shfl_sync(p.g.mask, li, j, p.g.G);
-      const int i = p.lane;
-      if (i >= j && i < n) {
-        const double is2 = 0.70710678118654752440;
-        const double v = i == j ? Y[i + n * j] : ((Y[i + n * j] + Y[j + n * i]) * is2) * is2;
-        out[i * (i + 1) / 2 + j] = v * (li * lj);
-      }
-    }
-    p.g.sync();
-  }
-}
+// cones; now 0.24 ms in the two kernels).
 constexpr int kPsdEigThreads = 32;
 __global__ void __launch_bounds__(kPsdEigThreads) k_psd_step_eig(ConeSet cs, double *alpha) {
   extern __shared__ double sm_psd[];
@@ -1765,6 +1753,238 @@ __global__ void __launch_bounds__(kPsdEigThreads) k_psd_step_eig(ConeSet cs, dou
   }
   const double amax = alpha[inst];
   if (gmin < 0) atomic_min_nonneg_filtered(alpha + inst, fmin(1.0 / (-gmin), amax));
+}
+
+// -- congruences op(R)' X op(R) for sides up to kPsdPairSide, 16 lanes per cone:
+// lane i keeps column i of op(R) and of X op(R) in registers, X (packed, one
+// read for both halves) and R come from shared memory as broadcasts, so a
+// product is one shared read per multiply-add and needs no barrier or index
+// division.  Loops are unrolled to the limit and cut off in pairs at n; R and X
+// carry one row and column of zeros when n is odd.  40 000 cones of side 10,
+// before and after (the element-per-lane products with n^2 / 16 divisions):
+// combined
+// shift 260 -> 189 us, step matrices 230 -> 140, H x 154 -> 104, offset 110 -> 80;
+// what is left is instruction issue (2 900 per warp for two cones' H x).
+struct PsdSmall {
+  static constexpr int ld = kPsdPairSide + 1;  // odd, and the same for every n: the
+                                               // addresses are immediates
+  double *R, *X, *Y;
+  int lane;
+};
+constexpr int kPsdSmallWords =
+    2 * (kPsdPairSide + 1) * kPsdPairSide + (kPsdPairSide + 1) * kPsdPairSide / 2;
+__device__ __forceinline__ PsdSmall psd_small_ctx(const PsdCtx &p) {
+  extern __shared__ double smem[];
+  PsdSmall q;
+  q.R = smem + (threadIdx.x >> 4) * kPsdSmallWords;
+  q.Y = q.R + PsdSmall::ld * kPsdPairSide;
+  q.X = q.Y + PsdSmall::ld * kPsdPairSide;
+  q.lane = p.lane;
+  if ((p.n & 1) && p.lane <= p.n) {
+    q.R[p.n + q.ld * p.lane] = 0;
+    q.R[p.lane + q.ld * p.n] = 0;
+    q.X[p.n * (p.n + 1) / 2 + p.lane] = 0;
+  }
+  return q;
+}
+// (every load is issued before the first store)
+__device__ __forceinline__ void psd_load_R(const PsdSmall &q, int n,
+                                           const double *__restrict__ R) {
+  double v[kPsdPairSide];
+#pragma unroll
+  for (int j = 0; j < kPsdPairSide; ++j)
+    v[j] = j < n && q.lane < n ? R[q.lane + n * j] : 0.0;
+#pragma unroll
+  for (int j = 0; j < kPsdPairSide; ++j)
+    if (j < n && q.lane < n) q.R[q.lane + q.ld * j] = v[j];
+}
+__device__ __forceinline__ void psd_load_X(const PsdSmall &q, int n,
+                                           const double *__restrict__ x) {
+  const double is2 = 0.70710678118654752440;
+  double v[kPsdPairSide];
+#pragma unroll
+  for (int j = 0; j < kPsdPairSide; ++j)
+    v[j] = j < n && q.lane <= j ? x[j * (j + 1) / 2 + q.lane] : 0.0;
+#pragma unroll
+  for (int j = 0; j < kPsdPairSide; ++j)
+    if (j < n && q.lane <= j) q.X[j * (j + 1) / 2 + q.lane] = q.lane == j ? v[j] : v[j] * is2;
+}
+// y[j] = (op(R)' X op(R))(lane, j), op(R) = R' with tr
+template <bool tr>
+__device__ __forceinline__ void psd_congr(const PsdSmall &q, int n,
+                                          double (&y)[kPsdPairSide]) {
+  double r[kPsdPairSide], t[kPsdPairSide];
+  constexpr int si = tr ? 1 : PsdSmall::ld, sk = tr ? PsdSmall::ld : 1;  // strides of op(R)'s column, row
+#pragma unroll
+  for (int k = 0; k < kPsdPairSide; ++k)
+    r[k] = k < n && q.lane < n ? q.R[si * q.lane + sk * k] : 0.0;
+#pragma unroll
+  for (int k = 0; k < kPsdPairSide; k += 2) {
+    t[k] = t[k + 1] = 0;
+    if (k < n) {
+#pragma unroll
+      for (int l = 0; l < kPsdPairSide; l += 2)
+        if (l < n) {
+          const int a = l > k ? l : k, b = l > k ? k : l;  // the 2 x 2 block at (a, b)
+          const double x00 = q.X[a * (a + 1) / 2 + b], x10 = q.X[(a + 1) * (a + 2) / 2 + b],
+                       x11 = q.X[(a + 1) * (a + 2) / 2 + b + 1],
+                       x01 = l == k ? x10 : q.X[a * (a + 1) / 2 + b + 1];
+          // x(row, col) of the block: rows are a, a + 1; t's index runs over
+          // the rows if k is the larger one
+          t[k] += x00 * r[l];
+          t[k] += (l > k ? x10 : x01) * r[l + 1];
+          t[k + 1] += (l > k ? x01 : x10) * r[l];
+          t[k + 1] += x11 * r[l + 1];
+        }
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < kPsdPairSide; ++j) {
+    y[j] = 0;
+    if (j < n) {
+      double v = 0;
+#pragma unroll
+      for (int k = 0; k < kPsdPairSide; k += 2)
+        if (k < n) {
+          v += t[k] * q.R[si * j + sk * k];
+          v += t[k + 1] * q.R[si * j + sk * (k + 1)];
+        }
+      y[j] = v;
+    }
+  }
+}
+// y becomes the symmetric part of the matrix whose row `lane` it is (scaled
+// off the diagonal by both factors of the reference's svec round trip); Y is
+// written
+__device__ __forceinline__ void psd_symmetric(const PsdSmall &q, int n, const PsdGrp &g,
+                                              double (&y)[kPsdPairSide]) {
+  const double is2 = 0.70710678118654752440;
+#pragma unroll
+  for (int j = 0; j < kPsdPairSide; ++j)
+    if (j < n && q.lane < n) q.Y[q.lane + q.ld * j] = y[j];
+  g.sync();
+#pragma unroll
+  for (int j = 0; j < kPsdPairSide; ++j)
+    if (j < n && q.lane < n && j != q.lane)
+      y[j] = ((y[j] + q.Y[j + q.ld * q.lane]) * is2) * is2;
+  g.sync();
+}
+// svec of the matrix whose symmetric part's row `lane` is y; minus sub on the
+// diagonal
+__device__ __forceinline__ void psd_store(const PsdSmall &q, int n,
+                                          const double (&y)[kPsdPairSide], double sub,
+                                          double *out) {
+  const double sqrt2 = 1.4142135623730951;
+#pragma unroll
+  for (int j = 0; j < kPsdPairSide; ++j)
+    if (j < n && q.lane <= j)
+      out[j * (j + 1) / 2 + q.lane] = q.lane == j ? y[j] - sub : y[j] * sqrt2;
+}
+__global__ void k_psd_mul_hs_small(ConeSet cs, double *y, const double *__restrict__ x) {
+  PsdCtx p = psd_ctx(cs);
+  if (!p.valid) return;
+  const PsdSmall q = psd_small_ctx(p);
+  const int n = p.n;
+  double v[kPsdPairSide];
+  psd_load_R(q, n, cs.psd_R + (size_t)p.c * cs.psd_nmax * cs.psd_nmax);
+  psd_load_X(q, n, x + p.off);
+  p.g.sync();
+  psd_congr<false>(q, n, v);  // W x
+  psd_symmetric(q, n, p.g, v);
+#pragma unroll
+  for (int j = 0; j < kPsdPairSide; ++j)
+    if (j < n && q.lane <= j) q.X[j * (j + 1) / 2 + q.lane] = v[j];
+  p.g.sync();
+  psd_congr<true>(q, n, v);  // W^T W x
+  psd_symmetric(q, n, p.g, v);
+  psd_store(q, n, v, 0.0, y + p.off);
+}
+__global__ void k_psd_combined_small(ConeSet cs, double *shift, const double *__restrict__ dz,
+                                     const double *__restrict__ ds, const double *sm) {
+  PsdCtx p = psd_ctx(cs);
+  if (!p.valid) return;
+  const PsdSmall q = psd_small_ctx(p);
+  const int n = p.n;
+  const size_t rc = (size_t)p.c * cs.psd_nmax * cs.psd_nmax;
+  double a[kPsdPairSide], b[kPsdPairSide], c[kPsdPairSide];
+  psd_load_R(q, n, cs.psd_R + rc);
+  psd_load_X(q, n, dz + p.off);
+  p.g.sync();
+  psd_congr<false>(q, n, a);  // W dz
+  psd_symmetric(q, n, p.g, a);
+  psd_load_R(q, n, cs.psd_Rinv + rc);
+  psd_load_X(q, n, ds + p.off);
+  p.g.sync();
+  psd_congr<true>(q, n, b);  // W^{-T} ds
+  psd_symmetric(q, n, p.g, b);
+  // (A B + B A) / 2 from the rows in registers and in shared memory (R, Y)
+#pragma unroll
+  for (int j = 0; j < kPsdPairSide; ++j)
+    if (j < n && q.lane < n) {
+      q.R[q.lane + q.ld * j] = a[j];
+      q.Y[q.lane + q.ld * j] = b[j];
+    }
+  p.g.sync();
+#pragma unroll
+  for (int j = 0; j < kPsdPairSide; ++j) {
+    c[j] = 0;
+    if (j < n) {
+      double t = 0;
+#pragma unroll
+      for (int k = 0; k < kPsdPairSide; ++k)
+        if (k < n) t += b[k] * q.R[k + q.ld * j] + a[k] * q.Y[k + q.ld * j];
+      c[j] = 0.5 * t;
+    }
+  }
+  p.g.sync();
+  psd_symmetric(q, n, p.g, c);
+  psd_store(q, n, c, sm[p.inst], shift + p.off);
+}
+__global__ void k_psd_ds_offset_small(ConeSet cs, double *out, const double *__restrict__ ds) {
+  PsdCtx p = psd_ctx(cs);
+  if (!p.valid) return;
+  const PsdSmall q = psd_small_ctx(p);
+  const int n = p.n;
+  const double l = p.lane < n ? cs.psd_lam[(size_t)p.c * cs.psd_nmax + p.lane] : 1.0;
+  double v[kPsdPairSide];
+  psd_load_R(q, n, cs.psd_R + (size_t)p.c * cs.psd_nmax * cs.psd_nmax);
+  psd_load_X(q, n, ds + p.off);
+#pragma unroll
+  for (int j = 0; j < kPsdPairSide; ++j) {
+    const double lj = __shfl_sync(p.g.mask, l, j, 16);
+    if (j < n && q.lane <= j) q.X[j * (j + 1) / 2 + q.lane] *= 2 / (l + lj);
+  }
+  p.g.sync();
+  psd_congr<true>(q, n, v);  // R X R'
+  psd_symmetric(q, n, p.g, v);
+  psd_store(q, n, v, 0.0, out + p.off);
+}
+__global__ void k_psd_step_matrices(ConeSet cs, const double *__restrict__ dz,
+                                    const double *__restrict__ ds) {
+  PsdCtx p = psd_ctx(cs);
+  if (!p.valid) return;
+  const PsdSmall q = psd_small_ctx(p);
+  const int n = p.n, nm = cs.psd_nmax;
+  const double li = p.lane < n ? 1.0 / sqrt(cs.psd_lam[(size_t)p.c * nm + p.lane]) : 0.0;
+  double v[kPsdPairSide];
+#pragma unroll
+  for (int side = 0; side < 2; ++side) {
+    psd_load_R(q, n, (side == 0 ? cs.psd_R : cs.psd_Rinv) + (size_t)p.c * nm * nm);
+    psd_load_X(q, n, (side == 0 ? dz : ds) + p.off);
+    p.g.sync();
+    if (side == 0)
+      psd_congr<false>(q, n, v);  // W dz
+    else
+      psd_congr<true>(q, n, v);  // W^{-T} ds
+    psd_symmetric(q, n, p.g, v);
+    double *out = cs.psd_eig + (size_t)(2 * p.c + side) * (nm * (nm + 1) / 2);
+#pragma unroll
+    for (int j = 0; j < kPsdPairSide; ++j) {
+      const double lj = __shfl_sync(p.g.mask, li, j, 16);
+      if (j < n && q.lane <= j) out[j * (j + 1) / 2 + q.lane] = v[j] * (li * lj);
+    }
+    p.g.sync();
+  }
 }
 // coneops_nonsymmetric_common.jl:5-34 backtracking, per cone
 template <class Ops>
@@ -2590,12 +2810,17 @@ static inline void psd_launch_dims(const ConeSet &cs, int nmats, int &nb, int &n
     }                                                                                  \
   } while (0)
 
+// the congruence kernels: 16 lanes per cone, kPsdWarps warps per block
+#define LAUNCH_PSD_SMALL(KERNEL, ...)                                                  \
+  KERNEL<<<blocks_for(16LL * cs.n_psd, 32 * kPsdWarps), 32 * kPsdWarps,                \
+           2 * kPsdWarps * kPsdSmallWords * sizeof(double), st>>>(__VA_ARGS__)
+
 // sides up to kPsdPairSide take the pair-per-lane scaling and the
 // thread-per-matrix step length: at 16 their matrices still leave three blocks
 // per SM and a row fits in registers; above, the group kernels' 32 lanes are
-// filled by one column (side 8, 96 cones: scaling 231 us by groups, 92 by
-// pairs, step 217 against 46; side 10, 40 000 cones: 3866 against 655 and 2892
-// against 329)
+// filled by one column (side 8, 96 cones: scaling 231 us by groups, 85 by
+// pairs, step 217 against 45; side 10, 40 000 cones: 3866 against 601 and 2892
+// against 240)
 static inline bool psd_small(const ConeSet &cs) {
   return cs.n_psd > 0 && cs.psd_nmax <= kPsdPairSide;
 }
@@ -2621,8 +2846,9 @@ void cones_update_scaling(const ConeSet &cs, const double *s, const double *z,
     k_nonsym_update_scaling<PowOps><<<blocks_for(cs.n_pow, 128), 128, 0, st>>>(
         cs, pow_args(cs), s, z, mu, scaling);
   if (psd_small(cs)) {
-    const size_t sm = (size_t)kPsdPairWarps * 8 * (2 * cs.psd_nmax * (cs.psd_nmax | 1) +
-                                                   2 * cs.psd_nmax) * sizeof(double);
+    const size_t sm = (size_t)kPsdPairWarps * 8 * sizeof(double) *
+                      (2 * cs.psd_nmax * (cs.psd_nmax + 1 + (cs.psd_nmax & 1)) +
+                       2 * cs.psd_nmax);
     static const bool attr = cudaFuncSetAttribute(k_psd_update_pairs,
                                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                   96 * 1024) == cudaSuccess;
@@ -2669,7 +2895,10 @@ void cones_mul_Hs(const ConeSet &cs, double *y, const double *x, cudaStream_t st
   if (cs.n_pow)
     k_nonsym_mul_hs<<<blocks_for(cs.n_pow), kBlock, 0, st>>>(cs, cs.n_pow, cs.pow_begin,
                                                             cs.pow_inst, cs.pow_Hs, y, x);
-  LAUNCH_PSD(k_psd_mul_hs, 3, cs, y, x);
+  if (psd_small(cs))
+    LAUNCH_PSD_SMALL(k_psd_mul_hs_small, cs, y, x);
+  else
+    LAUNCH_PSD(k_psd_mul_hs, 3, cs, y, x);
 }
 
 void cones_affine_ds(const ConeSet &cs, double *ds, const double *s, cudaStream_t st) {
@@ -2697,7 +2926,10 @@ void cones_combined_ds_shift(const ConeSet &cs, double *shift, const double *dz,
   if (cs.n_pow)
     k_nonsym_combined<PowOps><<<blocks_for(cs.n_pow, 128), 128, 0, st>>>(
         cs, pow_args(cs), shift, dz, ds, sm);
-  LAUNCH_PSD(k_psd_combined, 5, cs, shift, dz, ds, sm);
+  if (psd_small(cs))
+    LAUNCH_PSD_SMALL(k_psd_combined_small, cs, shift, dz, ds, sm);
+  else
+    LAUNCH_PSD(k_psd_combined, 5, cs, shift, dz, ds, sm);
 }
 
 void cones_ds_from_dz_offset(const ConeSet &cs, double *out, const double *ds,
@@ -2711,7 +2943,10 @@ void cones_ds_from_dz_offset(const ConeSet &cs, double *out, const double *ds,
   if (cs.n_pow)
     k_nonsym_copy<<<blocks_for(3 * cs.n_pow), kBlock, 0, st>>>(cs, cs.n_pow, cs.pow_begin,
                                                               cs.pow_inst, out, ds);
-  LAUNCH_PSD(k_psd_ds_offset, 4, cs, out, ds);
+  if (psd_small(cs))
+    LAUNCH_PSD_SMALL(k_psd_ds_offset_small, cs, out, ds);
+  else
+    LAUNCH_PSD(k_psd_ds_offset, 4, cs, out, ds);
 }
 
 void cones_step_length_sym(const ConeSet &cs, const double *dz, const double *ds,
@@ -2722,7 +2957,7 @@ void cones_step_length_sym(const ConeSet &cs, const double *dz, const double *ds
                 st>>>(cs, dz, ds, z, s, alpha);
   LAUNCH_SOC_SHAPED(kSocStep, k_soc_tile_step, 4, k_soc_step, dz, ds, z, s, alpha);
   if (psd_small(cs)) {
-    LAUNCH_PSD(k_psd_step_matrices, 3, cs, dz, ds);
+    LAUNCH_PSD_SMALL(k_psd_step_matrices, cs, dz, ds);
     const size_t sm = (size_t)(kPsdEigThreads + 1) * (cs.psd_nmax * (cs.psd_nmax + 1) / 2 +
                                                 2 * cs.psd_nmax) * sizeof(double);
     k_psd_step_eig<<<blocks_for(2 * cs.n_psd, kPsdEigThreads), kPsdEigThreads, sm, st>>>(cs,
