@@ -20,11 +20,16 @@ struct SnDev {
   const long long *foff, *woff, *soff;
   const int2 *amap;
   const int4 *tasks;
+  // forward contributions to a blocked front's positions: entries
+  // gidx[gptr[gath0[s] + p] .. gptr[gath0[s] + p + 1]) of U, in child order
+  const int *gath0, *gptr, *gidx;
   const int *cl_ptr;   // per chunk of a blocked front: its children in clist
   const int4 *clist;   // {child, q_begin, q_end}
   void *F;       // fronts (T)
   void *W;       // factor workspace of blocked fronts (T): dinv, W
-  double *S;     // solve workspace of blocked fronts: work vector, partial sums
+  double *S;     // substitution of blocked fronts: published vectors, forward and backward
+  unsigned *tickets;  // of the substitution launches
+  int ntickets;
   double *U;     // forward-substitution contributions, nrow per supernode
   double *Dinv;  // [global vector index] 1 / pivot
   double *eps;   // [B] static regularisation of the last factorisation

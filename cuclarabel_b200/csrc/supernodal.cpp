@@ -339,7 +339,9 @@ bool sn_build_plan(const std::vector<SnInstance> &in, SnPlan &P, std::string *er
         P.woff[s] = wo;
         wo += align32(kSnNB + (long long)P.ld[s] * kSnNB);
         P.soff[s] = so;
-        so += align32(2LL * P.ld[s]);
+        // published vectors, and the backward tile sums that do not fit on chip
+        const long long np = (P.u0[s] + kSnNB - 1) / kSnNB, nt = np + (P.ld[s] - P.u0[s]) / kSnNB;
+        so += align32(2LL * P.u0[s] + (nt > 36 ? np * nt * kSnNB : 0));
       }
       gpar[s] = S.parent[t] >= 0 ? sbase + S.parent[t] : -1;
     }
@@ -451,6 +453,30 @@ bool sn_build_plan(const std::vector<SnInstance> &in, SnPlan &P, std::string *er
     P.clist.reserve(P.cl_ptr.back());
     for (auto &l : lists) P.clist.insert(P.clist.end(), l.begin(), l.end());
   }
+  // ---- children's contributions per position of the blocked fronts
+  P.gath0.assign(ns, 0);
+  P.gptr.assign(1, 0);
+  for (int s = 0; s < ns; ++s) {
+    if (!P.large[s]) continue;
+    P.gath0[s] = (int)P.gptr.size() - 1;
+    const int g0 = P.gath0[s], ld = P.ld[s];
+    P.gptr.resize(g0 + ld + 1, 0);
+    std::vector<int> fill(ld + 1, 0);
+    auto each = [&](auto &&f) {
+      for (int a = P.ch_ptr[s]; a < P.ch_ptr[s + 1]; ++a) {
+        const int c = P.ch[a];
+        const int *rel = P.rel.data() + P.rel_off[c];
+        for (int q = 0; q < P.nrow[c]; ++q) f(rel[q], P.uoff[c] + q);
+      }
+    };
+    each([&](int p, int) { fill[p + 1]++; });
+    const size_t base = P.gidx.size();
+    for (int p = 0; p < ld; ++p) fill[p + 1] += fill[p];
+    if (base + fill[ld] >= (1ULL << 31)) return fail("too many contributions");
+    for (int p = 0; p <= ld; ++p) P.gptr[g0 + p] = (int)base + fill[p];
+    P.gidx.resize(base + fill[ld]);
+    each([&](int p, int u) { P.gidx[base + fill[p]++] = u; });
+  }
   // ---- schedules, level by level
   int H = 0;
   for (int s = 0; s < ns; ++s) H = std::max(H, level[s] + 1);
@@ -537,76 +563,31 @@ bool sn_build_plan(const std::vector<SnInstance> &in, SnPlan &P, std::string *er
     }
   }
   P.flops = flops;
-  // forward substitution, leaves first
-  for (int L = 0; L < H; ++L) {
-    int b0 = (int)P.tasks.size();
+  // substitutions; a blocked front's row tiles: u0 mod kSnNB rows first (when
+  // nonzero), then kSnNB each
+  auto panels = [&](int s) { return (P.u0[s] + kSnNB - 1) / kSnNB; };
+  // tasks (tile, front) in an order in which each waits for earlier ones only
+  auto fronts = [&](std::vector<SnLaunch> &sched, int kind, int L, bool forward) {
+    if (big[L].empty()) return;
+    const int b0 = (int)P.tasks.size();
+    int most = 0;
+    auto tiles = [&](int s) { return panels(s) + (forward ? (P.ld[s] - P.u0[s]) / kSnNB : 0); };
+    for (int s : big[L]) most = std::max(most, tiles(s));
+    for (int k = 0; k < most; ++k)
+      for (int s : big[L])
+        if (k < tiles(s)) P.tasks.push_back({s, forward ? k : tiles(s) - 1 - k, P.ntickets, 0});
+    P.ntickets++;
+    launch(sched, kind, b0);
+  };
+  for (int L = 0; L < H; ++L) {  // forward, leaves first
+    const int b0 = (int)P.tasks.size();
     for (int s : small[L]) P.tasks.push_back({s, 0, 0, 0});
     launch(P.fwd, SN_FWD_SMALL, b0);
-    if (big[L].empty()) continue;
-    b0 = (int)P.tasks.size();
-    for (int s : big[L])
-      for (int c = 0; c < P.ld[s]; c += kSnAsmCols)
-        P.tasks.push_back({s, c, std::min(P.ld[s], c + kSnAsmCols),
-                           P.chunk_off[s] + c / kSnAsmCols});
-    launch(P.fwd, SN_FWD_GATHER, b0);
-    std::vector<std::vector<std::pair<int, int>>> pl(big[L].size());
-    size_t maxp = 0;
-    for (size_t a = 0; a < big[L].size(); ++a) {
-      panels_of(P.u0[big[L][a]], pl[a]);
-      maxp = std::max(maxp, pl[a].size());
-    }
-    for (size_t p = 0; p < maxp; ++p) {
-      b0 = (int)P.tasks.size();
-      for (size_t a = 0; a < big[L].size(); ++a)
-        if (p < pl[a].size()) P.tasks.push_back({big[L][a], kK(pl[a][p].first, pl[a][p].second), 0, 0});
-      launch(P.fwd, SN_FWD_DIAG, b0);
-      b0 = (int)P.tasks.size();
-      for (size_t a = 0; a < big[L].size(); ++a) {
-        if (p >= pl[a].size()) continue;
-        const int s = big[L][a], k = pl[a][p].first, K = pl[a][p].second;
-        for (int r0 = k + K; r0 < P.ld[s]; r0 += kSnNB) P.tasks.push_back({s, kK(k, K), r0, 0});
-      }
-      launch(P.fwd, SN_FWD_GEMV, b0);
-    }
-    b0 = (int)P.tasks.size();
-    for (int s : big[L]) P.tasks.push_back({s, 0, 0, 0});
-    launch(P.fwd, SN_FWD_SCATTER, b0);
+    fronts(P.fwd, SN_FWD_DIAG, L, true);
   }
-  // backward substitution, roots first
-  for (int L = H - 1; L >= 0; --L) {
-    int b0;
-    if (!big[L].empty()) {
-      b0 = (int)P.tasks.size();
-      for (int s : big[L]) P.tasks.push_back({s, 0, 0, 0});
-      launch(P.bwd, SN_BWD_GATHER, b0);
-      std::vector<std::vector<std::pair<int, int>>> pl(big[L].size());
-      size_t maxp = 0;
-      for (size_t a = 0; a < big[L].size(); ++a) {
-        panels_of(P.u0[big[L][a]], pl[a]);
-        maxp = std::max(maxp, pl[a].size());
-      }
-      for (size_t pp = 0; pp < maxp; ++pp) {
-        b0 = (int)P.tasks.size();
-        for (size_t a = 0; a < big[L].size(); ++a) {
-          if (pp >= pl[a].size()) continue;
-          const size_t p = pl[a].size() - 1 - pp;
-          const int s = big[L][a], k = pl[a][p].first, K = pl[a][p].second;
-          for (int r0 = k + K; r0 < P.ld[s]; r0 += kSnNB) P.tasks.push_back({s, kK(k, K), r0, 0});
-        }
-        launch(P.bwd, SN_BWD_PARTIAL, b0);
-        b0 = (int)P.tasks.size();
-        for (size_t a = 0; a < big[L].size(); ++a) {
-          if (pp >= pl[a].size()) continue;
-          const size_t p = pl[a].size() - 1 - pp;
-          P.tasks.push_back({big[L][a], kK(pl[a][p].first, pl[a][p].second), 0, 0});
-        }
-        launch(P.bwd, SN_BWD_DIAG, b0);
-      }
-      b0 = (int)P.tasks.size();
-      for (int s : big[L]) P.tasks.push_back({s, 0, 0, 0});
-      launch(P.bwd, SN_BWD_SCATTER, b0);
-    }
-    b0 = (int)P.tasks.size();
+  for (int L = H - 1; L >= 0; --L) {  // backward, roots first
+    fronts(P.bwd, SN_BWD_DIAG, L, false);
+    const int b0 = (int)P.tasks.size();
     for (int s : small[L]) P.tasks.push_back({s, 0, 0, 0});
     launch(P.bwd, SN_BWD_SMALL, b0);
   }

@@ -78,15 +78,15 @@ enum SnLaunchKind : int {
                         //   by substitution, L = W D^-1
   SN_UPDATE,            // {s, k | K << 16, r0, c0}: 128 x 64 tile (r0, c0) -= L(r0 rows) W(c0 rows)^T
   SN_FWD_SMALL,         // {s}: forward substitution of a small front (one warp)
-  SN_FWD_GATHER,        // {s, c_begin, c_end, chunk}: positions of a blocked front's work vector
-  SN_FWD_DIAG,          // {s, k | K << 16}: v(panel) <- L11^-1 v(panel)
-  SN_FWD_GEMV,          // {s, k | K << 16, r0}: v(r0 rows) -= L(r0 rows, panel) v(panel)
-  SN_FWD_SCATTER,       // {s}
+  SN_FWD_GATHER,        // (no launches: part of the next; the profile's layout is kept)
+  SN_FWD_DIAG,          // {s, tile, ticket}: forward substitution of a blocked front's row tile
+  SN_FWD_GEMV,          // (no launches)
+  SN_FWD_SCATTER,       // (no launches)
   SN_BWD_SMALL,         // {s}
-  SN_BWD_GATHER,        // {s}
-  SN_BWD_PARTIAL,       // {s, k | K << 16, r0}: L(r0 rows, panel)^T v(r0 rows)
-  SN_BWD_DIAG,          // {s, k | K << 16}: v(panel) <- L11^-T (v(panel) - partial sums)
-  SN_BWD_SCATTER,       // {s}
+  SN_BWD_GATHER,        // (no launches)
+  SN_BWD_PARTIAL,       // (no launches)
+  SN_BWD_DIAG,          // {s, panel, ticket}: backward substitution of a blocked front's panel
+  SN_BWD_SCATTER,       // (no launches)
   SN_KINDS
 };
 struct SnLaunch {
@@ -116,7 +116,7 @@ struct SnPlan {
       uoff;
   std::vector<long long> foff;  // front offsets (elements, multiples of 32)
   std::vector<long long> woff;  // factor workspace of blocked fronts: dinv (kSnNB), W (ld x kSnNB)
-  std::vector<long long> soff;  // solve workspace of blocked fronts: v (ld), partial sums (ld)
+  std::vector<long long> soff;  // substitution of blocked fronts: published x, forward (u0), backward (u0), tile sums
   std::vector<int> ch;          // children, in order
   std::vector<int> fidx;        // front position -> global vector index (-1 none)
   std::vector<int> rel;         // struct row k of s -> position in the parent's front
@@ -128,9 +128,13 @@ struct SnPlan {
   // of front s is chunk_off[s] + k, its entries clist[cl_ptr[..]..)
   std::vector<int> chunk_off, cl_ptr;
   std::vector<SnQuad> clist;
+  // the children's entries of U that fall on each position of a blocked front,
+  // in child order: gidx[gptr[gath0[s] + p] .. gptr[gath0[s] + p + 1])
+  std::vector<int> gath0, gptr, gidx;
   std::vector<SnQuad> tasks;
   std::vector<SnLaunch> fact, fwd, bwd;
   std::vector<int> insts;       // the instances of the plan
+  int ntickets = 0;             // substitution launches of blocked fronts
   long long f_elems = 0, w_elems = 0, s_elems = 0, u_elems = 0;
   int small_smem_max = 0;       // largest small front, elements
   double flops = 0;             // factorisation flops of the padded fronts (sum over launches)
