@@ -339,9 +339,9 @@ bool sn_build_plan(const std::vector<SnInstance> &in, SnPlan &P, std::string *er
         P.woff[s] = wo;
         wo += align32(kSnNB + (long long)P.ld[s] * kSnNB);
         P.soff[s] = so;
-        // published vectors, and the backward tile sums that do not fit on chip
+        // published vectors, and the backward tile sums
         const long long np = (P.u0[s] + kSnNB - 1) / kSnNB, nt = np + (P.ld[s] - P.u0[s]) / kSnNB;
-        so += align32(2LL * P.u0[s] + (nt > 36 ? np * nt * kSnNB : 0));
+        so += align32(2LL * P.u0[s] + np * nt * kSnNB);
       }
       gpar[s] = S.parent[t] >= 0 ? sbase + S.parent[t] : -1;
     }
@@ -573,6 +573,17 @@ bool sn_build_plan(const std::vector<SnInstance> &in, SnPlan &P, std::string *er
     int most = 0;
     auto tiles = [&](int s) { return panels(s) + (forward ? (P.ld[s] - P.u0[s]) / kSnNB : 0); };
     for (int s : big[L]) most = std::max(most, tiles(s));
+    // the helpers' shares: about one helper per SM, of 2 to 8 tiles
+    auto update = [&](int s) { return (P.ld[s] - P.u0[s]) / kSnNB; };
+    long long all = 0;
+    for (int s : big[L]) all += update(s) > kSubOwn ? (long long)panels(s) * update(s) : 0;
+    const int share = (int)std::min(8LL, std::max(2LL, (all + 147) / 148));
+    for (int k = 0; !forward && k < most; ++k)
+      for (int s : big[L])
+        for (int i = 0; k < tiles(s) && update(s) > kSubOwn && i < update(s); i += share) {
+          const int np = panels(s), e = std::min(i + share, update(s));
+          P.tasks.push_back({s, np - 1 - k, P.ntickets, (np + i) | (np + e) << 16});
+        }
     for (int k = 0; k < most; ++k)
       for (int s : big[L])
         if (k < tiles(s)) P.tasks.push_back({s, forward ? k : tiles(s) - 1 - k, P.ntickets, 0});

@@ -792,6 +792,10 @@ __global__ void __launch_bounds__(256) k_sn_bwd_small(SnDev d, int base, int cou
 // order; per panel four interleaved column sums forward; per tile and column a
 // balanced tree over the rows, and four interleaved sums over the tiles in
 // ascending order, backward.
+// The update rows' part of a backward panel needs nothing from the front's other
+// panels; above kSubOwn tiles it is given to blocks of its own, a few tiles each,
+// which publish their tile sums (one block streamed 16 tiles in 38 us: a level's
+// backward launch 51 us on average, 26 now).
 // Tasks are taken in list order (a ticket per launch), a task waits only for
 // earlier ones, so the waits end whatever is resident; a bounded wait that runs
 // out makes the solution NaN, which the caller reports as a failed solve.
@@ -799,6 +803,7 @@ constexpr int kSubThreads = 256;
 constexpr int kSubCols = 32;   // columns (rows) of a chunk, columns of a block column
 constexpr int kSubRing = 3;
 constexpr int kSubSpin = 1 << 21;  // polls, about a second
+constexpr int kSubNear = 36;  // tile sums of a backward panel kept on chip
 constexpr int kSubB = kSnNB / kSubCols;  // block columns of a diagonal block
 template <typename T>
 struct Sub {
@@ -813,7 +818,7 @@ struct Sub {
     return kSubCols * (b * (kSnNB + pad) - kSubCols * (b * (b - 1) / 2));
   }
   static constexpr int ring = kSubRing * stage, l11 = boff(kSubB);
-  static constexpr int aux = 36 * kSnNB;  // gathered values and column sums; tile sums
+  static constexpr int aux = kSubNear * kSnNB;  // gathered values and column sums; tile sums
   static constexpr size_t bytes =
       (ring + l11) * sizeof(T) + (aux + kSnNB + 2 * kSubCols + 2 * kSnNB) * sizeof(double);
 };
@@ -911,6 +916,12 @@ __global__ void __launch_bounds__(kSubThreads) k_sn_fwd_front(SnDev d, int base)
   issue(1);
   if (pivot && tid < h)
     reinterpret_cast<unsigned long long *>(v)[d.u0[s] + r0 + tid] = kSubEmpty;
+  if (pivot) {  // and the helpers' tile sums
+    const int nu = (int)(ld - d.u0[s]) / kSnNB;
+    unsigned long long *q = reinterpret_cast<unsigned long long *>(v) + 2LL * d.u0[s] +
+                            ((long long)t * (np + nu) + np - t - 1) * kSnNB;
+    for (int e = tid; nu > kSubOwn && e < nu * kSnNB; e += kSubThreads) q[e] = kSubEmpty;
+  }
   // own rows: y plus the children's contributions in child order; the tile's
   // lists are one run, gathered by all threads and summed by a thread per row
   {
@@ -1017,20 +1028,23 @@ __global__ void __launch_bounds__(kSubThreads) k_sn_bwd_front(SnDev d, int base)
   const int *fi = d.fidx + d.fix_off[s];
   const T *f = reinterpret_cast<const T *>(d.F) + d.foff[s];
   double *v = d.S + d.soff[s] + u0;  // published here; the forward vector is before it
-  // the m-th tile: the update rows' first, then the panels from the last down
-  auto tile = [&](int m) { return m < nt - np ? np + m : nt - 1 - m; };
+  // tiles [i0, i1) of the update rows first, then (unless the task is only these)
+  // the panels from the last down
+  const bool helped = nt - np > kSubOwn, helper = tk.w != 0;
+  const int i0 = helper ? tk.w & 0xffff : np, i1 = helper ? tk.w >> 16 : helped ? np : nt;
+  auto tile = [&](int m) { return m < i1 - i0 ? i0 + m : np - 1 - (m - (i1 - i0)); };
   constexpr int nr = kSnNB / kSubCols;  // chunks of a tile, taken from its last rows up
-  const int G = (nt - 1 - t) * nr;
+  const int M = i1 - i0 + (helper ? 0 : np - 1 - t), G = M * nr;
   auto row = [&](int g) { return P.start(tile(g / nr)) + kSubCols * (nr - 1 - g % nr); };
   auto issue = [&](int g) {
     if (g < G) sub_copy_rows(ring + (g % kSubRing) * Sub<T>::stage, f, ld, row(g), k0, K);
     cp_async_commit();
   };
-  sub_copy_diag(L, f, ld, k0, K);
+  if (!helper) sub_copy_diag(L, f, ld, k0, K);
   cp_async_commit();
   issue(0);
   issue(1);
-  if (tid < kSnNB) {
+  if (tid < kSnNB && !helper) {
     const int g = tid < K ? fi[k0 + tid] : -1;
     vs[tid] = g >= 0 ? d.y[vix(d, g)] : 0.0;
     if (tid < K) reinterpret_cast<unsigned long long *>(v)[k0 + tid - u0] = kSubEmpty;
@@ -1041,14 +1055,19 @@ __global__ void __launch_bounds__(kSubThreads) k_sn_bwd_front(SnDev d, int base)
   // threads, then the tile's two halves.
   const int cl = tid & (kSnNB - 1), odd = tid / kSnNB;
   double pr[8], hi = 0, lo = 0;
-  // tile sums: the nearest 36 tiles in shared memory, others in the workspace
-  double *far = d.S + d.soff[s] + 2LL * u0 + (long long)t * nt * kSnNB;
+  // tile sums: the nearest tiles in shared memory, others in the workspace
+  double *far = d.S + d.soff[s] + 2LL * u0 + (long long)t * nt * kSnNB + cl;
   auto slot = [&](int i) -> double & {
     const int k = i - t - 1;
-    return k < Sub<T>::aux / kSnNB ? aux[k * kSnNB + cl] : far[(long long)k * kSnNB + cl];
+    return k < kSubNear ? aux[k * kSnNB + cl] : far[(long long)k * kSnNB];
   };
   auto finish = [&](int i) {
-    if (!odd) slot(i) = (lo + red[cl]) + (hi + red[kSnNB + cl]);
+    const double p = (lo + red[cl]) + (hi + red[kSnNB + cl]);
+    if (odd) return;
+    if (helper)
+      sub_publish(far + (long long)(i - t - 1) * kSnNB, p);
+    else
+      slot(i) = p;
   };
   double ahead = 0;
   bool lost = false;
@@ -1057,6 +1076,23 @@ __global__ void __launch_bounds__(kSubThreads) k_sn_bwd_front(SnDev d, int base)
     const int p = G > 0 && row(0) >= u0 ? fi[row(0) + lane] : -1;
     pos = G > 1 && row(1) >= u0 ? fi[row(1) + lane] : -1;
     ahead = p >= 0 ? d.y[vix(d, p)] : 0.0;
+  }
+  if (helped && !helper) {  // the helpers' sums, while the chain gets here
+    for (int b = np + odd; b < nt; b += 16) {
+      double p[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        p[k] = b + 2 * k < nt ? __ldcg(far + (long long)(b + 2 * k - t - 1) * kSnNB) : 0.0;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const int i = b + 2 * k;
+        if (i < nt) {
+          if (__double_as_longlong(p[k]) == (long long)kSubEmpty)
+            p[k] = sub_wait(far + (long long)(i - t - 1) * kSnNB, lost);
+          if (i - t - 1 < kSubNear) aux[(i - t - 1) * kSnNB + cl] = p[k];
+        }
+      }
+    }
   }
   for (int g = 0; g < G; ++g) {
     const int r = row(g);
@@ -1094,7 +1130,8 @@ __global__ void __launch_bounds__(kSubThreads) k_sn_bwd_front(SnDev d, int base)
   }
   cp_async_wait<0>();
   __syncthreads();
-  if (G > 0) finish(tile(nt - 2 - t));
+  if (G > 0) finish(tile(M - 1));
+  if (helper) return;
   __syncthreads();
   // four interleaved sums over the tiles in ascending order, two per thread
   {
@@ -1102,7 +1139,8 @@ __global__ void __launch_bounds__(kSubThreads) k_sn_bwd_front(SnDev d, int base)
 #pragma unroll
     for (int u = 0; u < 2; ++u)
 #pragma unroll 4
-      for (int i = t + 1 + 2 * odd + u; i < nt; i += 4) a[u] += slot(i);
+      for (int i = t + 1 + 2 * odd + u; i < nt; i += 4)
+        a[u] += i - t - 1 < kSubNear ? slot(i) : __ldcg(&slot(i));
     __syncthreads();
     if (odd) {
       red[cl] = a[0];

@@ -59,6 +59,7 @@ bool sn_analyse(int N, const std::vector<int> &xadj, const std::vector<int> &adj
 // kSnNB x kSnNB tiles: the first panel takes u0 mod kSnNB columns (when
 // nonzero), every later panel kSnNB.
 constexpr int kSnKPad = 16;
+constexpr int kSubOwn = 2;   // update tiles that a backward panel's block sums itself
 constexpr int kSnAsmCols = 32;  // parent columns per assembly task
 
 struct SnPair {
@@ -85,7 +86,8 @@ enum SnLaunchKind : int {
   SN_BWD_SMALL,         // {s}
   SN_BWD_GATHER,        // (no launches)
   SN_BWD_PARTIAL,       // (no launches)
-  SN_BWD_DIAG,          // {s, panel, ticket}: backward substitution of a blocked front's panel
+  SN_BWD_DIAG,          // {s, panel, ticket, 0}: backward substitution of a blocked front's panel;
+                        //   {.., i0 | i1 << 16}: only its sums over the update tiles [i0, i1)
   SN_BWD_SCATTER,       // (no launches)
   SN_KINDS
 };
