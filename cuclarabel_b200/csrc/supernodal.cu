@@ -409,6 +409,10 @@ __global__ void __launch_bounds__(kDiagThreads) k_sn_diag(SnDev d, KKTDev k, LDL
   if (bad) ok[inst] = 0;
 }
 
+// row q of the packed strict lower triangle: rows padded to even lengths, so that
+// every row starts on a pair
+__device__ __forceinline__ int lrow(int q) { return q * q / 2; }
+
 // one column block of the TRSM below: (a) then (b), NB columns from b0
 template <typename T, int NB>
 __device__ __forceinline__ void trsm_block(T *X, const T *Lr, int b0, int K, int m, int half) {
@@ -419,7 +423,7 @@ __device__ __forceinline__ void trsm_block(T *X, const T *Lr, int b0, int K, int
 #pragma unroll
     for (int j = 0; j < NB - 1; ++j)
 #pragma unroll
-      for (int q = j + 1; q < NB; ++q) x[q] -= x[j] * Lr[(b0 + q) * (b0 + q - 1) / 2 + b0 + j];
+      for (int q = j + 1; q < NB; ++q) x[q] -= x[j] * Lr[lrow(b0 + q) + b0 + j];
 #pragma unroll
     for (int j = 0; j < NB; ++j) X[(b0 + j) * kSnNB + m] = x[j];
   }
@@ -436,12 +440,16 @@ __device__ __forceinline__ void trsm_block(T *X, const T *Lr, int b0, int K, int
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         const int q = min(q0 + u * H, K - 1);
-        lq[u] = Lr + q * (q - 1) / 2 + b0;
+        lq[u] = Lr + lrow(q) + b0;
       }
 #pragma unroll
-      for (int j = 0; j < NB; ++j)
+      for (int j = 0; j < NB; j += 2)
 #pragma unroll
-        for (int u = 0; u < 4; ++u) acc[u] += x[j] * lq[u][j];
+        for (int u = 0; u < 4; ++u) {
+          const Pair<T> l = load_pair(lq[u] + j);
+          acc[u] += x[j] * l.x;
+          acc[u] += x[j + 1] * l.y;
+        }
 #pragma unroll
       for (int u = 0; u < 4; ++u)
         if (q0 + u * H < K) X[(q0 + u * H) * kSnNB + m] -= acc[u];
@@ -459,7 +467,7 @@ __device__ __forceinline__ void trsm_block(T *X, const T *Lr, int b0, int K, int
 // row take the block's contribution, sum_j w(m, j) L11(q, j), the two
 // halves of the thread block splitting the columns.  Two barriers per
 // column block.  The tile (K x 128, column-major) and the strict lower triangle
-// of L11 packed by rows (row q at q (q - 1) / 2) sit in shared memory.
+// of L11 packed by rows sit in shared memory.
 template <typename T>
 __global__ void __launch_bounds__(kTrsmThreads) k_sn_trsm(SnDev d, int base, const int *run) {
   const int4 t = d.tasks[base + blockIdx.x];
@@ -467,28 +475,31 @@ __global__ void __launch_bounds__(kTrsmThreads) k_sn_trsm(SnDev d, int base, con
   if (!run[d.inst[s]]) return;
   extern __shared__ __align__(16) unsigned char sraw[];
   T *X = reinterpret_cast<T *>(sraw);  // column q of the tile at X + q kSnNB
-  T *Lr = X + K * kSnNB;               // L11(q, j), j < q, at Lr[q (q - 1) / 2 + j]
+  T *Lr = X + K * kSnNB;               // L11(q, j), j < q, at Lr[lrow(q) + j]
   const long long ld = d.ld[s];
   T *f = reinterpret_cast<T *>(d.F) + d.foff[s];
   const T *ws = reinterpret_cast<const T *>(d.W) + d.woff[s];
   T *wr = reinterpret_cast<T *>(d.W) + d.woff[s] + kSnNB;
   const int tid = threadIdx.x;
-  // stage the tile and L11 by row pairs, fixed trip counts (many 16-byte
+  // the tile by cp.async, then L11 by row pairs, fixed trip counts (many 16-byte
   // loads in flight)
+  constexpr int E = 16 / (int)sizeof(T), per = kSnNB / E;
 #pragma unroll 8
-  for (int it = 0; it < kSnNB * kSnNB / 2 / kTrsmThreads; ++it) {
-    const int p = tid + it * kTrsmThreads, q = p >> 6, m = (p & 63) * 2;
-    if (q < K) store_pair(X + q * kSnNB + m, load_pair(f + (k0 + q) * ld + r0 + m));
+  for (int it = 0; it < kSnNB * per / kTrsmThreads; ++it) {
+    const int p = tid + it * kTrsmThreads, q = p / per, m = (p % per) * E;
+    if (q < K) cp_async16(X + q * kSnNB + m, f + (k0 + q) * ld + r0 + m);
   }
+  cp_async_commit();
 #pragma unroll 8
   for (int it = 0; it < kSnNB * kSnNB / 2 / kTrsmThreads; ++it) {
     const int p = tid + it * kTrsmThreads, j = p >> 6, q = (p & 63) * 2;
     if (j < K && q + 1 > j && q < K) {
       const Pair<T> w = load_pair(f + (k0 + j) * ld + k0 + q);
-      if (q > j) Lr[q * (q - 1) / 2 + j] = w.x;
-      Lr[(q + 1) * q / 2 + j] = w.y;  // q + 1 > j
+      if (q > j) Lr[lrow(q) + j] = w.x;
+      Lr[lrow(q + 1) + j] = w.y;  // q + 1 > j
     }
   }
+  cp_async_wait<0>();
   __syncthreads();
   const int m = tid & (kSnNB - 1), half = tid / kSnNB;
   for (int b0 = 0; b0 < K; b0 += 32) {
@@ -498,13 +509,14 @@ __global__ void __launch_bounds__(kTrsmThreads) k_sn_trsm(SnDev d, int base, con
     else
       trsm_block<T, 16>(X, Lr, b0, K, m, half);
   }
-#pragma unroll 4
-  for (int it = 0; it < kSnNB * kSnNB / kTrsmThreads; ++it) {
-    const int idx = tid + it * kTrsmThreads, q = idx >> 7, mm = idx & (kSnNB - 1);
+#pragma unroll 8
+  for (int it = 0; it < kSnNB * kSnNB / 2 / kTrsmThreads; ++it) {
+    const int p = tid + it * kTrsmThreads, q = p >> 6, mm = (p & 63) * 2;
     if (q < K) {
-      const T w = X[idx];
-      wr[(long long)q * ld + r0 + mm] = w;
-      f[(k0 + q) * ld + r0 + mm] = w * ws[q];
+      const Pair<T> w = load_pair(X + q * kSnNB + mm);
+      const T di = ws[q];
+      store_pair(wr + (long long)q * ld + r0 + mm, w);
+      store_pair(f + (k0 + q) * ld + r0 + mm, Pair<T>{w.x * di, w.y * di});
     }
   }
 }
@@ -1273,7 +1285,7 @@ size_t diag_smem() {  // the block and the scaled columns of one column block
 }
 template <typename T>
 size_t trsm_smem() {  // the tile (kSnNB x kSnNB) and the packed strict lower L11
-  return (size_t)kSnNB * kSnNB * sizeof(T) + (size_t)kSnNB * (kSnNB - 1) / 2 * sizeof(T);
+  return (size_t)kSnNB * kSnNB * sizeof(T) + (size_t)kSnNB * kSnNB / 2 * sizeof(T);
 }
 template <typename T>
 size_t gemm_smem() {

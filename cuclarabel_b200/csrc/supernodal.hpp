@@ -60,7 +60,7 @@ bool sn_analyse(int N, const std::vector<int> &xadj, const std::vector<int> &adj
 // nonzero), every later panel kSnNB.
 constexpr int kSnKPad = 16;
 constexpr int kSubOwn = 2;   // update tiles that a backward panel's block sums itself
-constexpr int kSnAsmCols = 32;  // parent columns per assembly task
+constexpr int kSnAsmCols = 8;   // parent columns per assembly task
 
 struct SnPair {
   int x, y;
