@@ -1183,7 +1183,18 @@ extern "C" int clgpu_debug_check_instance(const clgpu_problem *pb, const clgpu_s
           if (k > 0 && rel[k] <= rel[k - 1]) return -35;
         }
       }
+    // contributions of the children: entries of U in child order
+    for (int s = 0; s < plan.ns; ++s)
+      for (int q = 0; plan.large[s] && q < plan.ld[s]; ++q) {
+        const int *gp = plan.gptr.data() + plan.gath0[s] + q;
+        if (gp[0] < 0 || gp[0] > gp[1] || gp[1] > (int)plan.gidx.size()) return -52;
+        for (int e = gp[0]; e < gp[1]; ++e)
+          if (plan.gidx[e] < 0 || plan.gidx[e] >= plan.u_elems ||
+              (e > gp[0] && plan.gidx[e] <= plan.gidx[e - 1]))
+            return -53;
+      }
     // every launch's tasks inside the task list, tiles inside their fronts
+    std::set<std::pair<int, int>> sub_done[2];
     for (auto *sched : {&plan.fact, &plan.fwd, &plan.bwd})
       for (const SnLaunch &L : *sched) {
         if (L.begin < 0 || L.count <= 0 || (size_t)L.begin + L.count > plan.tasks.size()) return -36;
@@ -1191,18 +1202,47 @@ extern "C" int clgpu_debug_check_instance(const clgpu_problem *pb, const clgpu_s
           const SnQuad t = plan.tasks[q];
           if (t.x < 0 || t.x >= plan.ns) return -37;
           const int ld = plan.ld[t.x], k0 = t.y & 0xffff, K = t.y >> 16;
-          if (L.kind == SN_DIAG || L.kind == SN_TRSM || L.kind == SN_UPDATE ||
-              L.kind == SN_FWD_DIAG || L.kind == SN_FWD_GEMV || L.kind == SN_BWD_PARTIAL ||
-              L.kind == SN_BWD_DIAG) {
-            if (!plan.large[t.x] || K <= 0 || K > kSnNB || K % kSnKPad || k0 + K > plan.u0[t.x])
+          if (L.kind == SN_DIAG || L.kind == SN_TRSM || L.kind == SN_UPDATE) {
+            const int most = L.kind == SN_UPDATE ? 2 * kSnNB : kSnNB;
+            if (!plan.large[t.x] || K <= 0 || K > most || K % kSnKPad || k0 + K > plan.u0[t.x])
               return -38;
-            if ((L.kind == SN_TRSM || L.kind == SN_UPDATE || L.kind == SN_FWD_GEMV ||
-                 L.kind == SN_BWD_PARTIAL) &&
+            if (L.kind != SN_DIAG &&
                 (t.z < k0 + K || t.z + kSnNB > ld || (t.z - k0 - K) % kSnNB))
               return -39;
             if (L.kind == SN_UPDATE &&
                 (t.w < k0 + K || t.w + 64 > ld || (t.w - k0 - K) % 64 || t.z + kSnNB <= t.w))
               return -40;
+            if (L.kind == SN_TRSM &&
+                (t.w < 0 || t.w + K > (plan.u0[t.x] > kSnNB ? 2 : 1) * kSnNB ||
+                 plan.woff[t.x] + kSnNB + (long long)(t.w + K) * ld > plan.w_elems))
+              return -47;
+          }
+          if (L.kind == SN_FWD_DIAG || L.kind == SN_BWD_DIAG) {
+            const int np = (plan.u0[t.x] + kSnNB - 1) / kSnNB;
+            const int nt = np + (ld - plan.u0[t.x]) / kSnNB;
+            const int i0 = t.w & 0xffff, i1 = t.w >> 16;
+            if (!plan.large[t.x] || t.y < 0 || t.y >= (L.kind == SN_FWD_DIAG ? nt : np) ||
+                t.z < 0 || t.z >= plan.ntickets || t.z != plan.tasks[L.begin].z)
+              return -48;
+            if (t.w && (L.kind != SN_BWD_DIAG || nt - np <= kSubOwn || i0 < np || i0 >= i1 || i1 > nt))
+              return -49;
+            // a task's panels (forward: earlier, backward: later ones) and helpers
+            // come before it
+            std::set<std::pair<int, int>> &done = sub_done[L.kind == SN_FWD_DIAG];
+            if (t.w) {
+              for (int i = i0; i < i1; ++i) done.insert({t.x, (t.y + 1) * nt + i + (1 << 24)});
+            } else {
+              if (L.kind == SN_FWD_DIAG)
+                for (int j = 0; j < std::min(t.y, np); ++j)
+                  if (!done.count({t.x, j})) return -50;
+              if (L.kind == SN_BWD_DIAG) {
+                for (int j = t.y + 1; j < np; ++j)
+                  if (!done.count({t.x, j})) return -50;
+                for (int i = np; nt - np > kSubOwn && i < nt; ++i)
+                  if (!done.count({t.x, (t.y + 1) * nt + i + (1 << 24)})) return -51;
+              }
+              done.insert({t.x, t.y});
+            }
           }
           if ((L.kind == SN_ASSEMBLE || L.kind == SN_FWD_GATHER) &&
               (t.y < 0 || t.z > ld || t.y >= t.z))

@@ -337,7 +337,7 @@ bool sn_build_plan(const std::vector<SnInstance> &in, SnPlan &P, std::string *er
       fo += align32((long long)P.ld[s] * P.ld[s]);
       if (lg) {
         P.woff[s] = wo;
-        wo += align32(kSnNB + (long long)P.ld[s] * kSnNB);
+        wo += align32(kSnNB + (long long)P.ld[s] * kSnNB * (P.u0[s] > kSnNB ? 2 : 1));
         P.soff[s] = so;
         // published vectors, and the backward tile sums
         const long long np = (P.u0[s] + kSnNB - 1) / kSnNB, nt = np + (P.ld[s] - P.u0[s]) / kSnNB;
@@ -433,25 +433,28 @@ bool sn_build_plan(const std::vector<SnInstance> &in, SnPlan &P, std::string *er
   for (int s = 0; s < ns; ++s)
     P.chunk_off[s + 1] = P.chunk_off[s] + (P.large[s] ? (P.ld[s] + kSnAsmCols - 1) / kSnAsmCols : 0);
   {
-    std::vector<std::vector<SnQuad>> lists(P.chunk_off[ns]);
-    for (int s = 0; s < ns; ++s) {
-      if (!P.large[s]) continue;
-      for (int a = P.ch_ptr[s]; a < P.ch_ptr[s + 1]; ++a) {
-        const int c = P.ch[a], cn = P.nrow[c];
-        const int *rel = P.rel.data() + P.rel_off[c];
-        for (int q = 0; q < cn;) {
-          const int chunk = rel[q] / kSnAsmCols;
-          int qe = q + 1;
-          while (qe < cn && rel[qe] / kSnAsmCols == chunk) ++qe;
-          lists[P.chunk_off[s] + chunk].push_back({c, q, qe, 0});
-          q = qe;
+    auto runs = [&](auto &&f) {  // f(chunk, {child, q, qe, 0}), children in order
+      for (int s = 0; s < ns; ++s) {
+        if (!P.large[s]) continue;
+        for (int a = P.ch_ptr[s]; a < P.ch_ptr[s + 1]; ++a) {
+          const int c = P.ch[a], cn = P.nrow[c];
+          const int *rel = P.rel.data() + P.rel_off[c];
+          for (int q = 0; q < cn;) {
+            const int chunk = rel[q] / kSnAsmCols, stop = (chunk + 1) * kSnAsmCols;
+            int qe = q + 1;
+            while (qe < cn && rel[qe] < stop) ++qe;
+            f(P.chunk_off[s] + chunk, SnQuad{c, q, qe, 0});
+            q = qe;
+          }
         }
       }
-    }
+    };
     P.cl_ptr.assign(P.chunk_off[ns] + 1, 0);
-    for (size_t g = 0; g < lists.size(); ++g) P.cl_ptr[g + 1] = P.cl_ptr[g] + (int)lists[g].size();
-    P.clist.reserve(P.cl_ptr.back());
-    for (auto &l : lists) P.clist.insert(P.clist.end(), l.begin(), l.end());
+    runs([&](int g, const SnQuad &) { P.cl_ptr[g + 1]++; });
+    for (int g = 0; g < P.chunk_off[ns]; ++g) P.cl_ptr[g + 1] += P.cl_ptr[g];
+    P.clist.resize(P.cl_ptr.back());
+    std::vector<int> at(P.cl_ptr.begin(), P.cl_ptr.end() - 1);
+    runs([&](int g, const SnQuad &r) { P.clist[at[g]++] = r; });
   }
   // ---- children's contributions per position of the blocked fronts
   P.gath0.assign(ns, 0);
@@ -518,7 +521,23 @@ bool sn_build_plan(const std::vector<SnInstance> &in, SnPlan &P, std::string *er
       panels_of(P.u0[big[L][a]], pl[a]);
       maxp = std::max(maxp, pl[a].size());
     }
+    bool pair = false;  // panels p - 1 and p (p odd), p and p + 1 (p even)
     for (size_t p = 0; p < maxp; ++p) {
+      // Panels go in pairs while what both leave fills the chip (two blocks on
+      // each of 148 SMs): the first one updates only the second one's columns,
+      // the second one the rest of the front for both.  Below that the update is
+      // one short wave either way (17 us a launch single, 20 paired, over 2 000
+      // second-order cones' fronts).
+      if (p % 2 == 0) {
+        long long tiles = 0;
+        for (size_t a = 0; a < big[L].size(); ++a)
+          if (p + 1 < pl[a].size()) {
+            const int s = big[L][a];
+            const long long t = (P.ld[s] - pl[a][p + 1].first - pl[a][p + 1].second) / kSnNB;
+            tiles += t * (t + 1);
+          }
+        pair = tiles > 2 * 148;
+      }
       // flops: 2 K^3 / 3 per diagonal block; K^2 per TRSM row; 2 K per
       // lower-triangle entry of the update
       b0 = (int)P.tasks.size();
@@ -536,8 +555,10 @@ bool sn_build_plan(const std::vector<SnInstance> &in, SnPlan &P, std::string *er
       for (size_t a = 0; a < big[L].size(); ++a) {
         if (p >= pl[a].size()) continue;
         const int s = big[L][a], k = pl[a][p].first, K = pl[a][p].second, e = k + K;
+        // the second panel of a pair keeps its W behind the first one's
+        const int w = pair && p % 2 ? pl[a][p - 1].second : 0;
         for (int r0 = e; r0 < P.ld[s]; r0 += kSnNB) {
-          P.tasks.push_back({s, kK(k, K), r0, 0});
+          P.tasks.push_back({s, kK(k, K), r0, w});
           fl += 1.0 * K * K * kSnNB;
         }
       }
@@ -547,10 +568,12 @@ bool sn_build_plan(const std::vector<SnInstance> &in, SnPlan &P, std::string *er
       fl = 0;
       for (size_t a = 0; a < big[L].size(); ++a) {
         if (p >= pl[a].size()) continue;
-        const int s = big[L][a], k = pl[a][p].first, K = pl[a][p].second, e = k + K;
+        const int s = big[L][a], e = pl[a][p].first + pl[a][p].second;
+        const int k = pl[a][pair ? p - p % 2 : p].first, K = e - k;
+        const int ce = pair && p % 2 == 0 && p + 1 < pl[a].size() ? e + pl[a][p + 1].second : P.ld[s];
         // 128 x 64 tiles: for every 64-column block, the 128-row tiles from
         // the one holding its diagonal down
-        for (int c0 = e; c0 < P.ld[s]; c0 += 64)
+        for (int c0 = e; c0 < ce; c0 += 64)
           for (int r0 = e + (c0 - e) / kSnNB * kSnNB; r0 < P.ld[s]; r0 += kSnNB) {
             P.tasks.push_back({s, kK(k, K), r0, c0});
             double below = 0;  // entries on or below the diagonal

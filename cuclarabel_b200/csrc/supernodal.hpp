@@ -75,9 +75,9 @@ enum SnLaunchKind : int {
   SN_SMALL_FACTOR = 0,  // {s}: assemble + factor a small front in shared memory
   SN_ASSEMBLE,          // {s, c_begin, c_end, chunk}: zero + assemble columns of a blocked front
   SN_DIAG,              // {s, k | K << 16}: factor the K x K diagonal block
-  SN_TRSM,              // {s, k | K << 16, r0}: rows r0..r0+127 of the panel: W = A L11^-T
+  SN_TRSM,              // {s, k | K << 16, r0, column of W}: rows r0..r0+127 of the panel: W = A L11^-T
                         //   by substitution, L = W D^-1
-  SN_UPDATE,            // {s, k | K << 16, r0, c0}: 128 x 64 tile (r0, c0) -= L(r0 rows) W(c0 rows)^T
+  SN_UPDATE,            // {s, k | K << 16, r0, c0} (K: a panel or a pair): 128 x 64 tile (r0, c0) -= L(r0 rows) W(c0 rows)^T
   SN_FWD_SMALL,         // {s}: forward substitution of a small front (one warp)
   SN_FWD_GATHER,        // (no launches: part of the next; the profile's layout is kept)
   SN_FWD_DIAG,          // {s, tile, ticket}: forward substitution of a blocked front's row tile
@@ -117,7 +117,7 @@ struct SnPlan {
   std::vector<int> inst, col0g, ncol, nrow, u0, ld, large, cbase, fix_off, rel_off, ch_ptr,
       uoff;
   std::vector<long long> foff;  // front offsets (elements, multiples of 32)
-  std::vector<long long> woff;  // factor workspace of blocked fronts: dinv (kSnNB), W (ld x kSnNB)
+  std::vector<long long> woff;  // factor workspace of blocked fronts: dinv (kSnNB), W (ld x kSnNB, or two panels)
   std::vector<long long> soff;  // substitution of blocked fronts: published x, forward (u0), backward (u0), tile sums
   std::vector<int> ch;          // children, in order
   std::vector<int> fidx;        // front position -> global vector index (-1 none)
