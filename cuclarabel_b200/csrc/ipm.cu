@@ -1063,38 +1063,49 @@ static std::vector<long long> prefix(const std::vector<T> &counts) {
   return off;
 }
 
-// Concatenates the prepared instances into the batch layout and uploads it.
-// Every per-instance copy runs on nth host threads: offsets first (prefix
-// sums over instances), then each instance fills its own disjoint slices.
-// Launch groups of one kind: instances (sorted by decreasing need of shared
-// memory) that fit 4, 2 or 1 blocks per SM; a group's launches are sized for
-// its largest member.  Finer groups lose: groups run one after the other, and
-// at 4096 MPC instances two more of them took the two-side solves from 10.5 to
-// 14.0 ms.
-static SlGroups sl_groups(const std::vector<int> &items, const std::vector<long long> &need,
-                          const std::vector<long long> &need2) {
+// Dynamic shared memory of one class-1 instance (ldl_sliced.cu): solves with one
+// and two sides, the factorisation in FP64 and in FP32.
+struct SlNeed {
+  long long solve[2], factor[2];
+};
+static SlNeed sl_need(const SlicedPlan &p) {
+  const long long ring = (long long)kSlRing * kSlStage * (8 * kSlRun + 16) +
+                         (((long long)p.used.size() + 15) & ~15LL);
+  const long long slots = 2LL * p.N + 1 + p.ncarry;
+  const long long tab = (long long)kSlWarps * kSlOpRing * 512 + ((p.N + 15) & ~15LL);
+  const long long V = (long long)p.N + p.nl + 1 + p.nopcarry;
+  return {{ring + 8 * slots, ring + 16 * slots}, {tab + 8 * V, tab + 4 * V}};
+}
+
+// Launch groups of one kind: instances that fit 4, 2 or 1 blocks per SM, each
+// group's launches sized for its largest member.  The larger of the two needs
+// picks the group and orders the items (by it the groups are runs; by one need
+// alone they alternate, as the solves' stage table is in both needs once).
+// Finer groups lose: groups run one after the other, and at 4096 MPC instances
+// two more of them took the two-side solves from 10.5 to 14.0 ms.
+static SlGroups sl_groups(std::vector<int> &items, const std::vector<SlNeed> &need,
+                          long long (SlNeed::*kind)[2]) {
   SlGroups g{};
-  static constexpr long long cap[3] = {227 * 1024, 113 * 1024, 56 * 1024};
-  auto band = [&](int i) {
-    int c = 0;
-    while (c < 2 && std::max(need[i], need2[i]) <= cap[c + 1]) ++c;
-    return c;
-  };
-  for (size_t t = 0; t < items.size();) {
-    size_t u = t;
-    SlGroup gr{(int)t, 0, 0, 0};
-    while (u < items.size() && band(items[u]) == band(items[t])) {
-      gr.smem = std::max(gr.smem, (int)need[items[u]]);
-      gr.smem2 = std::max(gr.smem2, (int)need2[items[u]]);
-      ++u;
+  static constexpr long long cap[2] = {113 * 1024, 56 * 1024};
+  auto most = [&](int i) { return std::max((need[i].*kind)[0], (need[i].*kind)[1]); };
+  std::stable_sort(items.begin(), items.end(), [&](int a, int b) { return most(a) > most(b); });
+  auto t = items.begin();
+  for (int c = 0; c < 3; ++c) {
+    const auto u = std::find_if(t, items.end(), [&](int i) { return c < 2 && most(i) <= cap[c]; });
+    if (u == t) continue;
+    SlGroup &gr = g.g[g.n++];
+    gr = {(int)(t - items.begin()), (int)(u - t), 0, 0};
+    for (; t != u; ++t) {
+      gr.smem = std::max(gr.smem, (int)(need[*t].*kind)[0]);
+      gr.smem2 = std::max(gr.smem2, (int)(need[*t].*kind)[1]);
     }
-    gr.count = (int)(u - t);
-    g.g[g.n++] = gr;
-    t = u;
   }
   return g;
 }
 
+// Concatenates the prepared instances into the batch layout and uploads it.
+// Every per-instance copy runs on nth host threads: offsets first (prefix
+// sums over instances), then each instance fills its own disjoint slices.
 static int build_batch(clgpu_solver *h, std::vector<Prepared> &prep, int nth) {
   DevArena &A = h->arena;
   const int B = (int)prep.size();
@@ -1616,6 +1627,7 @@ static int build_batch(clgpu_solver *h, std::vector<Prepared> &prep, int nth) {
     const auto opage = prefix(cpage), olane = prefix(clane), ovp = prefix(cvp), oop = prefix(cop), oecol = prefix(cecol);
     if (olane[B] * 4 > 2000000000LL || oop[B] * kSlOpWords > 2000000000LL) return -4;
     std::vector<SlInst> sl(B);
+    std::vector<SlNeed> need(B);
     hvec<uint16_t> kdst((size_t)knz), lpos(ovp[B] * kSlRun), leaf(VT), ecols(oecol[B]);
     hvec<uint32_t> ent(olane[B] * 4), ops(oop[B] * kSlOpWords);
     hvec<int> kdiag(VT);
@@ -1626,6 +1638,7 @@ static int build_batch(clgpu_solver *h, std::vector<Prepared> &prep, int nth) {
       d = SlInst{};
       if (cls[i] != 1) return;
       SlicedPlan &sp = plan[i];
+      need[i] = sl_need(sp);
       d.N = sp.N;
       d.nl = sp.nl;
       d.nk = (int)sp.kslot.size();
@@ -1685,31 +1698,14 @@ static int build_batch(clgpu_solver *h, std::vector<Prepared> &prep, int nth) {
     const size_t nval = (size_t)(ovp[B] * kSlRun);
     kk.sl_val = h->mixed ? (void *)A.alloc<float>(nval, false) : A.alloc<double>(nval, false);
     // launch order: the largest need of shared memory first
-    std::vector<long long> s1(B, 0), s2(B, 0), f1(B, 0), f2(B, 0);
-    std::vector<int> items;
+    std::vector<int> so, fo;
     for (int i = 0; i < B; ++i)
-      if (cls[i] == 1) {
-        items.push_back(i);
-        const SlInst &d = sl[i];
-        const long long ring = (long long)kSlRing * kSlStage * (8 * kSlRun + 16) +
-                               (((long long)cpage[i] + 15) & ~15LL);
-        const long long slots = 2LL * N[i] + 1 + d.ncarry;
-        s1[i] = ring + 8 * slots;
-        s2[i] = ring + 16 * slots;
-        const long long tab = (long long)kSlWarps * kSlOpRing * 512 + ((N[i] + 15) & ~15LL);
-        f1[i] = tab + 8LL * (N[i] + d.nl + 1 + d.nopcarry);
-        f2[i] = tab + 4LL * (N[i] + d.nl + 1 + d.nopcarry);
-      }
-    auto order = [&](const std::vector<long long> &need) {
-      std::vector<int> v = items;
-      std::stable_sort(v.begin(), v.end(), [&](int a, int b) { return need[a] > need[b]; });
-      return v;
-    };
-    const auto so = order(s1), fo = order(f1);
+      if (cls[i] == 1) so.push_back(i);
+    fo = so;
+    kk.sl_solve = sl_groups(so, need, &SlNeed::solve);
+    kk.sl_factor = sl_groups(fo, need, &SlNeed::factor);
     kk.sl_solve_inst = A.upload(so);
     kk.sl_factor_inst = A.upload(fo);
-    kk.sl_solve = sl_groups(so, s1, s2);
-    kk.sl_factor = sl_groups(fo, f1, f2);
     mark("sliced upload");
   }
   kk.cls = A.upload(cls);
@@ -1929,6 +1925,52 @@ static int build_batch(clgpu_solver *h, std::vector<Prepared> &prep, int nth) {
   if (e != cudaSuccess) return -1000 - (int)e;
   A.settle();  // the uploads have completed: their host sources go back to the pool
   mark("scratch + tail");
+  return 0;
+}
+
+// The launch groups build_batch forms of n problems as one batch (solves and
+// factorisations of the class-1 instances): counts[0..1] the groups, counts[2]
+// the class-1 instances.  0, -2 when an instance cannot be prepared, -3 when a
+// group's launches are too small for a member or a block cannot have them, -4
+// when the groups do not cover the class-1 instances once each.
+extern "C" int clgpu_debug_launch_groups(const clgpu_problem *pbs, int n, const clgpu_settings *st,
+                                         int *counts) {
+  using namespace clgpu;
+  if (!pbs || n < 0 || !counts) return -1;
+  SetupOptions opt;
+  if (st) {
+    opt.equilibrate_enable = st->equilibrate_enable;
+    if (st->soc_threshold > 0) opt.soc_threshold = st->soc_threshold;
+  }
+  std::vector<SlNeed> need(n);
+  std::vector<int> items;
+  const bool mixed = st && st->direct_solve_method != CLGPU_METHOD_FP64;
+  for (int i = 0; i < n; ++i) {
+    Prepared p;
+    SlicedPlan sp;
+    if (!prepare_instance(pbs[i], opt, p)) return -2;
+    if (!sl_fits(p) || !sl_build(p, mixed ? 4 : 2, sp)) continue;
+    need[i] = sl_need(sp);
+    items.push_back(i);
+  }
+  counts[2] = (int)items.size();
+  int k = 0;
+  for (auto kind : {&SlNeed::solve, &SlNeed::factor}) {
+    std::vector<int> order = items;
+    const SlGroups g = sl_groups(order, need, kind);
+    counts[k++] = g.n;
+    int next = 0;
+    for (int a = 0; a < g.n; ++a) {
+      if (g.g[a].first != next || g.g[a].count <= 0) return -4;
+      next += g.g[a].count;
+      for (int t = g.g[a].first; t < next; ++t) {
+        const long long *q = need[order[t]].*kind;
+        if (q[0] > g.g[a].smem || q[1] > g.g[a].smem2 || std::max(q[0], q[1]) > kSlSmemMax)
+          return -3;
+      }
+    }
+    if (next != (int)order.size()) return -4;
+  }
   return 0;
 }
 

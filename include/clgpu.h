@@ -471,6 +471,14 @@ int clgpu_debug_instance_path(const clgpu_problem *prob, const clgpu_settings *s
  * when N > 2000, other negative codes for structure errors.  Needs no GPU. */
 int clgpu_debug_factor_stream(const clgpu_problem *prob, const clgpu_settings *settings,
                               double *resid);
+/* Host-only view of the launches of the block-per-instance LDL^T when n
+ * problems are set up as one batch (diagnostic, no reference counterpart):
+ * counts[0] launches of a solve, counts[1] of a factorisation (at most three
+ * each, by shared memory), counts[2] instances that take these kernels.
+ * Returns 0, -2 when an instance cannot be prepared, other negative codes when
+ * a launch would not fit its members.  Needs no GPU. */
+int clgpu_debug_launch_groups(const clgpu_problem *probs, int n, const clgpu_settings *settings,
+                              int *counts);
 /* Counters of the process-wide page-locked host pool that setup arrays,
  * upload staging and result staging come from (diagnostic, no reference
  * counterpart): out[0] buffers served from the pool, out[1] page-locked

@@ -98,3 +98,21 @@ def test_banded_problems_keep_dissection(seed):
     sn, ent = _entries(pb)
     nnz = 2 * pb[2].nnz + n + m  # K without the cones' blocks
     assert sn == 0 and ent > 0.5 * nnz
+
+
+@pytest.mark.parametrize("method", ["cudss", "cudssmixed"])
+def test_launch_groups_of_needs_around_a_threshold(method):
+    """The first two need the same shared memory with one side and, with two,
+    exactly 56 KB and 16 bytes more (the stage table is in both needs once), so
+    by the one-side need alone they alternate between two launch groups.  Any
+    batch takes at most three launches of each kind, every instance in one."""
+    from cuclarabel_b200._lib import ClgpuProblem
+    pair = [problems.mpc_qp(557, n=440), problems.mpc_qp(64, n=443)]
+    pbs = pair * 5 + [problems.mpc_qp(5, n=n) for n in (20, 430, 1000)]
+    base = [_prep_problem(*p) for p in pbs]
+    arr = (ClgpuProblem * len(base))(*[b[0] for b in base])
+    st = Settings(direct_solve_method=method).to_c()
+    counts = (ctypes.c_int * 3)()
+    rc = _lib.load().clgpu_debug_launch_groups(arr, len(base), ctypes.byref(st), counts)
+    assert rc == 0 and counts[2] == len(base)
+    assert 1 <= counts[0] <= 3 and 1 <= counts[1] <= 3, list(counts)
