@@ -1678,6 +1678,7 @@ __global__ void __launch_bounds__(kPsdEigThreads) k_psd_step_eig(ConeSet cs, dou
   const int c = (first + tid) >> 1, inst = cs.psd_inst[c];
   if (!active_inst(cs, inst)) return;
   const int n = cs.psd_n[c];
+  if (n == 0) return;  // no eigenvalue
   // tridiagonal form: diagonal d, subdiagonal e[1 .. n - 1]
   for (int i = n - 1; i > 0; --i) {
     double *Ai = A + W * (i * (i + 1) / 2);

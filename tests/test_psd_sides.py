@@ -100,3 +100,21 @@ def test_psd_scaling_failure_small_side(cuda_device):
     assert G.L.clgpu_update_scaling(G.h, d_s.data_ptr(), d_s.data_ptr(), 1.0, 0, None) == 0
     assert G.L.clgpu_update_scaling(G.h, d_b.data_ptr(), d_s.data_ptr(), 1.0, 0, None) != 0
     assert G.L.clgpu_update_scaling(G.h, d_s.data_ptr(), d_b.data_ptr(), 1.0, 0, None) != 0
+
+
+@pytest.mark.parametrize("sides", [[0, 0], [0, 3, 0, 5], [0, 17]])
+def test_psd_empty_cones_set_no_limit(cuda_device, sides):
+    """A cone of side 0 has no eigenvalue and limits no step, alone, beside
+    small cones and beside large ones."""
+    specs = [(5, n, 0.0) for n in sides]
+    G = GPUCones(specs)
+    s = svec_eye(sides, 1.0)
+    d_s, d_d = G.dev(np.append(s, 0.0)), G.dev(np.append(-0.5 * s, 0.0))
+    assert G.L.clgpu_update_scaling(G.h, d_s.data_ptr(), d_s.data_ptr(), 1.0, 0, None) == 0
+    for _ in range(3):
+        a = ctypes.c_double()
+        assert G.L.clgpu_step_length(G.h, d_d.data_ptr(), d_d.data_ptr(), d_s.data_ptr(),
+                                     d_s.data_ptr(), 5.0, 0.99, 0.8, 1e-4, ctypes.byref(a),
+                                     None) == 0
+        # the other cones' step to the boundary is 2
+        assert a.value == pytest.approx(2.0 if max(sides) else 5.0, rel=1e-12)
