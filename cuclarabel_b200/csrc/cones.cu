@@ -1679,14 +1679,32 @@ __global__ void __launch_bounds__(kPsdEigThreads) k_psd_step_eig(ConeSet cs, dou
   if (!active_inst(cs, inst)) return;
   const int n = cs.psd_n[c];
   if (n == 0) return;  // no eigenvalue
+  // The largest entry.  Away from the middle of FP64's range the matrix is scaled
+  // by a power of two, so that no square below overflows and a row whose squares
+  // underflow is negligible beside it.  An infinite entry: the smallest diagonal
+  // one stands for the eigenvalue (the Jacobi iteration of the larger sides takes
+  // such a matrix for converged); a NaN sets no limit.
+  double big = 0;
+  bool nan = false;
+  for (int k = 0; k < n * (n + 1) / 2; ++k) {
+    const double v = fabs(A[W * k]);
+    nan = nan || isnan(v);
+    big = fmax(big, v);
+  }
+  if (nan) return;
+  int shift = 0;
+  if (isfinite(big) && big > 0 && !(big > 0x1p-400 && big < 0x1p400)) {
+    shift = ilogb(big);
+    for (int k = 0; k < n * (n + 1) / 2; ++k) A[W * k] = scalbn(A[W * k], -shift);
+  }
   // tridiagonal form: diagonal d, subdiagonal e[1 .. n - 1]
-  for (int i = n - 1; i > 0; --i) {
+  for (int i = n - 1; i > 0 && isfinite(big); --i) {
     double *Ai = A + W * (i * (i + 1) / 2);
     const int l = i - 1;
     double h = 0;
     for (int k = 0; k < l; ++k) h += Ai[W * k] * Ai[W * k];
     const double f = Ai[W * l];
-    if (h == 0) {  // already tridiagonal here
+    if (h < 0x1p-1022) {  // already tridiagonal here (1 / h would overflow)
       e[W * i] = f;
       continue;
     }
@@ -1716,7 +1734,9 @@ __global__ void __launch_bounds__(kPsdEigThreads) k_psd_step_eig(ConeSet cs, dou
   }
   for (int i = 0; i < n; ++i) d[W * i] = A[W * (i * (i + 1) / 2 + i)];
   double gmin = d[0];
-  if (n > 1) {
+  if (!isfinite(big)) {
+    for (int i = 1; i < n; ++i) gmin = fmin(gmin, d[W * i]);
+  } else if (n > 1) {
     // Laguerre's iteration on det(T - x I) from Gershgorin's lower bound: the
     // roots are real, so x rises to the smallest one monotonically.  With the
     // pivots q of T - x I, G = sum 1 / (lambda - x) is the sum of the g = -q'/q
@@ -1727,8 +1747,7 @@ __global__ void __launch_bounds__(kPsdEigThreads) k_psd_step_eig(ConeSet cs, dou
       const double r =
           (i > 0 ? fabs(e[W * i]) : 0.0) + (i + 1 < n ? fabs(e[W * (i + 1)]) : 0.0);
       x = fmin(x, d[W * i] - r);
-      if (!(fabs(d[W * i]) + r <= norm)) norm = fabs(d[W * i]) + r;
-      if (!isfinite(norm)) return;  // no eigenvalue to limit the step by
+      norm = fmax(norm, fabs(d[W * i]) + r);
     }
     x -= kDEps * norm;
     for (int it = 0; it < 100; ++it) {
@@ -1752,6 +1771,7 @@ __global__ void __launch_bounds__(kPsdEigThreads) k_psd_step_eig(ConeSet cs, dou
     }
     gmin = x;
   }
+  gmin = scalbn(gmin, shift);
   const double amax = alpha[inst];
   if (gmin < 0) atomic_min_nonneg_filtered(alpha + inst, fmin(1.0 / (-gmin), amax));
 }

@@ -118,3 +118,44 @@ def test_psd_empty_cones_set_no_limit(cuda_device, sides):
                                      None) == 0
         # the other cones' step to the boundary is 2
         assert a.value == pytest.approx(2.0 if max(sides) else 5.0, rel=1e-12)
+
+
+@pytest.mark.parametrize("n", [4, 16])
+@pytest.mark.parametrize("coupling", [3e-155, 1e-158, 1e-161, 1e-170, 1e-320, 0.25])
+@pytest.mark.parametrize("scale", [1.0, 1e-300, 1e-150, 1e155, 1e250])
+def test_psd_step_at_the_ends_of_the_range(cuda_device, n, coupling, scale):
+    """s = z = I, so the step's matrix is the direction itself: rows whose squares
+    leave FP64's range, beside entries of order one and alone.  The eigenvalue's
+    error is at most about n^1.5 eps |A|, and |A| is of its own order: far below
+    the 1e-12 asked for."""
+    G = GPUCones([(5, n, 0.0)] * 3)
+    s = svec_eye([n] * 3, 1.0)
+    d_s = G.dev(s)
+    assert G.L.clgpu_update_scaling(G.h, d_s.data_ptr(), d_s.data_ptr(), 1.0, 0, None) == 0
+    M = np.full((n, n), coupling) * np.sign(np.sin(np.add.outer(np.arange(n), np.arange(n)) + 1.0))
+    M[np.diag_indices(n)] = np.resize([-4.0, -1.0, 2.0, 3.0], n)
+    low = np.linalg.eigvalsh(M)[0]
+    v = np.array([M[i, j] * (1.0 if i == j else np.sqrt(2))
+                  for j in range(n) for i in range(j + 1)]) * scale
+    for ds in (np.concatenate([0 * v, v, 0 * v]), np.concatenate([-v[:1] * np.abs(s[:len(v)]), v, v])):
+        a = ctypes.c_double()
+        d_d, zero = G.dev(ds), G.dev(0 * ds)
+        assert G.L.clgpu_step_length(G.h, d_d.data_ptr(), zero.data_ptr(), d_s.data_ptr(),
+                                     d_s.data_ptr(), 1e305, 0.99, 0.8, 1e-4, ctypes.byref(a),
+                                     None) == 0
+        assert a.value == pytest.approx(1.0 / (-low * scale), rel=1e-12, abs=0)
+
+
+def test_psd_step_of_directions_that_are_not_finite(cuda_device):
+    """As the iteration of the larger sides answers: a NaN sets no limit, an
+    infinite direction of a 1 x 1 cone a step of zero."""
+    for n, value, want in ((5, np.nan, 1.0), (1, -np.inf, 0.0), (1, np.inf, 1.0)):
+        G = GPUCones([(5, n, 0.0)])
+        d_s = G.dev(svec_eye([n], 1.0))
+        d_d, zero = G.dev(np.full(n * (n + 1) // 2, value)), G.dev(np.zeros(n * (n + 1) // 2))
+        assert G.L.clgpu_update_scaling(G.h, d_s.data_ptr(), d_s.data_ptr(), 1.0, 0, None) == 0
+        a = ctypes.c_double()
+        assert G.L.clgpu_step_length(G.h, d_d.data_ptr(), zero.data_ptr(), d_s.data_ptr(),
+                                     d_s.data_ptr(), 1.0, 0.99, 0.8, 1e-4, ctypes.byref(a),
+                                     None) == 0
+        assert a.value == want, (n, value, a.value)
