@@ -903,7 +903,7 @@ struct clgpu_solver {
     for (auto ex : pass_exec)
       if (ex) cudaGraphExecDestroy(ex);
     if (h_counter) pinned_give(h_counter);
-    if (st_own) cudaStreamDestroy(st_own);  // (every solve waits for its work)
+    if (st_cap) cudaStreamDestroy(st_cap);
     if (st_admit) {
       cudaStreamSynchronize(st_admit);
       cudaStreamDestroy(st_admit);
@@ -925,7 +925,7 @@ struct clgpu_solver {
     }
     return (int)ev_next++;
   }
-  cudaStream_t st_own = nullptr;  // solves asked for on the legacy stream
+  cudaStream_t st_cap = nullptr;  // the pass is captured on it; nothing runs there
   bool graph_ok() const {
     return use_graphs && !any_asym && !any_sn && !profiling && !st.verbose &&
            !std::isfinite(st.time_limit);
@@ -2477,11 +2477,15 @@ static void ipm_pass_kernels(clgpu_solver *h, Phase &P, cudaStream_t st, double 
 // h->h_list (count in *nfin).  Without host decisions inside the pass (no
 // asymmetric-cone backtracking, no profiling or tracing, no time limit) the
 // pass is captured once as a CUDA graph and replayed: one launch instead of
-// ~60.  A solver's first solve launches kernel by kernel: capturing and
+// 45.  A solver's first solve launches kernel by kernel: capturing and
 // instantiating the graph costs more than the launches of one solve, so a
 // solver used once (a cold pass) never pays it; the second solve captures.
 // The serving steps capture at once (their lanes warm up before serving, and
-// no capture may be open while other threads allocate).
+// no capture may be open while other threads allocate).  The capture is on a
+// stream that the legacy stream does not wait for: while a blocking stream (or
+// the caller's, which may be one) captures, any use of the legacy stream in any
+// thread is an error and ends the capture.  The graph is replayed on the
+// caller's stream, the legacy one included.
 static int ipm_pass(clgpu_solver *h, Phase &P, cudaStream_t st, double elapsed, bool serve,
                     int *nfin) {
   Dev &dv = h->dv;
@@ -2493,9 +2497,14 @@ static int ipm_pass(clgpu_solver *h, Phase &P, cudaStream_t st, double elapsed, 
     if (!ex) {
       cudaGraph_t g = nullptr;
       const long long l0 = h->launches;
-      if (cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
-        ipm_pass_kernels(h, P, st, 0.0, serve);
-        if (cudaStreamEndCapture(st, &g) == cudaSuccess && g) {
+      if (!h->st_cap &&
+          cudaStreamCreateWithFlags(&h->st_cap, cudaStreamNonBlocking) != cudaSuccess)
+        h->st_cap = nullptr;
+      Phase C{h, h->st_cap, P.dp, P.cp};
+      if (h->st_cap &&
+          cudaStreamBeginCapture(h->st_cap, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
+        ipm_pass_kernels(h, C, h->st_cap, 0.0, serve);
+        if (cudaStreamEndCapture(h->st_cap, &g) == cudaSuccess && g) {
           if (cudaGraphInstantiate(&ex, g, 0) != cudaSuccess) ex = nullptr;
           cudaGraphDestroy(g);
         }
@@ -2570,16 +2579,6 @@ extern "C" int clgpu_solver_solve(clgpu_solver *h, clgpu_stream_t stream) {
   if (!h) return -1;
   cudaStream_t st = (cudaStream_t)stream;
   auto t0 = std::chrono::steady_clock::now();
-  // The legacy stream cannot be captured: a solve on it runs on a stream of
-  // the solver's own that orders itself with the legacy stream (a blocking
-  // stream), so its passes are replayed as a graph too.
-  if (!st && h->graph_ok() && h->solves_done > 0) {
-    if (!h->st_own && cudaStreamCreate(&h->st_own) != cudaSuccess) {
-      cudaGetLastError();
-      h->st_own = nullptr;
-    }
-    if (h->st_own) st = h->st_own;
-  }
   Phase P{h, st};
   Dev &dv = h->dv;
   const int B = h->B;
