@@ -34,9 +34,16 @@ constexpr unsigned kFull = 0xffffffffu;
 __device__ __forceinline__ void cp16(unsigned dst, const void *src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src));
 }
+// The block meets, its warps at different places of the code: the copying warp and
+// the adding ones in the solves, warps with different numbers of pages in the
+// factorisation.  (__syncthreads is only defined where the whole block takes the
+// same path; barrier.sync counts the warps that arrive.)
+__device__ __forceinline__ void meet() {
+  asm volatile("barrier.sync.aligned 1, %0;\n" ::"n"(kNT) : "memory");
+}
 __device__ __forceinline__ void meet(int n) {
 #pragma unroll 1
-  for (; n > 0; --n) __syncthreads();
+  for (; n > 0; --n) meet();
 }
 
 // The block's stage ring in shared memory: the forward, backward and residual
@@ -131,7 +138,7 @@ __device__ __forceinline__ void sl_stages(Ring<T> &ring, int ns, int N, double *
     for (; ns > 0; --ns) {
       ring.issue(tid - kSlStage);
       ring.landed();
-      __syncthreads();
+      meet();
     }
     return;
   }
@@ -198,7 +205,7 @@ __device__ __forceinline__ void sl_stages(Ring<T> &ring, int ns, int N, double *
       }
     }
     ring.take(tid);
-    __syncthreads();
+    meet();
   }
 }
 
