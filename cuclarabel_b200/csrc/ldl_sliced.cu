@@ -32,7 +32,7 @@ constexpr int kNT = 32 * kSlWarps;
 constexpr unsigned kFull = 0xffffffffu;
 
 __device__ __forceinline__ void cp16(unsigned dst, const void *src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src));
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
 }
 // The block meets, its warps at different places of the code: the copying warp and
 // the adding ones in the solves, warps with different numbers of pages in the
@@ -84,7 +84,7 @@ struct Ring {
         cp16(s + kVals + 16 * l, words + 512 * h);
       }
     }
-    asm volatile("cp.async.commit_group;\n" ::);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
     words += 16 * nu;
     (fac ? vals : kvals) += 16 * halves * nu;
     if (++at == n) {
@@ -97,7 +97,7 @@ struct Ring {
   }
   // stages up to the one after the next are in shared memory
   __device__ __forceinline__ void landed() {
-    asm volatile("cp.async.wait_group %0;\n" ::"n"(kSlRing - 2));
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(kSlRing - 2) : "memory");
   }
   __device__ __forceinline__ void take(int tid) {
     const int nu = table[cur];
@@ -433,7 +433,7 @@ __global__ void __launch_bounds__(kNT, kSlSolveBlocks)
     block_max_nr<1>(bad, red);
     if (bad[0] > 0.0) good = false;
   }
-  asm volatile("cp.async.wait_all;\n" ::);  // stages of a round that is not run
+  asm volatile("cp.async.wait_all;\n" ::: "memory");  // stages of a round that is not run
   if (k.prof_bytes && tid == 0) {
     // algorithmic bytes: a substitution reads the factor (value + word per
     // entry, both directions) and D^-1, a residual reads K (value + word);
@@ -514,7 +514,7 @@ __global__ void __launch_bounds__(kNT, kSlFactorBlocks)
 #pragma unroll
   for (int h = 0; h < kSlOpRing; ++h) {
     if (h < nop) cp16(oaddr + 512 * h, ops + (size_t)h * 512);
-    asm volatile("cp.async.commit_group;\n" ::);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
   }
   // ---- K into the work positions, the diagonal's static regularisation
   for (int i = tid; i < N + nl + 1 + si.nopcarry; i += kNT) V[i] = A(0);
@@ -578,10 +578,10 @@ __global__ void __launch_bounds__(kNT, kSlFactorBlocks)
   int slot = 0;
   // op page p into registers, its slot refilled; one page ahead of use
   auto take = [&](int p) {
-    asm volatile("cp.async.wait_group %0;\n" ::"n"(kSlOpRing - 1));
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(kSlOpRing - 1) : "memory");
     o = *reinterpret_cast<const uint4 *>(oring + 512 * slot + 16 * lane);
     if (p + kSlOpRing < nop) cp16(oaddr + 512 * slot, ops + (size_t)(p + kSlOpRing) * 512);
-    asm volatile("cp.async.commit_group;\n" ::);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
     slot = slot + 1 == kSlOpRing ? 0 : slot + 1;
   };
   if (nop > 0) take(0);  // (a lane reads back the 16 bytes it copied)
