@@ -343,8 +343,8 @@ __global__ void __launch_bounds__(kNT, kSlSolveBlocks)
                               [](uint32_t, double (&)[NR]) {});
     }
   };
-  // e_r = b_r - K y_r; norme[r] = ||e_r||_inf (+inf when not finite)
-  auto residual = [&](unsigned m, double (&norme)[NR]) {
+  // e_r = b_r - K y_r; norme[r] = ||e_r||_inf (+inf when not finite), the sides on[r]
+  auto residual = [&](const bool (&on)[NR], double (&norme)[NR]) {
     ++nres;
     double mx[NR];
 #pragma unroll
@@ -352,7 +352,7 @@ __global__ void __launch_bounds__(kNT, kSlSolveBlocks)
     sl_stages<T, NR, true>(ring, nr, N, y, tid, [&](uint32_t t, double (&sum)[NR]) {
 #pragma unroll
       for (int r = 0; r < NR; ++r)
-        if ((m >> r) & 1u) {
+        if (on[r]) {
           const double ev = __dsub_rn(b[t * NR + r], sum[r]);
           e[r][t] = ev;
           mx[r] = fmax(mx[r], isfinite(ev) ? fabs(ev) : CUDART_INF);
@@ -361,36 +361,49 @@ __global__ void __launch_bounds__(kNT, kSlSolveBlocks)
     block_max_nr<NR>(mx, red);
 #pragma unroll
     for (int r = 0; r < NR; ++r)
-      if ((m >> r) & 1u) norme[r] = mx[r];
+      if (on[r]) norme[r] = mx[r];
   };
-  constexpr unsigned all = (1u << NR) - 1u;
   trisolve();
   bool good = true;
   if (prm.ir_enable) {
     // x keeps the accepted iterate; y holds the candidate the residual reads.
-    // m: the sides still refining.  Its value is passed through an empty asm:
-    // without it the two-side build drops the sweeps (seen as results that
-    // differ from the one-side kernel's, which a test compares bit for bit).
+    // One thread decides which sides go on and leaves it in shared memory: a
+    // sweep has meetings of the whole block, so the block follows one decision.
+    // (As a bit mask in a register of every thread, nvcc 12.9 drops the two-side
+    // build's sweeps.  It is its optimiser, before ptxas: the same with ptxas at
+    // -O1, right when written with a flag per side.  The one-side results, which
+    // the two-side ones equal bit for bit, show it.)
+    __shared__ bool todo[NR];
+    bool on[NR];
     double norme[NR], tol[NR];
-    residual(all, norme);
-    unsigned m = 0;
+#pragma unroll
+    for (int r = 0; r < NR; ++r) on[r] = true;
+    residual(on, norme);
 #pragma unroll
     for (int r = 0; r < NR; ++r) {
       tol[r] = prm.ir_abstol + prm.ir_reltol * normb[r];
       for (int i = tid; i < N; i += kNT) x[r][i] = y[i * NR + r];
       good = good && isfinite(norme[r]);
-      if (norme[r] > tol[r]) m |= 1u << r;
     }
-    if (!good) m = 0;
-    asm volatile("" : "+r"(m));
-#pragma unroll 1
-    for (int it = 0; m && it < prm.ir_maxiter; ++it) {
+    if (tid == 0) {
+#pragma unroll
+      for (int r = 0; r < NR; ++r) todo[r] = good && norme[r] > tol[r];
+    }
+    __syncthreads();
+    for (int it = 0; it < prm.ir_maxiter; ++it) {
+      bool any = false;
+#pragma unroll
+      for (int r = 0; r < NR; ++r) {
+        on[r] = todo[r];
+        any = any || on[r];
+      }
+      if (!any) break;
       double last[NR];
       // (block_max_nr has synchronised since the last reads of y)
 #pragma unroll
       for (int r = 0; r < NR; ++r) {
         last[r] = norme[r];
-        if ((m >> r) & 1u) {
+        if (on[r]) {
           ++nir;
           SL_VEC(i, N, tv[u] = e[r][i];, y[i * NR + r] = tv[u];)
         }
@@ -399,14 +412,13 @@ __global__ void __launch_bounds__(kNT, kSlSolveBlocks)
       trisolve();
 #pragma unroll
       for (int r = 0; r < NR; ++r)
-        if ((m >> r) & 1u)
+        if (on[r])
           SL_VEC(i, N, tv[u] = x[r][i];, y[i * NR + r] += tv[u];)
       __syncthreads();
-      residual(m, norme);
-      unsigned next = 0;
+      residual(on, norme);
 #pragma unroll
       for (int r = 0; r < NR; ++r)
-        if ((m >> r) & 1u) {
+        if (on[r]) {
           if (isfinite(norme[r])) {
             // kktsolver_directldl_gpu.jl:390-400: keep the candidate if it
             // improved on the last error; stop when the improvement ratio is
@@ -414,13 +426,17 @@ __global__ void __launch_bounds__(kNT, kSlSolveBlocks)
             const double ratio = last[r] / norme[r];
             if (ratio > 1.0 || ratio >= prm.ir_stopratio)
               for (int i = tid; i < N; i += kNT) x[r][i] = y[i * NR + r];
-            if (!(ratio < prm.ir_stopratio) && norme[r] > tol[r]) next |= 1u << r;
+            on[r] = !(ratio < prm.ir_stopratio) && norme[r] > tol[r];
           } else {
             good = false;
           }
         }
-      m = good ? next : 0u;
-      asm volatile("" : "+r"(m));
+      // (every thread has read todo before the sweep's meetings)
+      if (tid == 0) {
+#pragma unroll
+        for (int r = 0; r < NR; ++r) todo[r] = good && on[r];
+      }
+      __syncthreads();
     }
   } else {
     double bad[1] = {0.0};

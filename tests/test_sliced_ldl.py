@@ -70,6 +70,19 @@ def test_mixed_sizes_give_the_bits_of_each_alone(cuda_device, method):
         assert np.array_equal(a.x, s.x) and np.array_equal(a.s, s.s) and np.array_equal(a.z, s.z)
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("method", ["cudss", "cudssmixed", "mixed_f64elim"])
+def test_two_sides_in_one_launch_are_each_its_own_solve(cuda_device, method):
+    """Bit for bit, refinement included (the FP32 factors need several sweeps,
+    and the two sides stop after different numbers of them)."""
+    pbs = [c() for c in CASES.values()] + [problems.portfolio(2, 50, 5), problems.mpc_qp(7, n=900)]
+    opts = dict(direct_solve_method=method, max_iter=8)
+    for a, b in zip(BatchSolver(pbs, fused_solves=True, **opts).solve(),
+                    BatchSolver(pbs, fused_solves=False, **opts).solve()):
+        assert a.status == b.status and a.iterations == b.iterations
+        assert np.array_equal(a.x, b.x) and np.array_equal(a.s, b.s) and np.array_equal(a.z, b.z)
+
+
 def _entries(pb):
     cp, keep, n, m = _prep_problem(*pb)
     st = Settings().to_c()
