@@ -1063,20 +1063,6 @@ static std::vector<long long> prefix(const std::vector<T> &counts) {
   return off;
 }
 
-// Dynamic shared memory of one class-1 instance (ldl_sliced.cu): solves with one
-// and two sides, the factorisation in FP64 and in FP32.
-struct SlNeed {
-  long long solve[2], factor[2];
-};
-static SlNeed sl_need(const SlicedPlan &p) {
-  const long long ring = (long long)kSlRing * kSlStage * (8 * kSlRun + 16) +
-                         (((long long)p.used.size() + 15) & ~15LL);
-  const long long slots = 2LL * p.N + 1 + p.ncarry;
-  const long long tab = (long long)kSlWarps * kSlOpRing * 512 + ((p.N + 15) & ~15LL);
-  const long long V = (long long)p.N + p.nl + 1 + p.nopcarry;
-  return {{ring + 8 * slots, ring + 16 * slots}, {tab + 8 * V, tab + 4 * V}};
-}
-
 // Launch groups of one kind: instances that fit 4, 2 or 1 blocks per SM, each
 // group's launches sized for its largest member.  The larger of the two needs
 // picks the group and orders the items (by it the groups are runs; by one need
@@ -2058,17 +2044,23 @@ extern "C" int clgpu_debug_factor_stream(const clgpu_problem *pb, const clgpu_se
         };
         double x[32];
         for (int t = 0; t < 32; ++t) {
-          for (int b = 0; b < 8; ++b)
-            if (f(t, 14 * b, 14) >= (int)V.size()) return -9;
-          x[t] = V[f(t, 98, 14)];
-          for (int c = 0; c < kSlOpRun; ++c)
-            x[t] += V[f(t, 42 * c, 14)] * V[f(t, 42 * c + 14, 14)] * V[f(t, 42 * c + 28, 14)];
+          const int ini = zero + f(t, kSlOpIni.bit, kSlOpIni.width);
+          if (ini >= (int)V.size() || f(t, kSlOpT.bit, kSlOpT.width) >= (int)V.size()) return -9;
+          x[t] = V[ini];
+          for (int c = 0; c < kSlOpRun; ++c) {
+            const int a = f(t, kSlOpA[c].bit, kSlOpA[c].width),
+                      b = f(t, kSlOpB[c].bit, kSlOpB[c].width),
+                      k = f(t, kSlOpK[c].bit, kSlOpK[c].width);
+            // (D is set when a pivot is taken)
+            if (a >= (int)V.size() || b >= (int)V.size() || k >= N || D[k] == 0.0) return -9;
+            x[t] += V[a] * V[b] * V[k];
+          }
           if (f(t, 118, 10) != f(0, 118, 10)) return -10;
         }
         scan(x, [&](int t) { return f(t, 112, 5); }, [&](int t) { return f(t, 117, 1) != 0; },
              f(0, 118, 3));
         for (int t = 0; t < 32; ++t) {
-          const int to = f(t, 84, 14);
+          const int to = f(t, kSlOpT.bit, kSlOpT.width);
           if (to < zero)
             V[to] -= x[t];
           else if (to > zero)

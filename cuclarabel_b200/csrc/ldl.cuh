@@ -15,10 +15,6 @@ struct SnExec;
 
 // blocks per SM the register budgets of the class-1 kernels aim at
 constexpr int kSlSolveBlocks = 5;
-// stages (op pages of a warp) copied ahead of use
-constexpr int kSlRing = 3;
-constexpr int kSlOpRing = 4;
-constexpr int kSlSmemMax = 224 * 1024;  // dynamic shared memory of a block
 constexpr int kSlFactorBlocks = 6;
 
 // One class-1 instance: sizes, and where its part of each array begins.

@@ -604,15 +604,15 @@ __global__ void __launch_bounds__(kNT, kSlFactorBlocks)
   meet(oskip);
 #pragma unroll 1
   for (int p = 0; p < nop; ++p) {
-    constexpr unsigned m = 0x3fffu;
-    const unsigned t = __funnelshift_r(o.z, o.w, 20) & m;
+    constexpr unsigned m = 0x7fffu, mk = 0x1fffu;  // positions, diagonal positions
+    const unsigned t = __funnelshift_r(o.z, o.w, 22) & m;
     // each target is written once per level end, so its old value is read
     // before the sum, off the dependent chain
     const A old = V[t];
-    A x = sl_mul(sl_mul(V[o.x & m], V[(o.x >> 14) & m]), V[__funnelshift_r(o.x, o.y, 28) & m]);
-    x = sl_add(x, V[(o.w >> 2) & m]);  // the carry, or zero
-    const A x1 = sl_mul(sl_mul(V[(o.y >> 10) & m], V[__funnelshift_r(o.y, o.z, 24) & m]),
-                        V[(o.z >> 6) & m]);
+    A x = sl_mul(sl_mul(V[o.x & m], V[(o.x >> 15) & m]), V[__funnelshift_r(o.x, o.y, 30) & mk]);
+    x = sl_add(x, V[zero + ((o.w >> 5) & 0x7ffu)]);  // the carry, or zero
+    const A x1 = sl_mul(sl_mul(V[(o.y >> 11) & m], V[__funnelshift_r(o.y, o.z, 26) & m]),
+                        V[(o.z >> 9) & mk]);
     x = sl_add(x, x1);
     const int reach = (int)((o.w >> 16) & 31u), steps = (int)((o.w >> 22) & 7u);
 #pragma unroll 1

@@ -284,14 +284,14 @@ bool sl_build(const Prepared &p, int vgroup, SlicedPlan &s) {
   // one lane of an op page (the fields of sliced.hpp)
   auto encode = [](uint32_t *w, const Op &o0, const Op &o1, uint32_t t, uint32_t ini,
                    uint32_t meta) {
-    w[0] = o0.a | ((uint32_t)o0.b << 14) | ((uint32_t)o0.k << 28);
-    w[1] = ((uint32_t)o0.k >> 4) | ((uint32_t)o1.a << 10) | ((uint32_t)o1.b << 24);
-    w[2] = ((uint32_t)o1.b >> 8) | ((uint32_t)o1.k << 6) | (t << 20);
-    w[3] = (t >> 12) | (ini << 2) | (meta << 16);
+    w[0] = o0.a | ((uint32_t)o0.b << 15) | ((uint32_t)o0.k << 30);
+    w[1] = ((uint32_t)o0.k >> 2) | ((uint32_t)o1.a << 11) | ((uint32_t)o1.b << 26);
+    w[2] = ((uint32_t)o1.b >> 6) | ((uint32_t)o1.k << 9) | (t << 22);
+    w[3] = (t >> 10) | (ini << 5) | (meta << 16);
   };
-  const Op none{(uint16_t)zero, (uint16_t)zero, (uint16_t)zero};
+  auto none = [&](uint16_t k) { return Op{(uint16_t)zero, (uint16_t)zero, k}; };
   uint32_t padw[4];
-  encode(padw, none, none, (uint32_t)zero, (uint32_t)zero, 0u);
+  encode(padw, none(0), none(0), (uint32_t)zero, 0u, 0u);
   thread_local std::vector<int> page_reach;
   for (int l = 0; l < nlev; ++l) {
     const int qa = p.lvl_ptr[l], qb = p.lvl_ptr[l + 1];
@@ -372,7 +372,7 @@ bool sl_build(const Prepared &p, int vgroup, SlicedPlan &s) {
       at0 += (segs[sb[w + 1]] - s0 + chunk - 1) / chunk * chunk;
     }
     s.nopcarry = std::max(s.nopcarry, split.ncarry);
-    if (zero + 1 + s.nopcarry > kSlOpPositions) return false;
+    if (zero + s.nopcarry >= 1 << kSlOpT.width || s.nopcarry >= 1 << kSlOpIni.width) return false;
     auto part_of = [&](int g) {
       int w = 0;
       while (g >= sb[w + 1]) ++w;
@@ -405,13 +405,13 @@ bool sl_build(const Prepared &p, int vgroup, SlicedPlan &s) {
         for (int r = 0; r < q.lanes; ++r) {
           const Op &o0 = lev[t + off];
           const bool two = t % kSlOpRun == 0 && t + 1 < end;
-          const Op &o1 = two ? lev[t + 1 + off] : none;
+          const Op o1 = two ? lev[t + 1 + off] : none(o0.k);
           t += two ? 2 : 1;
           const bool last = r == q.lanes - 1;
           const bool prev = last && !q.scan_last && r > 0;
           if (!prev) page_reach[pgi] = std::max(page_reach[pgi], r);
           const int to = !last ? zero : (q.more ? zero + 1 + q.carry_out : target[q.seg]);
-          const int ini = r == 0 && q.carry_in >= 0 ? zero + 1 + q.carry_in : zero;
+          const int ini = r == 0 && q.carry_in >= 0 ? 1 + q.carry_in : 0;
           encode(e + 4 * (l0 + r), o0, o1, (uint32_t)to, (uint32_t)ini,
                  prev ? 32u : (uint32_t)r);
         }
@@ -441,7 +441,17 @@ bool sl_build(const Prepared &p, int vgroup, SlicedPlan &s) {
     s.op.skip[w] = oskip[w];
     s.ops.insert(s.ops.end(), opg[w].begin(), opg[w].end());
   }
-  return true;
+  const SlNeed need = sl_need(s);
+  return std::max({need.solve[0], need.solve[1], need.factor[0]}) <= kSlSmemMax;
+}
+
+SlNeed sl_need(const SlicedPlan &p) {
+  const long long ring = (long long)kSlRing * kSlStage * (8 * kSlRun + 16) +
+                         (((long long)p.used.size() + 15) & ~15LL);
+  const long long slots = 2LL * p.N + 1 + p.ncarry;
+  const long long tab = (long long)kSlWarps * kSlOpRing * 512 + ((p.N + 15) & ~15LL);
+  const long long V = (long long)p.N + p.nl + 1 + p.nopcarry;
+  return {{ring + 8 * slots, ring + 16 * slots}, {tab + 8 * V, tab + 4 * V}};
 }
 
 }  // namespace clgpu

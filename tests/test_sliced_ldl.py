@@ -83,6 +83,42 @@ def test_two_sides_in_one_launch_are_each_its_own_solve(cuda_device, method):
         assert np.array_equal(a.x, b.x) and np.array_equal(a.s, b.s) and np.array_equal(a.z, b.z)
 
 
+# factors of more than 2^14 positions, up to what a block's shared memory takes
+# (28 k), and one above it
+LARGE = {"psd_10x4": lambda: problems.psd_lp(10, 4, seed=2),
+         "psd_12x3": lambda: problems.psd_lp(12, 3, seed=2),
+         "mpc_1200": lambda: problems.mpc_qp(5, n=1200),
+         "mpc_2000": lambda: problems.mpc_qp(5, n=2000),
+         "psd_12x4": lambda: problems.psd_lp(12, 4, seed=2)}
+
+
+@pytest.mark.parametrize("name,want", [("psd_10x4", 0), ("psd_12x3", 0), ("mpc_1200", -4),
+                                       ("mpc_2000", -4), ("psd_12x4", -3)])
+def test_large_layouts_replay_on_the_host(name, want):
+    """-4: takes these kernels, too large for the dense comparison; -3: does not
+    take them."""
+    cp, keep, n, m = _prep_problem(*LARGE[name]())
+    st = Settings().to_c()
+    r = ctypes.c_double()
+    rc = _lib.load().clgpu_debug_factor_stream(ctypes.byref(cp), ctypes.byref(st),
+                                               ctypes.byref(r))
+    assert rc == want and (rc or r.value < 1e-12), (rc, r.value)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", LARGE)
+def test_large_solves_match_the_oracle(cuda_device, name):
+    import oracle
+    pb = LARGE[name]()
+    sol = Solver(*pb).solve()
+    ref = oracle.solve(*pb)
+    assert sol.status.name in ("SOLVED", "ALMOST_SOLVED") and ref["status_name"] == "SOLVED"
+    assert rel_err(sol.obj_val, ref["obj_val"]) < OBJ_RTOL
+    two = BatchSolver([pb] * 2, max_iter=6, fused_solves=False).solve()
+    one = BatchSolver([pb], max_iter=6).solve()[0]
+    assert all(np.array_equal(one.x, t.x) and np.array_equal(one.z, t.z) for t in two)
+
+
 def _entries(pb):
     cp, keep, n, m = _prep_problem(*pb)
     st = Settings().to_c()
