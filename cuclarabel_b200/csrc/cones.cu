@@ -2836,14 +2836,31 @@ static inline void psd_launch_dims(const ConeSet &cs, int nmats, int &nb, int &n
   KERNEL<<<blocks_for(16LL * cs.n_psd, 32 * kPsdWarps), 32 * kPsdWarps,                \
            2 * kPsdWarps * kPsdSmallWords * sizeof(double), st>>>(__VA_ARGS__)
 
-// sides up to kPsdPairSide take the pair-per-lane scaling and the
-// thread-per-matrix step length: at 16 their matrices still leave three blocks
-// per SM and a row fits in registers; above, the group kernels' 32 lanes are
-// filled by one column (side 8, 96 cones: scaling 231 us by groups, 85 by
-// pairs, step 217 against 45; side 10, 40 000 cones: 3866 against 601 and 2892
-// against 240)
+// sides up to kPsdPairSide take the pair-per-lane scaling: at 16 its matrices
+// still leave three blocks per SM and a row fits in registers; above, the group
+// kernels' 32 lanes are filled by one column (groups against pairs, us: side 1,
+// 1000 cones 11 / 9; side 8, 100 cones 265 / 101; side 10, 40 000 cones 3866 /
+// 601; side 16, 20 000 cones 15 100 / 1530)
 static inline bool psd_small(const ConeSet &cs) {
   return cs.n_psd > 0 && cs.psd_nmax <= kPsdPairSide;
+}
+// The thread-per-matrix step length needs a matrix to reduce: on sides 1 and 2 the
+// group kernel's eigenvalues are found as soon as they are loaded (1000 cones,
+// groups against threads, us: side 1 13 / 19, side 2 18 / 20, side 3 34 / 25; whole
+// calls with 200 000 cones: 275 / 420, 391 / 433, 987 / 479; with 20 000 of side
+// 16: 9990 / 360).
+static inline bool psd_small_step(const ConeSet &cs) {
+  return psd_small(cs) && cs.psd_nmax > 2;
+}
+// The products from registers pass through 16 columns whatever the side, so they
+// win from side 9 on (H x and combined shift, an element per lane against a column
+// per lane, us: side 9, 200 000 cones 475 / 441 and 827 / 801; side 10, 40 000
+// cones 154 / 104 and 260 / 189), lose below 7 (side 4, 10 000 cones: 11 / 25 and
+// 15 / 36; 1000 cones 9 / 12 and 11 / 15), and between them win while the cones
+// are about one wave (side 8: 1000 cones 13 / 13 and 19 / 17, 4000 cones 17 / 15 and
+// 23 / 27, 10 000 cones 28 / 30 and 38 / 42).
+static inline bool psd_small_products(const ConeSet &cs) {
+  return psd_small(cs) && (cs.psd_nmax > 8 || (cs.psd_nmax > 6 && cs.n_psd <= 2000));
 }
 static NonsymArgs<ExpOps> exp_args(const ConeSet &cs) {
   return NonsymArgs<ExpOps>{cs.n_exp, cs.exp_begin, cs.exp_inst, nullptr,
@@ -2916,7 +2933,7 @@ void cones_mul_Hs(const ConeSet &cs, double *y, const double *x, cudaStream_t st
   if (cs.n_pow)
     k_nonsym_mul_hs<<<blocks_for(cs.n_pow), kBlock, 0, st>>>(cs, cs.n_pow, cs.pow_begin,
                                                             cs.pow_inst, cs.pow_Hs, y, x);
-  if (psd_small(cs))
+  if (psd_small_products(cs))
     LAUNCH_PSD_SMALL(k_psd_mul_hs_small, cs, y, x);
   else
     LAUNCH_PSD(k_psd_mul_hs, 3, cs, y, x);
@@ -2947,7 +2964,7 @@ void cones_combined_ds_shift(const ConeSet &cs, double *shift, const double *dz,
   if (cs.n_pow)
     k_nonsym_combined<PowOps><<<blocks_for(cs.n_pow, 128), 128, 0, st>>>(
         cs, pow_args(cs), shift, dz, ds, sm);
-  if (psd_small(cs))
+  if (psd_small_products(cs))
     LAUNCH_PSD_SMALL(k_psd_combined_small, cs, shift, dz, ds, sm);
   else
     LAUNCH_PSD(k_psd_combined, 5, cs, shift, dz, ds, sm);
@@ -2964,7 +2981,7 @@ void cones_ds_from_dz_offset(const ConeSet &cs, double *out, const double *ds,
   if (cs.n_pow)
     k_nonsym_copy<<<blocks_for(3 * cs.n_pow), kBlock, 0, st>>>(cs, cs.n_pow, cs.pow_begin,
                                                               cs.pow_inst, out, ds);
-  if (psd_small(cs))
+  if (psd_small_products(cs))
     LAUNCH_PSD_SMALL(k_psd_ds_offset_small, cs, out, ds);
   else
     LAUNCH_PSD(k_psd_ds_offset, 4, cs, out, ds);
@@ -2977,7 +2994,7 @@ void cones_step_length_sym(const ConeSet &cs, const double *dz, const double *ds
     k_nn_step<<<blocks_for(cs.n_nn, nn_block(cs) * (cs.B == 1 ? kNNRows : 1)), nn_block(cs), 0,
                 st>>>(cs, dz, ds, z, s, alpha);
   LAUNCH_SOC_SHAPED(kSocStep, k_soc_tile_step, 4, k_soc_step, dz, ds, z, s, alpha);
-  if (psd_small(cs)) {
+  if (psd_small_step(cs)) {
     LAUNCH_PSD_SMALL(k_psd_step_matrices, cs, dz, ds);
     const size_t sm = (size_t)(kPsdEigThreads + 1) * (cs.psd_nmax * (cs.psd_nmax + 1) / 2 +
                                                 2 * cs.psd_nmax) * sizeof(double);

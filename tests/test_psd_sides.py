@@ -65,6 +65,17 @@ def test_psd_sides(cuda_device, name):
         assert abs(a.value - ref) <= 1e-10 * max(1.0, ref), (a.value, ref)
 
 
+# both sides of the lines between the products' and the step lengths' kernels
+LINES = {"two_many": [2, 1] * 40, "six": [6, 4] * 9, "seven": [7] * 33, "eight_2000": [8] * 2000,
+         "eight_2001": [8, 3, 5] * 667, "nine": [9, 2] * 17}
+
+
+@pytest.mark.parametrize("name", list(LINES))
+def test_psd_sides_at_the_lines(cuda_device, name):
+    SIDES[name] = LINES[name]
+    test_psd_sides(cuda_device, name)
+
+
 @pytest.mark.parametrize("n", [1, 8, 16])
 def test_psd_repeated_eigenvalues(cuda_device, n):
     """s = z = I: the scaling is the identity and every eigenvalue of the step's
