@@ -1611,7 +1611,10 @@ static int build_batch(clgpu_solver *h, std::vector<Prepared> &prep, int nth) {
       cecol[i] = (long long)sp.ecol.size();
     }
     const auto opage = prefix(cpage), olane = prefix(clane), ovp = prefix(cvp), oop = prefix(cop), oecol = prefix(cecol);
-    if (olane[B] * 4 > 2000000000LL || oop[B] * kSlOpWords > 2000000000LL) return -4;
+    // (an instance's parts begin at int offsets, counted in lanes and pages)
+    if (olane[B] > 2000000000LL || ovp[B] > 2000000000LL || oop[B] > 2000000000LL ||
+        opage[B] > 2000000000LL || oecol[B] > 2000000000LL)
+      return -4;
     std::vector<SlInst> sl(B);
     std::vector<SlNeed> need(B);
     hvec<uint16_t> kdst((size_t)knz), lpos(ovp[B] * kSlRun), leaf(VT), ecols(oecol[B]);
