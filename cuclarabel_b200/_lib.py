@@ -86,7 +86,7 @@ EXPORTED = [
     "clgpu_ds_from_dz_offset", "clgpu_step_length", "clgpu_compute_barrier",
     "clgpu_margins", "clgpu_scaled_unit_shift", "clgpu_unit_initialization",
     "clgpu_debug_check_instance", "clgpu_debug_instance_path", "clgpu_debug_pinned_stats",
-    "clgpu_debug_factor_stream", "clgpu_debug_launch_groups",
+    "clgpu_debug_factor_stream", "clgpu_debug_launch_groups", "clgpu_debug_ldl_plan",
     "clgpu_margins_static",
     "clgpu_cones_set_profiling", "clgpu_cones_last_kernel_ms",
     "clgpu_cones_get_launch_shapes", "clgpu_cones_set_launch_shapes",
@@ -159,6 +159,7 @@ def _declare(L):
     L.clgpu_debug_factor_stream.argtypes = [ctypes.POINTER(ClgpuProblem),
                                             ctypes.POINTER(ClgpuSettings), dp]
     # KKT-level boundary (device pointers as integers)
+    L.clgpu_debug_ldl_plan.argtypes = [c_int, ip, ip, ctypes.POINTER(ctypes.c_longlong)]
     L.clgpu_debug_launch_groups.argtypes = [ctypes.POINTER(ClgpuProblem), c_int,
                                             ctypes.POINTER(ClgpuSettings), ip]
     L.clgpu_mul_Hs_diag.argtypes = [c_void_p, V, V, c_void_p]

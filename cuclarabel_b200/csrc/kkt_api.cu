@@ -161,6 +161,51 @@ extern "C" int clgpu_ldl_create(int N, const int *Kp, const int *Kj, const signe
   return 0;
 }
 
+// Shape of the plan for a symmetric pattern (host only): shape[0] the widest
+// update (columns), [1] the largest distance of a front's tile from a panel that
+// takes it in the backward substitution (tiles), [2] the updates wider than a
+// panel, [3] the helper tasks of the backward substitution.
+extern "C" int clgpu_debug_ldl_plan(int N, const int *Kp, const int *Kj, long long *shape) {
+  if (N <= 0 || !Kp || !Kj || !shape) return -1;
+  std::vector<int> xadj(N + 1, 0), adj;
+  std::vector<int> P(N + 1, 0), J, perm;
+  for (int r = 0; r < N; ++r) {
+    for (int q = Kp[r]; q < Kp[r + 1]; ++q)
+      if (Kj[q] != r) adj.push_back(Kj[q]);
+    xadj[r + 1] = (int)adj.size();
+  }
+  SnSymbolic sym;
+  std::string err;
+  if (!sn_analyse(N, xadj, adj, perm, sym, &err)) return -3;
+  std::vector<int> ip(N);
+  for (int k = 0; k < N; ++k) ip[perm[k]] = k;
+  for (int k = 0; k < N; ++k) {
+    const int r = perm[k], j0 = (int)J.size();
+    for (int q = Kp[r]; q < Kp[r + 1]; ++q) J.push_back(ip[Kj[q]]);
+    std::sort(J.begin() + j0, J.end());
+    P[k + 1] = (int)J.size();
+  }
+  std::vector<SnInstance> in{{&sym, P.data(), J.data(), 0, 0, 0}};
+  SnPlan plan;
+  if (!sn_build_plan(in, plan, &err)) return -3;
+  std::fill(shape, shape + 4, 0LL);
+  for (const SnLaunch &L : plan.fact)
+    for (int q = L.begin; L.kind == SN_UPDATE && q < L.begin + L.count; ++q) {
+      const long long K = plan.tasks[q].y >> 16;
+      shape[0] = std::max(shape[0], K);
+      shape[2] += K > kSnNB;
+    }
+  for (const SnLaunch &L : plan.bwd)
+    for (int q = L.begin; L.kind == SN_BWD_DIAG && q < L.begin + L.count; ++q) {
+      const SnQuad t = plan.tasks[q];
+      const int np = (plan.u0[t.x] + kSnNB - 1) / kSnNB;
+      const int nt = np + (plan.ld[t.x] - plan.u0[t.x]) / kSnNB;
+      shape[1] = std::max(shape[1], (long long)(nt - 1 - t.y));
+      shape[3] += t.w != 0;
+    }
+  return 0;
+}
+
 extern "C" int clgpu_ldl_destroy(clgpu_ldl *h) {
   if (!h) return -1;
   delete h;

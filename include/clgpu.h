@@ -479,6 +479,13 @@ int clgpu_debug_factor_stream(const clgpu_problem *prob, const clgpu_settings *s
  * a launch would not fit its members.  Needs no GPU. */
 int clgpu_debug_launch_groups(const clgpu_problem *probs, int n, const clgpu_settings *settings,
                               int *counts);
+/* Host-only view of the supernodal plan of a symmetric pattern (CSR, both
+ * triangles and the diagonal; diagnostic, no reference counterpart): shape[0]
+ * the widest trailing update in columns, shape[1] the largest distance of a tile
+ * from the panel that takes it in a backward substitution, in tiles of 128,
+ * shape[2] the updates wider than one panel, shape[3] the helper tasks of the
+ * backward substitution.  Needs no GPU. */
+int clgpu_debug_ldl_plan(int N, const int *Kp, const int *Kj, long long *shape);
 /* Counters of the process-wide page-locked host pool that setup arrays,
  * upload staging and result staging come from (diagnostic, no reference
  * counterpart): out[0] buffers served from the pool, out[1] page-locked
