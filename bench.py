@@ -1090,7 +1090,8 @@ def main():
                              "constant and affine right-hand sides + refinement)",
                "ldl_factor": "k_sl_factor<double, double> (block-per-instance LDL "
                              "factorisation)"}
-    summaries = {}  # profiles/ summaries of these kernels' DRAM traffic
+    summaries = {"ldl_solve": "sl_solve_mpc4096.md", "ldl_solve2": "sl_solve2_mpc4096.md",
+                 "ldl_factor": "sl_factor_mpc4096.md"}
 
     def roofline(name):
         ms, calls = phases[name]
@@ -1099,8 +1100,8 @@ def main():
         return {"bound": "hbm", "kernel": kernels.get(name, name), "achieved": ach,
                 "peak": hbm, "unit": "GB/s", "frac": ach / hbm,
                 "traffic": ncu_traffic(summaries[name]) if name in summaries else None,
-                "traffic_source": ("profiles/" + summaries[name] + " (one captured launch; "
-                                   "dram__bytes_read.sum + dram__bytes_write.sum)")
+                "traffic_source": ("profiles/" + summaries[name] + " (mean of one solve's "
+                                   "launches; dram__bytes_read.sum + dram__bytes_write.sum)")
                 if name in summaries else None,
                 "peak_kind": peak_note,
                 "algorithmic_bytes_per_launch": by / max(calls, 1),
