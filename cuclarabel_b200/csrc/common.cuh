@@ -34,6 +34,14 @@ __device__ __forceinline__ double logsafe(double v) {
   return v < 0 ? -kDMax : log(v);
 }
 
+// PSD sides up to here have kernels of their own (cones.cu), by the cone's side
+// alone: a cone's results do not depend on what else is in the set.  Classes: up
+// to 2, up to this, above.
+constexpr int kPsdSmallSide = 16;
+__host__ __device__ __forceinline__ int psd_class(int n) {
+  return n <= 2 ? 0 : (n <= kPsdSmallSide ? 1 : 2);
+}
+
 // Device-side description of all cones of a batch.
 struct ConeSet {
   int B;            // instances
@@ -67,7 +75,10 @@ struct ConeSet {
   // PSD triangle cones
   int n_psd, psd_begin;
   const int *psd_off, *psd_n, *psd_inst;
-  int psd_nmax;
+  int psd_nmax, psd_smax;  // largest side, and of classes 0 and 1
+  int psd_count[3];        // cones per class
+  int psd_take = 7;        // bit c: a launch works on the cones of class c
+  int psd_lanes = 0;       // lanes per cone in a launch, 0: by the largest side
   // state
   double *nn_w, *nn_lambda;           // [n_nn]
   double *soc_w, *soc_lambda;         // [soc_rows] (indexed g - soc_begin)
@@ -76,7 +87,7 @@ struct ConeSet {
   double *exp_Hd, *exp_Hs, *exp_grad, *exp_z;  // 9,9,3,3 per cone
   double *pow_Hd, *pow_Hs, *pow_grad, *pow_z;
   double *psd_R, *psd_Rinv, *psd_lam;  // nmax^2, nmax^2, nmax per cone
-  double *psd_eig;  // step length scratch, nmax (nmax + 1) per cone
+  double *psd_eig;  // step length scratch, smax (smax + 1) per cone
   // per-instance flags
   const int *inst_active;  // [B] nonzero -> instance takes part
   const int *inst_sym;     // [B] 1 if every cone of the instance is symmetric

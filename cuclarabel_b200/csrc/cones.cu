@@ -821,7 +821,10 @@ __device__ double warp_eig_min(int n, double *A, double *ev, const PsdGrp &g) {
 
 __device__ __forceinline__ PsdCtx psd_ctx(const ConeSet &cs) {
   PsdCtx p;
-  const int G = psd_group(cs.psd_nmax);
+  // (read from the set also where it is always 16: with a constant here the step's
+  // matrices took 268 us instead of 238, the combined shift 220 instead of 175, 40
+  // 000 cones of side 10)
+  const int G = cs.psd_lanes ? cs.psd_lanes : psd_group(cs.psd_nmax);
   int w = (blockIdx.x * blockDim.x + threadIdx.x) / G;
   p.lane = threadIdx.x % G;
   p.g.lane = p.lane;
@@ -833,7 +836,8 @@ __device__ __forceinline__ PsdCtx psd_ctx(const ConeSet &cs) {
   p.t = p.n * (p.n + 1) / 2;
   p.off = cs.psd_off[p.c];
   p.inst = cs.psd_inst[p.c];
-  if (p.valid && !active_inst(cs, p.inst)) p.valid = false;
+  if (p.valid && !(active_inst(cs, p.inst) && ((cs.psd_take >> psd_class(p.n)) & 1)))
+    p.valid = false;
   p.g.warp = __ballot_sync(0xffffffffu, p.valid);
   return p;
 }
@@ -891,22 +895,22 @@ __global__ void k_psd_update_scaling(ConeSet cs, const double *__restrict__ s,
 // division and square roots on all lanes: 79 k warp instructions per 10 x 10
 // cone, 3.87 ms for 40 000; now 0.60 ms.)  Matrices are interleaved over
 // the warp's cones, so lanes of one step read neighbouring words.
-constexpr int kPsdPairSide = 16, kPsdPairWarps = 2;
+constexpr int kPsdPairSide = kPsdSmallSide, kPsdPairWarps = 2;
 __global__ void __launch_bounds__(32 * kPsdPairWarps)
     k_psd_update_pairs(ConeSet cs, const double *__restrict__ s, const double *__restrict__ z,
                        int *scale_ok) {
   extern __shared__ double sm_psd[];
-  const int nm = cs.psd_nmax, nn = nm * nm, nb = nm * (nm + 1 + (nm & 1));
+  const int nm = cs.psd_nmax, nn = nm * nm, ns = cs.psd_smax, nb = ns * (ns + 1 + (ns & 1));
   const int lane = threadIdx.x & 31, c8 = lane & 7, q4 = lane >> 3;
-  double *M = sm_psd + (size_t)(threadIdx.x >> 5) * 8 * (2 * nb + 2 * nm) + c8;
+  double *M = sm_psd + (size_t)(threadIdx.x >> 5) * 8 * (2 * nb + 2 * ns) + c8;
   double *V = M + 8 * nb, *S = V + 8 * nb;
-  int *perm = reinterpret_cast<int *>(S - c8 + 8 * nm) + c8;
+  int *perm = reinterpret_cast<int *>(S - c8 + 8 * ns) + c8;
   const int c = (blockIdx.x * kPsdPairWarps + (threadIdx.x >> 5)) * 8 + c8;
   int n = 0, off = 0, inst = -1;
   if (c < cs.n_psd) {
     inst = cs.psd_inst[c];
     off = cs.psd_off[c];
-    if (active_inst(cs, inst)) n = cs.psd_n[c];
+    if (active_inst(cs, inst) && cs.psd_n[c] <= kPsdPairSide) n = cs.psd_n[c];
   }
   // odd, so that the four lanes of a cone meet different banks, and with room
   // for the row of zeros
@@ -1459,7 +1463,9 @@ __global__ void k_psd_combined(ConeSet cs, double *shift, const double *__restri
   for (int e = p.lane; e < n * n; e += p.g.G) {
     int i = e % n, j = e / n;
     double t = 0;
-    for (int k = 0; k < n; ++k) t += S[i + n * k] * Z[k + n * j] + Z[i + n * k] * S[k + n * j];
+    for (int k = 0; k < n; ++k)  // (spelled as in k_psd_combined_small)
+      t = __dadd_rn(t, __fma_rn(S[i + n * k], Z[k + n * j],
+                                __dmul_rn(Z[i + n * k], S[k + n * j])));
     X[e] = 0.5 * t;
   }
   p.g.sync();
@@ -1668,7 +1674,7 @@ constexpr int kPsdEigThreads = 32;
 __global__ void __launch_bounds__(kPsdEigThreads) k_psd_step_eig(ConeSet cs, double *alpha) {
   extern __shared__ double sm_psd[];
   constexpr int W = kPsdEigThreads + 1;  // odd: the copy in below is free of conflicts
-  const int nm = cs.psd_nmax, tm = nm * (nm + 1) / 2, tid = threadIdx.x;
+  const int nm = cs.psd_smax, tm = nm * (nm + 1) / 2, tid = threadIdx.x;
   double *A = sm_psd + tid, *d = A + W * tm, *e = d + W * nm;  // element k at [W k]
   const int first = blockIdx.x * kPsdEigThreads, m = min(kPsdEigThreads, 2 * cs.n_psd - first);
   const double *src = cs.psd_eig + (size_t)first * tm;
@@ -1678,7 +1684,7 @@ __global__ void __launch_bounds__(kPsdEigThreads) k_psd_step_eig(ConeSet cs, dou
   const int c = (first + tid) >> 1, inst = cs.psd_inst[c];
   if (!active_inst(cs, inst)) return;
   const int n = cs.psd_n[c];
-  if (n == 0) return;  // no eigenvalue
+  if (!((cs.psd_take >> psd_class(n)) & 1)) return;
   // The largest entry.  Away from the middle of FP64's range the matrix is scaled
   // by a power of two, so that no square below overflows and a row whose squares
   // underflow is negligible beside it.  An infinite entry: the smallest diagonal
@@ -1890,16 +1896,22 @@ __device__ __forceinline__ void psd_symmetric(const PsdSmall &q, int n, const Ps
       y[j] = ((y[j] + q.Y[j + q.ld * q.lane]) * is2) * is2;
   g.sync();
 }
-// svec of the matrix whose symmetric part's row `lane` is y; minus sub on the
-// diagonal
-__device__ __forceinline__ void psd_store(const PsdSmall &q, int n,
+// svec of the symmetric part of the matrix whose row `lane` is y, minus sub on the
+// diagonal; Y is written.  (As mat_to_svec forms it: the products of the group
+// kernels are the same bits, so either kernel may take a cone.)
+__device__ __forceinline__ void psd_store(const PsdSmall &q, int n, const PsdGrp &g,
                                           const double (&y)[kPsdPairSide], double sub,
                                           double *out) {
-  const double sqrt2 = 1.4142135623730951;
+  const double is2 = 0.70710678118654752440;
+#pragma unroll
+  for (int j = 0; j < kPsdPairSide; ++j)
+    if (j < n && q.lane < n) q.Y[q.lane + q.ld * j] = y[j];
+  g.sync();
 #pragma unroll
   for (int j = 0; j < kPsdPairSide; ++j)
     if (j < n && q.lane <= j)
-      out[j * (j + 1) / 2 + q.lane] = q.lane == j ? y[j] - sub : y[j] * sqrt2;
+      out[j * (j + 1) / 2 + q.lane] =
+          q.lane == j ? y[j] - sub : (y[j] + q.Y[j + q.ld * q.lane]) * is2;
 }
 __global__ void k_psd_mul_hs_small(ConeSet cs, double *y, const double *__restrict__ x) {
   PsdCtx p = psd_ctx(cs);
@@ -1917,8 +1929,7 @@ __global__ void k_psd_mul_hs_small(ConeSet cs, double *y, const double *__restri
     if (j < n && q.lane <= j) q.X[j * (j + 1) / 2 + q.lane] = v[j];
   p.g.sync();
   psd_congr<true>(q, n, v);  // W^T W x
-  psd_symmetric(q, n, p.g, v);
-  psd_store(q, n, v, 0.0, y + p.off);
+  psd_store(q, n, p.g, v, 0.0, y + p.off);
 }
 __global__ void k_psd_combined_small(ConeSet cs, double *shift, const double *__restrict__ dz,
                                      const double *__restrict__ ds, const double *sm) {
@@ -1953,32 +1964,40 @@ __global__ void k_psd_combined_small(ConeSet cs, double *shift, const double *__
       double t = 0;
 #pragma unroll
       for (int k = 0; k < kPsdPairSide; ++k)
-        if (k < n) t += b[k] * q.R[k + q.ld * j] + a[k] * q.Y[k + q.ld * j];
+        if (k < n)
+          t = __dadd_rn(t, __fma_rn(b[k], q.R[k + q.ld * j],
+                                    __dmul_rn(a[k], q.Y[k + q.ld * j])));
       c[j] = 0.5 * t;
     }
   }
   p.g.sync();
-  psd_symmetric(q, n, p.g, c);
-  psd_store(q, n, c, sm[p.inst], shift + p.off);
+  psd_store(q, n, p.g, c, sm[p.inst], shift + p.off);
 }
 __global__ void k_psd_ds_offset_small(ConeSet cs, double *out, const double *__restrict__ ds) {
   PsdCtx p = psd_ctx(cs);
   if (!p.valid) return;
   const PsdSmall q = psd_small_ctx(p);
+  const double is2 = 0.70710678118654752440;
   const int n = p.n;
   const double l = p.lane < n ? cs.psd_lam[(size_t)p.c * cs.psd_nmax + p.lane] : 1.0;
+  const double *x = ds + p.off;
   double v[kPsdPairSide];
+#pragma unroll
+  for (int j = 0; j < kPsdPairSide; ++j)
+    v[j] = j < n && q.lane <= j ? x[j * (j + 1) / 2 + q.lane] : 0.0;
   psd_load_R(q, n, cs.psd_R + (size_t)p.c * cs.psd_nmax * cs.psd_nmax);
-  psd_load_X(q, n, ds + p.off);
 #pragma unroll
   for (int j = 0; j < kPsdPairSide; ++j) {
     const double lj = __shfl_sync(p.g.mask, l, j, 16);
-    if (j < n && q.lane <= j) q.X[j * (j + 1) / 2 + q.lane] *= 2 / (l + lj);
+    if (j < n && q.lane <= j) {
+      const double w = 2 * (q.lane == j ? v[j] : v[j] * is2) / (l + lj);
+      // (as svec and back, as the reference keeps it)
+      q.X[j * (j + 1) / 2 + q.lane] = q.lane == j ? w : ((w + w) * is2) * is2;
+    }
   }
   p.g.sync();
   psd_congr<true>(q, n, v);  // R X R'
-  psd_symmetric(q, n, p.g, v);
-  psd_store(q, n, v, 0.0, out + p.off);
+  psd_store(q, n, p.g, v, 0.0, out + p.off);
 }
 __global__ void k_psd_step_matrices(ConeSet cs, const double *__restrict__ dz,
                                     const double *__restrict__ ds) {
@@ -1998,7 +2017,7 @@ __global__ void k_psd_step_matrices(ConeSet cs, const double *__restrict__ dz,
     else
       psd_congr<true>(q, n, v);  // W^{-T} ds
     psd_symmetric(q, n, p.g, v);
-    double *out = cs.psd_eig + (size_t)(2 * p.c + side) * (nm * (nm + 1) / 2);
+    double *out = cs.psd_eig + (size_t)(2 * p.c + side) * (cs.psd_smax * (cs.psd_smax + 1) / 2);
 #pragma unroll
     for (int j = 0; j < kPsdPairSide; ++j) {
       const double lj = __shfl_sync(p.g.mask, li, j, 16);
@@ -2817,6 +2836,18 @@ static inline void psd_launch_dims(const ConeSet &cs, int nmats, int &nb, int &n
   nb = blocks_for((long long)cs.n_psd * G, nt);
   smem = (size_t)groups * per + 256;
 }
+// cones of the classes of `take`
+static inline int psd_cones(const ConeSet &cs, int take) {
+  int n = 0;
+  for (int c = 0; c < 3; ++c) n += (take >> c) & 1 ? cs.psd_count[c] : 0;
+  return cs.n_psd > 0 ? n : 0;  // (the counts outlive a set cut down to other types)
+}
+static inline ConeSet psd_taking(const ConeSet &cs, int take, int lanes = 0) {
+  ConeSet c = cs;
+  c.psd_take = take;
+  c.psd_lanes = lanes;
+  return c;
+}
 #define LAUNCH_PSD(KERNEL, NMATS, ...)                                                 \
   do {                                                                                 \
     if (cs.n_psd > 0) {                                                                \
@@ -2836,32 +2867,43 @@ static inline void psd_launch_dims(const ConeSet &cs, int nmats, int &nb, int &n
   KERNEL<<<blocks_for(16LL * cs.n_psd, 32 * kPsdWarps), 32 * kPsdWarps,                \
            2 * kPsdWarps * kPsdSmallWords * sizeof(double), st>>>(__VA_ARGS__)
 
-// sides up to kPsdPairSide take the pair-per-lane scaling: at 16 its matrices
-// still leave three blocks per SM and a row fits in registers; above, the group
-// kernels' 32 lanes are filled by one column (groups against pairs, us: side 1,
-// 1000 cones 11 / 9; side 8, 100 cones 265 / 101; side 10, 40 000 cones 3866 /
-// 601; side 16, 20 000 cones 15 100 / 1530)
-static inline bool psd_small(const ConeSet &cs) {
-  return cs.n_psd > 0 && cs.psd_nmax <= kPsdPairSide;
-}
-// The thread-per-matrix step length needs a matrix to reduce: on sides 1 and 2 the
-// group kernel's eigenvalues are found as soon as they are loaded (1000 cones,
-// groups against threads, us: side 1 13 / 19, side 2 18 / 20, side 3 34 / 25; whole
-// calls with 200 000 cones: 275 / 420, 391 / 433, 987 / 479; with 20 000 of side
-// 16: 9990 / 360).
-static inline bool psd_small_step(const ConeSet &cs) {
-  return psd_small(cs) && cs.psd_nmax > 2;
-}
-// The products from registers pass through 16 columns whatever the side, so they
-// win from side 9 on (H x and combined shift, an element per lane against a column
-// per lane, us: side 9, 200 000 cones 475 / 441 and 827 / 801; side 10, 40 000
-// cones 154 / 104 and 260 / 189), lose below 7 (side 4, 10 000 cones: 11 / 25 and
-// 15 / 36; 1000 cones 9 / 12 and 11 / 15), and between them win while the cones
-// are about one wave (side 8: 1000 cones 13 / 13 and 19 / 17, 4000 cones 17 / 15 and
-// 23 / 27, 10 000 cones 28 / 30 and 38 / 42).
+// Which kernel takes a cone goes by its own side where the kernels round
+// differently (a set with cones on both sides of a line launches both), so an
+// instance's results do not depend on what it is batched with.
+//
+// Scaling: sides up to kPsdPairSide go by pairs: at 16 its matrices still leave
+// three blocks per SM and a row fits in registers; above, the group kernels' 32
+// lanes are filled by one column (groups against pairs, us: side 1, 1000 cones 11 /
+// 9; side 8, 100 cones 265 / 101; side 10, 40 000 cones 3866 / 601; side 16, 20 000
+// cones 15 100 / 1530).
+constexpr int kPsdPairsTake = 3;
+// Step length: the thread-per-matrix form needs a matrix to reduce; on sides 1 and
+// 2 the group kernel's eigenvalues are found as soon as they are loaded (1000
+// cones, groups against threads, us: side 1 13 / 19, side 2 18 / 20, side 3 34 / 25;
+// whole calls with 200 000 cones: 275 / 420, 391 / 433, 987 / 479; with 20 000 of
+// side 16: 9990 / 360).
+constexpr int kPsdStepTake = 2;
+// The products from registers and the group kernels' are the same bits.  The former
+// pass through 16 columns whatever the side, so they win from side 9 on (H x and
+// combined shift, an element per lane against a column per lane, us: side 9, 200
+// 000 cones 475 / 441 and 827 / 801; side 10, 40 000 cones 154 / 104 and 260 / 189),
+// lose below 7 (side 4, 10 000 cones: 11 / 25 and 15 / 36; 1000 cones 9 / 12 and 11 /
+// 15), and between them win while the cones are about one wave (side 8: 1000 cones
+// 13 / 13 and 19 / 17, 4000 cones 17 / 15 and 23 / 27, 10 000 cones 28 / 30 and 38 /
+// 42).
 static inline bool psd_small_products(const ConeSet &cs) {
-  return psd_small(cs) && (cs.psd_nmax > 8 || (cs.psd_nmax > 6 && cs.n_psd <= 2000));
+  const int n = psd_cones(cs, kPsdPairsTake);
+  return n > 0 && (cs.psd_smax > 8 || (cs.psd_smax > 6 && n <= 2000));
 }
+#define LAUNCH_PSD_PRODUCT(SMALL, KERNEL, NMATS, ...)                                  \
+  do {                                                                                 \
+    const bool _small = psd_small_products(cs);                                        \
+    if (_small)                                                                        \
+      LAUNCH_PSD_SMALL(SMALL, psd_taking(cs, kPsdPairsTake, 16), __VA_ARGS__);         \
+    if (!_small || psd_cones(cs, 7 - kPsdPairsTake))                                   \
+      LAUNCH_PSD(KERNEL, NMATS, psd_taking(cs, _small ? 7 - kPsdPairsTake : 7),        \
+                 __VA_ARGS__);                                                         \
+  } while (0)
 static NonsymArgs<ExpOps> exp_args(const ConeSet &cs) {
   return NonsymArgs<ExpOps>{cs.n_exp, cs.exp_begin, cs.exp_inst, nullptr,
                             cs.exp_Hd, cs.exp_Hs, cs.exp_grad, cs.exp_z};
@@ -2883,19 +2925,19 @@ void cones_update_scaling(const ConeSet &cs, const double *s, const double *z,
   if (cs.n_pow)
     k_nonsym_update_scaling<PowOps><<<blocks_for(cs.n_pow, 128), 128, 0, st>>>(
         cs, pow_args(cs), s, z, mu, scaling);
-  if (psd_small(cs)) {
+  if (psd_cones(cs, kPsdPairsTake)) {
+    const int ns = cs.psd_smax;
     const size_t sm = (size_t)kPsdPairWarps * 8 * sizeof(double) *
-                      (2 * cs.psd_nmax * (cs.psd_nmax + 1 + (cs.psd_nmax & 1)) +
-                       2 * cs.psd_nmax);
+                      (2 * ns * (ns + 1 + (ns & 1)) + 2 * ns);
     static const bool attr = cudaFuncSetAttribute(k_psd_update_pairs,
                                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                   96 * 1024) == cudaSuccess;
     (void)attr;
     k_psd_update_pairs<<<blocks_for(cs.n_psd, 8 * kPsdPairWarps), 32 * kPsdPairWarps, sm, st>>>(
         cs, s, z, scale_ok);
-  } else {
-    LAUNCH_PSD(k_psd_update_scaling, 7, cs, s, z, scale_ok);
   }
+  if (psd_cones(cs, 7 - kPsdPairsTake))
+    LAUNCH_PSD(k_psd_update_scaling, 7, psd_taking(cs, 7 - kPsdPairsTake), s, z, scale_ok);
 }
 
 void cones_refresh_kkt(const ConeSet &cs, const KKTMapDev &map, double *kv,
@@ -2933,10 +2975,7 @@ void cones_mul_Hs(const ConeSet &cs, double *y, const double *x, cudaStream_t st
   if (cs.n_pow)
     k_nonsym_mul_hs<<<blocks_for(cs.n_pow), kBlock, 0, st>>>(cs, cs.n_pow, cs.pow_begin,
                                                             cs.pow_inst, cs.pow_Hs, y, x);
-  if (psd_small_products(cs))
-    LAUNCH_PSD_SMALL(k_psd_mul_hs_small, cs, y, x);
-  else
-    LAUNCH_PSD(k_psd_mul_hs, 3, cs, y, x);
+  LAUNCH_PSD_PRODUCT(k_psd_mul_hs_small, k_psd_mul_hs, 3, y, x);
 }
 
 void cones_affine_ds(const ConeSet &cs, double *ds, const double *s, cudaStream_t st) {
@@ -2964,10 +3003,7 @@ void cones_combined_ds_shift(const ConeSet &cs, double *shift, const double *dz,
   if (cs.n_pow)
     k_nonsym_combined<PowOps><<<blocks_for(cs.n_pow, 128), 128, 0, st>>>(
         cs, pow_args(cs), shift, dz, ds, sm);
-  if (psd_small_products(cs))
-    LAUNCH_PSD_SMALL(k_psd_combined_small, cs, shift, dz, ds, sm);
-  else
-    LAUNCH_PSD(k_psd_combined, 5, cs, shift, dz, ds, sm);
+  LAUNCH_PSD_PRODUCT(k_psd_combined_small, k_psd_combined, 5, shift, dz, ds, sm);
 }
 
 void cones_ds_from_dz_offset(const ConeSet &cs, double *out, const double *ds,
@@ -2981,10 +3017,7 @@ void cones_ds_from_dz_offset(const ConeSet &cs, double *out, const double *ds,
   if (cs.n_pow)
     k_nonsym_copy<<<blocks_for(3 * cs.n_pow), kBlock, 0, st>>>(cs, cs.n_pow, cs.pow_begin,
                                                               cs.pow_inst, out, ds);
-  if (psd_small_products(cs))
-    LAUNCH_PSD_SMALL(k_psd_ds_offset_small, cs, out, ds);
-  else
-    LAUNCH_PSD(k_psd_ds_offset, 4, cs, out, ds);
+  LAUNCH_PSD_PRODUCT(k_psd_ds_offset_small, k_psd_ds_offset, 4, out, ds);
 }
 
 void cones_step_length_sym(const ConeSet &cs, const double *dz, const double *ds,
@@ -2994,15 +3027,16 @@ void cones_step_length_sym(const ConeSet &cs, const double *dz, const double *ds
     k_nn_step<<<blocks_for(cs.n_nn, nn_block(cs) * (cs.B == 1 ? kNNRows : 1)), nn_block(cs), 0,
                 st>>>(cs, dz, ds, z, s, alpha);
   LAUNCH_SOC_SHAPED(kSocStep, k_soc_tile_step, 4, k_soc_step, dz, ds, z, s, alpha);
-  if (psd_small_step(cs)) {
-    LAUNCH_PSD_SMALL(k_psd_step_matrices, cs, dz, ds);
-    const size_t sm = (size_t)(kPsdEigThreads + 1) * (cs.psd_nmax * (cs.psd_nmax + 1) / 2 +
-                                                2 * cs.psd_nmax) * sizeof(double);
-    k_psd_step_eig<<<blocks_for(2 * cs.n_psd, kPsdEigThreads), kPsdEigThreads, sm, st>>>(cs,
+  if (psd_cones(cs, kPsdStepTake)) {
+    const ConeSet sc = psd_taking(cs, kPsdStepTake, 16);
+    LAUNCH_PSD_SMALL(k_psd_step_matrices, sc, dz, ds);
+    const size_t sm = (size_t)(kPsdEigThreads + 1) * (cs.psd_smax * (cs.psd_smax + 1) / 2 +
+                                                2 * cs.psd_smax) * sizeof(double);
+    k_psd_step_eig<<<blocks_for(2 * cs.n_psd, kPsdEigThreads), kPsdEigThreads, sm, st>>>(sc,
                                                                                       alpha);
-  } else {
-    LAUNCH_PSD(k_psd_step, 4, cs, dz, ds, alpha);
   }
+  if (psd_cones(cs, 7 - kPsdStepTake))
+    LAUNCH_PSD(k_psd_step, 4, psd_taking(cs, 7 - kPsdStepTake), dz, ds, alpha);
 }
 
 void cones_step_length_asym(const ConeSet &cs, const double *dz, const double *ds,

@@ -141,6 +141,10 @@ extern "C" int clgpu_cones_create(int ncones, const int *types, const int *dims,
   while (G < soc_max && G < 32) G <<= 1;
   cs.soc_group = G;
   cs.psd_nmax = psd_max;
+  for (int n : psd_n) {
+    cs.psd_count[psd_class(n)]++;
+    if (n <= kPsdSmallSide) cs.psd_smax = std::max(cs.psd_smax, n);
+  }
   cs.row_inst = A.upload(row_inst);
   cs.soc_off = A.upload(soc_off);
   cs.soc_dim = A.upload(soc_dim);
@@ -184,7 +188,7 @@ extern "C" int clgpu_cones_create(int ncones, const int *types, const int *dims,
   cs.psd_R = A.alloc<double>(nn2 * cs.n_psd);
   cs.psd_Rinv = A.alloc<double>(nn2 * cs.n_psd);
   cs.psd_lam = A.alloc<double>((size_t)psd_max * cs.n_psd);
-  cs.psd_eig = A.alloc<double>((size_t)psd_max * (psd_max + 1) * cs.n_psd);
+  cs.psd_eig = A.alloc<double>((size_t)cs.psd_smax * (cs.psd_smax + 1) * cs.n_psd);
   cs.cone_tmp = A.alloc<double>((size_t)cs.n_soc + cs.n_exp + cs.n_pow + cs.n_psd);
   cs.cone_tmp2 = A.alloc<double>((size_t)cs.n_soc + cs.n_exp + cs.n_pow + cs.n_psd);
   {

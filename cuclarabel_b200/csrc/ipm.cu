@@ -1238,7 +1238,12 @@ static int build_batch(clgpu_solver *h, std::vector<Prepared> &prep, int nth) {
     npsd[i] = prep[i].type_cones[5];
     for (size_t k = 0; k < prep[i].ctype.size(); ++k) {
       if (prep[i].ctype[k] == CLGPU_CONE_SOC) soc_maxdim = std::max(soc_maxdim, prep[i].cdim[k]);
-      if (prep[i].ctype[k] == CLGPU_CONE_PSD) psd_nmax = std::max(psd_nmax, prep[i].cdim[k]);
+      if (prep[i].ctype[k] == CLGPU_CONE_PSD) {
+        const int n = prep[i].cdim[k];
+        psd_nmax = std::max(psd_nmax, n);
+        cs.psd_count[psd_class(n)]++;
+        if (n <= kPsdSmallSide) cs.psd_smax = std::max(cs.psd_smax, n);
+      }
     }
   }
   if (psd_nmax > kPsdMaxSide) return -3;  // warp-per-cone kernels, matrices in shared memory
@@ -1343,7 +1348,7 @@ static int build_batch(clgpu_solver *h, std::vector<Prepared> &prep, int nth) {
   cs.psd_R = A.alloc<double>(nn2 * cs.n_psd);
   cs.psd_Rinv = A.alloc<double>(nn2 * cs.n_psd);
   cs.psd_lam = A.alloc<double>((size_t)cs.psd_nmax * cs.n_psd);
-  cs.psd_eig = A.alloc<double>((size_t)cs.psd_nmax * (cs.psd_nmax + 1) * cs.n_psd);
+  cs.psd_eig = A.alloc<double>((size_t)cs.psd_smax * (cs.psd_smax + 1) * cs.n_psd);
   cs.cone_tmp = A.alloc<double>((size_t)cs.n_soc + cs.n_exp + cs.n_pow + cs.n_psd);
   cs.cone_tmp2 = A.alloc<double>((size_t)cs.n_soc + cs.n_exp + cs.n_pow + cs.n_psd);
   mark("data + cones");

@@ -170,3 +170,50 @@ def test_psd_step_of_directions_that_are_not_finite(cuda_device):
                                      d_s.data_ptr(), 1.0, 0.99, 0.8, 1e-4, ctypes.byref(a),
                                      None) == 0
         assert a.value == want, (n, value, a.value)
+
+
+@pytest.mark.parametrize("others", [[20], [17, 1], [8] * 2100, [2, 9, 16]])
+def test_psd_results_do_not_depend_on_the_other_cones(cuda_device, others):
+    """Bit for bit, with cones beside them that take other kernels: larger sides,
+    and so many that the products go the other way."""
+    sides = [3, 8, 2, 7, 16, 1, 9, 6]
+    rng = np.random.default_rng(5)
+    s, z = (np.concatenate([interior(rng, n) for n in sides]) for _ in range(2))
+    so, zo = (np.concatenate([interior(rng, n) for n in others]) for _ in range(2))
+    d1, d2 = (rng.standard_normal(len(s)) for _ in range(2))
+    do = np.zeros(len(so))
+    res = []
+    for extra in (False, True):
+        specs = [(5, n, 0.0) for n in sides + (others if extra else [])]
+        cat = lambda a, b: np.concatenate([a, b]) if extra else a  # noqa: E731
+        G = GPUCones(specs)
+        ds, dz, a1, a2 = (G.dev(v) for v in (cat(s, so), cat(z, zo), cat(d1, do), cat(d2, do)))
+        L, st = G.L, None
+        assert L.clgpu_update_scaling(G.h, ds.data_ptr(), dz.data_ptr(), 1.0, 0, st) == 0
+        out = []
+        o = G.empty(len(cat(s, so)))
+        assert L.clgpu_mul_Hs(G.h, o.data_ptr(), a1.data_ptr(), st) == 0
+        out.append(o.cpu().numpy()[:len(s)].copy())
+        assert L.clgpu_combined_ds_shift(G.h, o.data_ptr(), a1.data_ptr(), a2.data_ptr(),
+                                         dz.data_ptr(), 0.37, st) == 0
+        out.append(o.cpu().numpy()[:len(s)].copy())
+        assert L.clgpu_ds_from_dz_offset(G.h, o.data_ptr(), a2.data_ptr(), dz.data_ptr(), st) == 0
+        out.append(o.cpu().numpy()[:len(s)].copy())
+        for k in (0.1, 3.0):
+            b1, b2 = G.dev(k * cat(d1, do)), G.dev(k * cat(d2, do))
+            a = ctypes.c_double()
+            assert L.clgpu_step_length(G.h, b1.data_ptr(), b2.data_ptr(), dz.data_ptr(),
+                                       ds.data_ptr(), 1.0, 0.99, 0.8, 1e-4, ctypes.byref(a),
+                                       st) == 0
+            out.append(np.array([a.value]))
+        res.append(out)
+    for a, b in zip(*res):
+        assert np.array_equal(a, b)
+
+
+def test_psd_programs_give_the_bits_of_each_alone(cuda_device):
+    from cuclarabel_b200 import BatchSolver, problems
+    pbs = [problems.psd_lp(n, 2, seed=n) for n in (2, 3, 8, 9, 16, 18)]
+    for pb, s in zip(pbs, BatchSolver(pbs, max_iter=5).solve()):
+        a = BatchSolver([pb], max_iter=5).solve()[0]
+        assert np.array_equal(a.x, s.x) and np.array_equal(a.s, s.s) and np.array_equal(a.z, s.z)
