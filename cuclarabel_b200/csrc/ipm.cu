@@ -15,11 +15,12 @@
 // an instance that would "break" sets done and is frozen.  All vector kernels
 // read the per-instance active mask.
 #include <algorithm>
-#include <array>
 #include <atomic>
 #include <chrono>
 #include <cstdio>
 #include <cstring>
+#include <deque>
+#include <mutex>
 #include <thread>
 
 #include "cones.cuh"
@@ -1089,6 +1090,51 @@ static SlGroups sl_groups(std::vector<int> &items, const std::vector<SlNeed> &ne
   return g;
 }
 
+// One array of the batch whose parts several threads append as they are built, in
+// page-locked pieces that are uploaded side by side: the parts' sizes are known
+// only then, and a part is copied once, while it is in the cache.
+template <typename T>
+struct Pieces {
+  size_t piece;  // elements of a piece, unless a part is larger
+  std::mutex m;
+  std::deque<hvec<T>> data;
+  std::vector<long long> filled;
+  struct At {
+    int piece;
+    long long off;
+  };
+  explicit Pieces(size_t piece) : piece(piece) {}
+  At append(const std::vector<T> &part) {
+    At at;
+    T *to;
+    {
+      std::lock_guard<std::mutex> lock(m);
+      if (data.empty() || filled.back() + part.size() > data.back().size()) {
+        data.emplace_back(std::max(piece, part.size()));
+        filled.push_back(0);
+      }
+      at = {(int)data.size() - 1, filled.back()};
+      to = data.back().data() + at.off;
+      filled.back() += (long long)part.size();
+    }
+    std::copy(part.begin(), part.end(), to);
+    return at;
+  }
+  // (after the last append) the pieces' places in the whole array
+  std::vector<long long> first;
+  long long total() {
+    first = prefix(filled);
+    return first.back();
+  }
+  long long place(At at) const { return first[at.piece] + at.off; }
+  T *upload(DevArena &A) const {
+    T *to = A.alloc<T>((size_t)first.back(), first.back() == 0);
+    for (size_t k = 0; to && k < data.size(); ++k)
+      A.copy_in(to + first[k], data[k].data(), (size_t)filled[k] * sizeof(T));
+    return to;
+  }
+};
+
 // Concatenates the prepared instances into the batch layout and uploads it.
 // Every per-instance copy runs on nth host threads: offsets first (prefix
 // sums over instances), then each instance fills its own disjoint slices.
@@ -1359,13 +1405,40 @@ static int build_batch(clgpu_solver *h, std::vector<Prepared> &prep, int nth) {
   // factor fits it, else the block kernels with global scratch (2), or the
   // supernodal path (3)
   std::vector<int> cls(B);
+  // (the plans without their three large arrays, which go to the pieces)
   std::vector<SlicedPlan> plan(B);
+  std::vector<SlNeed> need(B);
+  struct Placed {
+    Pieces<uint32_t>::At ent, ops;
+    Pieces<uint16_t>::At lpos;
+    long long vlanes, pages;
+  };
+  std::vector<Placed> placed(B, Placed{});
+  // 32 MB a piece, less for a few instances (about 24 k words of ops each)
+  const size_t piece = std::min<size_t>((size_t)8 << 20, ((size_t)16 << 10) * B);
+  Pieces<uint32_t> ent(piece), ops(piece);
+  Pieces<uint16_t> lpos(piece);
   par_for(B, nth, [&](int i) {
     cls[i] = prep[i].supernodal ? 3 : (sl_fits(prep[i]) ? 1 : 2);
-    if (cls[i] == 1 && !sl_build(prep[i], h->mixed ? 4 : 2, plan[i])) {
+    if (cls[i] != 1) return;
+    thread_local SlicedPlan own;
+    SlicedPlan &sp = own;
+    if (!sl_build(prep[i], h->mixed ? 4 : 2, sp)) {
       cls[i] = 2;
-      plan[i] = SlicedPlan();
+      return;
     }
+    need[i] = sl_need(sp);
+    placed[i] = {ent.append(sp.ent), ops.append(sp.ops), lpos.append(sp.lpos),
+                 (long long)sp.lpos.size() / kSlRun, (long long)sp.ops.size() / kSlOpWords};
+    std::vector<uint32_t> e, o;
+    std::vector<uint16_t> l;
+    e.swap(sp.ent);
+    o.swap(sp.ops);
+    l.swap(sp.lpos);
+    plan[i] = sp;
+    sp.ent.swap(e);
+    sp.ops.swap(o);
+    sp.lpos.swap(l);
   }, B < 256 ? 2 : 16);
   mark("sliced layouts");
   bool has_large = false;
@@ -1606,24 +1679,20 @@ static int build_batch(clgpu_solver *h, std::vector<Prepared> &prep, int nth) {
   }
   // ---------------- sliced layouts of the class-1 instances, concatenated
   {
-    std::vector<long long> cpage(B), clane(B), cvp(B), cop(B), cecol(B);
+    std::vector<long long> cpage(B), cecol(B);
     for (int i = 0; i < B; ++i) {
-      const SlicedPlan &sp = plan[i];
-      cpage[i] = (long long)sp.used.size();
-      clane[i] = (long long)(sp.ent.size() / 4);
-      cvp[i] = (long long)(sp.lpos.size() / kSlRun);
-      cop[i] = (long long)(sp.ops.size() / kSlOpWords);
-      cecol[i] = (long long)sp.ecol.size();
+      cpage[i] = (long long)plan[i].used.size();
+      cecol[i] = (long long)plan[i].ecol.size();
     }
-    const auto opage = prefix(cpage), olane = prefix(clane), ovp = prefix(cvp), oop = prefix(cop), oecol = prefix(cecol);
+    const auto opage = prefix(cpage), oecol = prefix(cecol);
+    const long long words = ent.total(), slots = lpos.total(), opwords = ops.total();
     // (an instance's parts begin at int offsets, counted in lanes and pages)
-    if (olane[B] > 2000000000LL || ovp[B] > 2000000000LL || oop[B] > 2000000000LL ||
-        opage[B] > 2000000000LL || oecol[B] > 2000000000LL)
+    if (words / 4 > 2000000000LL || slots / kSlRun > 2000000000LL ||
+        opwords / kSlOpWords > 2000000000LL || opage[B] > 2000000000LL ||
+        oecol[B] > 2000000000LL)
       return -4;
     std::vector<SlInst> sl(B);
-    std::vector<SlNeed> need(B);
-    hvec<uint16_t> kdst((size_t)knz), lpos(ovp[B] * kSlRun), leaf(VT), ecols(oecol[B]);
-    hvec<uint32_t> ent(olane[B] * 4), ops(oop[B] * kSlOpWords);
+    hvec<uint16_t> kdst((size_t)knz), leaf(VT), ecols(oecol[B]);
     hvec<int> kdiag(VT);
     hvec<uint8_t> used(opage[B]);
     hvec<signed char> sign(VT);
@@ -1632,7 +1701,6 @@ static int build_batch(clgpu_solver *h, std::vector<Prepared> &prep, int nth) {
       d = SlInst{};
       if (cls[i] != 1) return;
       SlicedPlan &sp = plan[i];
-      need[i] = sl_need(sp);
       d.N = sp.N;
       d.nl = sp.nl;
       d.nk = (int)sp.kslot.size();
@@ -1641,13 +1709,13 @@ static int build_batch(clgpu_solver *h, std::vector<Prepared> &prep, int nth) {
       d.nf = sp.nstage[0];
       d.nb = sp.nstage[1];
       d.nr = sp.nstage[2];
-      d.lane0 = (int)olane[i];
-      d.vlane0 = (int)ovp[i];
-      d.nvlane = (int)cvp[i];
+      d.lane0 = (int)(ent.place(placed[i].ent) / 4);
+      d.vlane0 = (int)(lpos.place(placed[i].lpos) / kSlRun);
+      d.nvlane = (int)placed[i].vlanes;
       d.kx0 = (int)kof[i];
       d.nkx = (int)sp.kdst.size();
-      d.opage0 = (int)oop[i];
-      d.nops = (int)sp.ops.size();
+      d.opage0 = (int)(ops.place(placed[i].ops) / kSlOpWords);
+      d.nops = (int)placed[i].pages * kSlOpWords;
       d.nleaf = (int)sp.leaf.size();
       d.ncarry = sp.ncarry;
       d.nopcarry = sp.nopcarry;
@@ -1658,14 +1726,11 @@ static int build_batch(clgpu_solver *h, std::vector<Prepared> &prep, int nth) {
         std::copy(src.begin(), src.begin() + n, dst.begin() + at);
       };
       put(kdst, kof[i], sp.kdst, sp.kdst.size());
-      put(lpos, ovp[i] * kSlRun, sp.lpos, sp.lpos.size());
       put(used, opage[i], sp.used, sp.used.size());
       put(leaf, voff[i], sp.leaf, sp.leaf.size());
       put(sign, voff[i], sp.sign, sp.sign.size());
       for (int r = 0; r < sp.N; ++r) kdiag[voff[i] + r] = sp.kslot[prep[i].Kdiag[r]];
       put(ecols, oecol[i], sp.ecol, sp.ecol.size());
-      put(ent, olane[i] * 4, sp.ent, sp.ent.size());
-      put(ops, oop[i] * kSlOpWords, sp.ops, sp.ops.size());
       sp = SlicedPlan();  // freed here, by all threads
     });
     if (h->st.verbose) {
@@ -1677,19 +1742,19 @@ static int build_batch(clgpu_solver *h, std::vector<Prepared> &prep, int nth) {
       std::fprintf(stderr,
                    "clgpu setup: sliced L entries %lld in %lld slots (both passes), K %lld in "
                    "%lld, op words %lld\n",
-                   nl, ovp[B] * kSlRun, nk, knz, oop[B] * kSlOpWords);
+                   nl, slots, nk, knz, opwords);
     }
     kk.sl = A.upload(sl);
     kk.sl_kdst = A.upload(kdst);
     kk.sl_kdiag = A.upload(kdiag);
     kk.sl_used = A.upload(used);
-    kk.sl_ent = A.upload(ent);
-    kk.sl_ops = A.upload(ops);
-    kk.sl_lpos = A.upload(lpos);
+    kk.sl_ent = ent.upload(A);
+    kk.sl_ops = ops.upload(A);
+    kk.sl_lpos = lpos.upload(A);
     kk.sl_leaf = A.upload(leaf);
     kk.sl_sign = A.upload(sign);
     kk.sl_ecol = A.upload(ecols);
-    const size_t nval = (size_t)(ovp[B] * kSlRun);
+    const size_t nval = (size_t)slots;
     kk.sl_val = h->mixed ? (void *)A.alloc<float>(nval, false) : A.alloc<double>(nval, false);
     // launch order: the largest need of shared memory first
     std::vector<int> so, fo;

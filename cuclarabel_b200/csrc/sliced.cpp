@@ -1,83 +1,139 @@
 // sliced.cpp -- builds the layouts of sliced.hpp from a prepared instance.
+//
+// What bounds it: short loops (a row of L has three terms, a level a few dozen
+// rows) whose exits the host mispredicts, some 15 k terms and operations an
+// instance.  So parts point at their terms where these already lie, lanes are
+// written once, to their final place, and the operations of a level are listed
+// in one sweep and sorted flat.  The first form, which copied terms, filled pages
+// and then copied them into stages, took 430 us an instance of the MPC family
+// (4096 of them: 97-104 ms on 16 threads); this takes 290 us (58 ms).
 #include "sliced.hpp"
 
 #include <algorithm>
 #include <cstring>
+#include <type_traits>
 
 namespace clgpu {
 
 namespace {
 
-// A segment's part inside one chunk: its first term in the stream, terms, and
-// which part of the segment it is.
+// A segment's part inside one chunk: its first term in the stream and in its
+// source array, terms, lanes; where its sum goes, or the carry it starts from or
+// leaves (-1: none).
 struct Part {
-  int first, len, seg, lanes;
-  bool more, scan_last;  // continued in the next chunk; last lane's run is full
+  int first, src, len, to;
   int carry_in, carry_out;
+  int lanes;
+  bool scan_last;  // the last lane's run is full
 };
 
-// The parts of a stream's segments (ends[s] = one past segment s's last term,
-// from `begin`), chunk length 32 R, by phase: part i of a segment is in phase
-// i, which needs phase i - 1's carries.  Carry slots count from 0.
+// The parts of a stream's segments, chunk length 32 R, by phase: part i of a
+// segment is in phase i, which needs phase i - 1's carries.  Carry slots count
+// from 0.
 struct Splitter {
-  std::vector<std::vector<Part>> phase;
+  std::vector<std::vector<Part>> phase{1};
   int nphase = 0, ncarry = 0;
   void start() {
     for (int i = 0; i < nphase; ++i) phase[i].clear();
     nphase = ncarry = 0;
   }
-  // terms [p0, p1) of the stream, which starts at position 0 of a chunk
-  void add(int seg, int p0, int p1, int R) {
-    const int chunk = 32 * R;
-    int carry = -1;
+  // terms [p0, p1) of the stream, at src in their source
+  template <int R>
+  void add(int to, int src, int p0, int p1) {
+    constexpr int chunk = 32 * R;
+    if (p0 >= p1) return;
+    if (p0 / chunk == (p1 - 1) / chunk) {
+      nphase = std::max(nphase, 1);
+      phase[0].push_back({p0, src, p1 - p0, to, -1, -1,
+                          (p1 - 1) % chunk / R - p0 % chunk / R + 1, (p1 - 1) % R == R - 1});
+      return;
+    }
+    const int carry = ncarry++;
     for (int a = p0, i = 0; a < p1; ++i) {
       const int b = std::min(p1, (a / chunk + 1) * chunk);
       if (i == (int)phase.size()) phase.emplace_back();
       nphase = std::max(nphase, i + 1);
-      const int la = a % chunk / R, lb = (b - 1) % chunk / R;
-      Part q{a, b - a, seg, lb - la + 1, b < p1, (b - 1) % R == R - 1, i > 0 ? carry : -1, -1};
-      if (b < p1) {
-        if (carry < 0) carry = ncarry++;
-        q.carry_out = carry;
-      }
-      phase[i].push_back(q);
+      phase[i].push_back({a, src + (a - p0), b - a, to, i > 0 ? carry : -1, b < p1 ? carry : -1,
+                          (b - 1) % chunk / R - a % chunk / R + 1, (b - 1) % R == R - 1});
       a = b;
     }
   }
 };
 
-// Fills pages with whole parts, widest first, so a page's parts need about
-// the same scan steps.
-struct Packer {
-  std::vector<int> order, cnt;
-  std::vector<std::pair<int, int>> at;  // per part: page, first lane
-  int npages = 0;
-  void pack(const std::vector<Part> &parts) {
-    const int n = (int)parts.size();
-    cnt.assign(34, 0);
-    for (const Part &q : parts) cnt[33 - q.lanes]++;
-    for (int i = 1; i < 34; ++i) cnt[i] += cnt[i - 1];
-    order.resize(n);
-    for (int i = n - 1; i >= 0; --i) order[--cnt[33 - parts[i].lanes]] = i;
-    at.resize(n);
-    npages = 0;
-    int lane = 32;
-    for (int i : order) {
-      if (lane + parts[i].lanes > 32) {
-        ++npages;
-        lane = 0;
-      }
-      at[i] = {npages - 1, lane};
-      lane += parts[i].lanes;
-    }
-  }
-};
-
+// steps a scan takes to add `reach` lanes back
 int scan_steps(int reach) {
   int s = 0;
   for (int d = 1; d <= reach; d <<= 1) ++s;
   return s;
 }
+// The last lane of a part that ends inside its run is not scanned: it adds the
+// previous lane's scanned sum.
+bool adds_previous(const Part &q) { return !q.scan_last && q.lanes > 1; }
+
+// Fills pages with whole parts, widest first, so a page's parts need about
+// the same scan steps.
+struct Packer {
+  struct Page {
+    int used, steps;  // lanes with a part; the widest part's scan steps
+    bool prev, carry;  // some lane adds the previous one's sum; starts from a carry
+  };
+  std::vector<int> order;
+  std::vector<std::pair<int, int>> at;  // per part: page, first lane
+  std::vector<Page> pages;
+  void pack(const std::vector<Part> &parts) {
+    static const struct Steps {
+      int of[33];
+      Steps() {
+        for (int r = 0; r < 33; ++r) of[r] = scan_steps(r);
+      }
+    } steps;
+    const int n = (int)parts.size();
+    int cnt[34] = {};
+    for (const Part &q : parts) cnt[33 - q.lanes]++;
+    for (int i = 1; i < 34; ++i) cnt[i] += cnt[i - 1];
+    order.resize(n);
+    for (int i = n - 1; i >= 0; --i) order[--cnt[33 - parts[i].lanes]] = i;
+    at.resize(n);
+    pages.clear();
+    int lane = 32;
+    for (int i : order) {
+      const Part &q = parts[i];
+      if (lane + q.lanes > 32) {
+        pages.push_back({0, 0, false, false});
+        lane = 0;
+      }
+      Page &pg = pages.back();
+      at[i] = {(int)pages.size() - 1, lane};
+      lane += q.lanes;
+      const bool prev = adds_previous(q);
+      pg.used = lane;
+      pg.steps = std::max(pg.steps, steps.of[q.lanes - (prev ? 2 : 1)]);
+      pg.prev = pg.prev || prev;
+      pg.carry = pg.carry || q.carry_in >= 0;
+    }
+  }
+};
+
+struct Op {
+  uint16_t a, b, k;
+};
+struct Place {
+  int lane0, in_stage, used;  // first stored lane, lane in the stage, stage's lanes
+};
+struct Mark {
+  int of, at;
+};
+// A thread's working arrays, kept between instances (taken by reference once: a
+// thread_local's address is looked up at every use).
+struct Work {
+  Splitter split;
+  Packer packer;
+  std::vector<Place> place;
+  std::vector<Mark> mark;
+  std::vector<Op> lev, found;
+  std::vector<int> nodes, target_of, cnt, segs, target, page_of;
+  std::vector<uint32_t> opg[kSlWarps];
+};
 
 }  // namespace
 
@@ -86,174 +142,132 @@ bool sl_build(const Prepared &p, int vgroup, SlicedPlan &s) {
   s.N = N;
   s.nl = nl;
   s.nlev = nlev;
-  thread_local Splitter split;
-  thread_local Packer packer;
-  // one pass's pages, and the first page of every stage
-  struct Pages {
-    std::vector<uint32_t> ent;
-    std::vector<int> pos;    // value position of every term, -1: none
-    std::vector<int> used;   // lanes of every page
-    std::vector<int> stage;
-    void clear() {
-      ent.clear();
-      pos.clear();
-      used.clear();
-      stage.clear();
-    }
-  };
-  thread_local Pages pass[3];
-  thread_local std::vector<int> term_slot, term_pos, seg_target;
+  thread_local Work own;
+  Work &work = own;
+  Splitter &split = work.split;
+  Packer &packer = work.packer;
+  auto &place = work.place;
   s.ncarry = 0;
-  const uint32_t pad = 8u * (uint32_t)N | ((uint32_t)N << 16);
-  // The level's split parts into pages, phase by phase, and those into stages.
-  // Terms are term_slot / term_pos, targets seg_target.
-  auto emit = [&](Pages &P) {
+  s.ent.clear();
+  s.lpos.clear();
+  s.used.clear();
+  s.kslot.resize(p.Kj.size());
+  for (int &n : s.nstage) n = 0;
+  int nlane = 0, nklane = 0;  // lanes of the factor passes, of the residual
+  const uint32_t pad = 8u * (uint32_t)N, none = (uint32_t)N << 16;
+  // One pass's level: its split parts into pages, phase by phase, and those into
+  // stages.  slot[src]: gathered slot of a term; pos(src): its factor entry.
+  auto emit = [&](auto which, const int *slot, auto pos) {
+    constexpr int pass = decltype(which)::value;
     s.ncarry = std::max(s.ncarry, split.ncarry);
+    int &base = pass < 2 ? nlane : nklane;
     for (int ph = 0; ph < split.nphase; ++ph) {
       const auto &parts = split.phase[ph];
       packer.pack(parts);
-      const int p0 = (int)P.used.size();
-      for (int i = 0; i < packer.npages; i += kSlStagePages) P.stage.push_back(p0 + i);
-      P.used.resize(p0 + packer.npages, 0);
-      P.ent.resize((size_t)(p0 + packer.npages) * kSlPage, pad);
-      P.pos.resize((size_t)(p0 + packer.npages) * kSlPage, -1);
-      for (int i = p0; i < p0 + packer.npages; ++i)
-        for (int l = 0; l < 32; ++l) {
-          P.ent[(size_t)i * kSlPage + 4 * l + 1] = pad & 0xffffu;
-          P.ent[(size_t)i * kSlPage + 4 * l + 3] = pad & 0xffffu;
+      const int np = (int)packer.pages.size(), first = base;
+      place.resize(np);
+      for (int i = 0; i < np; i += kSlStagePages) {
+        const int last = std::min(np, i + kSlStagePages) - 1;
+        // every page but the last with all its lanes
+        const int used = 32 * (last - i) + packer.pages[last].used;
+        s.used.push_back((uint8_t)used);
+        s.nstage[pass]++;
+        for (int k = i; k <= last; ++k) place[k] = {base + 32 * (k - i), 32 * (k - i), used};
+        base += used;
+      }
+      const size_t e0 = s.ent.size();
+      s.ent.resize(e0 + 4 * (size_t)(base - first));
+      uint32_t *ent = s.ent.data() + e0;
+      if (pass < 2) s.lpos.resize((size_t)base * kSlRun, kSlNone);
+      uint16_t *lpos = s.lpos.data();
+      int *kslot = s.kslot.data();
+      auto control = [&](const Packer::Page &pg) {
+        return (uint32_t)(pg.steps | (pg.carry ? 8 : 0) | (pg.prev ? 16 : 0)) << 16;
+      };
+      for (int k = 0; k < np; ++k) {  // lanes without a part
+        const Packer::Page &pg = packer.pages[k];
+        const int end = std::min(32, place[k].used - place[k].in_stage);
+        for (int l = pg.used; l < end; ++l) {
+          uint32_t *w = ent + 4 * (place[k].lane0 - first + l);
+          w[0] = w[2] = pad | none;
+          w[1] = pad;
+          w[3] = pad | control(pg);
         }
-      for (size_t i = 0; i < parts.size(); ++i) {
+      }
+      for (int i : packer.order) {  // (parts of equal widths one after the other)
         const Part &q = parts[i];
-        const int pgi = p0 + packer.at[i].first, l0 = packer.at[i].second;
-        uint32_t *e = P.ent.data() + (size_t)pgi * kSlPage;
-        int *pos = P.pos.data() + (size_t)pgi * kSlPage;
-        P.used[pgi] = std::max(P.used[pgi], l0 + q.lanes);
-        int reach = 0;
-        int t = q.first;
-        const int end = q.first + q.len;
-        for (int r = 0; r < q.lanes; ++r) {
-          uint32_t *el = e + 4 * (l0 + r);
-          for (int c = 0; t < end && (c == 0 || t % kSlRun != 0); ++c, ++t) {
-            el[c] = (el[c] & 0xffff0000u) | (uint32_t)(8 * term_slot[t]);
-            pos[4 * (l0 + r) + c] = term_pos[t];
+        const Packer::Page &pg = packer.pages[packer.at[i].first];
+        const Place &pl = place[packer.at[i].first];
+        const int l0 = packer.at[i].second;
+        const uint32_t ctl = control(pg);
+        const bool prev = adds_previous(q);
+        const int to = q.carry_out >= 0 ? N + 1 + q.carry_out : q.to;
+        uint32_t *w = ent + 4 * (pl.lane0 - first + l0);
+        int x = q.src, left = q.len, room = kSlRun - q.first % kSlRun;
+        for (int r = 0; r < q.lanes; ++r, w += 4) {
+          const int n = std::min(left, room), lane = pl.in_stage + l0 + r;
+          // positions of the run's terms: sl_at of (0 .. 3, lane)
+          const int v = pass < 2 ? vgroup : 2;
+          const int v0 = (pl.lane0 - pl.in_stage) * kSlRun + lane * v;
+          const int v2 = v0 + (v == 2 ? 2 * pl.used : 2);
+          const int at[kSlRun] = {v0, v0 + 1, v2, v2 + 1};
+          uint32_t id[kSlRun] = {pad, pad, pad, pad};
+          for (int c = 0; c < n; ++c) {
+            id[c] = 8u * (uint32_t)slot[x + c];
+            if (pass < 2)
+              lpos[at[c]] = (uint16_t)pos(x + c);
+            else
+              kslot[x + c] = at[c];
           }
           const bool last = r == q.lanes - 1;
-          const bool prev = last && !q.scan_last && r > 0;
-          el[1] = (el[1] & 0xffffu) | ((uint32_t)(prev ? 32 : r) << 16);
-          if (!prev)
-            reach = std::max(reach, r);
-          else if (!(e[3] & (16u << 16)))
-            for (int l = 0; l < 32; ++l) e[4 * l + 3] |= 16u << 16;
-          if (last) {
-            const int to = q.more ? N + 1 + q.carry_out : seg_target[q.seg];
-            el[0] = (el[0] & 0xffffu) | ((uint32_t)to << 16);
-          }
-          if (r == 0 && q.carry_in >= 0) {
-            el[2] = (el[2] & 0xffffu) | ((uint32_t)(N + 1 + q.carry_in) << 16);
-            if (!(e[3] & (8u << 16)))
-              for (int l = 0; l < 32; ++l) e[4 * l + 3] |= 8u << 16;
-          }
+          w[0] = id[0] | (last ? (uint32_t)to << 16 : none);
+          w[1] = id[1] | (uint32_t)(last && prev ? 32 : r) << 16;
+          w[2] = id[2] | (r == 0 && q.carry_in >= 0 ? (uint32_t)(N + 1 + q.carry_in) << 16 : none);
+          w[3] = id[3] | ctl;
+          x += n;
+          left -= n;
+          room = kSlRun;
         }
-        const uint32_t steps = (uint32_t)scan_steps(reach);
-        if (((e[3] >> 16) & 7u) < steps)
-          for (int l = 0; l < 32; ++l) e[4 * l + 3] = (e[4 * l + 3] & ~(7u << 16)) | (steps << 16);
       }
     }
   };
   // ---- substitutions: rows of L, leaves first; columns of L, roots first
   for (int dir = 0; dir < 2; ++dir) {
     const bool fwd = dir == 0;
-    const auto &Xp = fwd ? p.Rp : p.Lp;
-    const auto &Xi = fwd ? p.Rk : p.Li;
-    Pages &pg = pass[dir];
-    pg.clear();
+    const int *Xp = fwd ? p.Rp.data() : p.Lp.data();
     for (int ll = 0; ll < nlev; ++ll) {
       const int l = fwd ? ll : nlev - 1 - ll;
       split.start();
-      term_slot.clear();
-      term_pos.clear();
-      seg_target.clear();
+      int at = 0;
       for (int t = p.lvl_ptr[l]; t < p.lvl_ptr[l + 1]; ++t) {
-        const int j = p.lvl_nodes[t], p0 = (int)term_slot.size();
-        for (int x = Xp[j]; x < Xp[j + 1]; ++x) {
-          term_slot.push_back(Xi[x]);
-          term_pos.push_back(fwd ? p.Rpos[x] : x);
-        }
-        if ((int)term_slot.size() == p0) continue;
-        split.add((int)seg_target.size(), p0, (int)term_slot.size(), kSlRun);
-        seg_target.push_back(j);
+        const int j = p.lvl_nodes[t], len = Xp[j + 1] - Xp[j];
+        split.add<kSlRun>(j, Xp[j], at, at + len);
+        at += len;
       }
-      if (seg_target.empty()) continue;
-      emit(pg);
+      if (fwd)
+        emit(std::integral_constant<int, 0>(), p.Rk.data(), [&](int x) { return p.Rpos[x]; });
+      else
+        emit(std::integral_constant<int, 1>(), p.Li.data(), [](int x) { return x; });
     }
   }
   // ---- residual: the rows of K as one stream
-  {
-    pass[2].clear();
-    split.start();
-    const int nk = (int)p.Kj.size();
-    term_slot.assign(p.Kj.begin(), p.Kj.end());
-    term_pos.resize(nk);
-    for (int t = 0; t < nk; ++t) term_pos[t] = t;
-    seg_target.resize(N);
-    for (int r = 0; r < N; ++r) {
-      seg_target[r] = r;
-      split.add(r, p.Kp[r], p.Kp[r + 1], kSlRun);
-    }
-    emit(pass[2]);
-  }
+  split.start();
+  for (int r = 0; r < N; ++r) split.add<kSlRun>(r, p.Kp[r], p.Kp[r], p.Kp[r + 1]);
+  emit(std::integral_constant<int, 2>(), p.Kj.data(), [](int x) { return x; });
   if (8 * (N + 1 + s.ncarry) >= 0xffff) return false;
-  // ---- stage arrays, pass by pass
-  s.ent.clear();
-  s.lpos.clear();
-  s.used.clear();
-  s.kslot.resize(p.Kj.size());
-  int nklane = 0;
-  for (int ps = 0; ps < 3; ++ps) {
-    Pages &P = pass[ps];
-    s.nstage[ps] = (int)P.stage.size();
-    P.stage.push_back((int)P.used.size());
-    for (int st = 0; st < s.nstage[ps]; ++st) {
-      const int pa = P.stage[st], pb = P.stage[st + 1];
-      // every page but the last with all its lanes
-      const int used = 32 * (pb - pa - 1) + P.used[pb - 1];
-      const uint32_t *e = P.ent.data() + (size_t)pa * kSlPage;
-      const int *pos = P.pos.data() + (size_t)pa * kSlPage;
-      s.used.push_back((uint8_t)used);
-      s.ent.insert(s.ent.end(), e, e + 4 * used);
-      const size_t v0 = s.lpos.size();
-      if (ps < 2) s.lpos.resize(v0 + (size_t)used * kSlRun, kSlNone);
-      for (int l = 0; l < used; ++l)
-        for (int c = 0; c < kSlRun; ++c) {
-          const int x = pos[4 * l + c];
-          if (x < 0) continue;
-          if (ps == 2)
-            s.kslot[x] = nklane * kSlRun + sl_at(c, l, 2, used);
-          else
-            s.lpos[v0 + sl_at(c, l, vgroup, used)] = (uint16_t)x;
-        }
-      if (ps == 2) nklane += used;
-    }
-  }
   // ---- the work position every stored K value initialises
   s.kdst.assign((size_t)nklane * kSlRun, kSlNone);
-  {
-    thread_local std::vector<int> mark, at;
-    mark.assign(N, -1);
-    at.resize(N);
-    for (int r = 0; r < N; ++r) {
-      for (int t = p.Rp[r]; t < p.Rp[r + 1]; ++t) {
-        mark[p.Rk[t]] = r;
-        at[p.Rk[t]] = p.Rpos[t];
-      }
-      for (int t = p.Kp[r]; t < p.Kp[r + 1]; ++t) {
-        const int col = p.Kj[t];
-        if (col == r) {
-          s.kdst[s.kslot[t]] = (uint16_t)r;
-        } else if (col < r) {
-          if (mark[col] != r) return false;  // not inside the factor's pattern
-          s.kdst[s.kslot[t]] = (uint16_t)(N + at[col]);
-        }
+  work.mark.assign(N, {-1, 0});
+  Mark *mark = work.mark.data();
+  for (int r = 0; r < N; ++r) {
+    for (int t = p.Rp[r]; t < p.Rp[r + 1]; ++t) mark[p.Rk[t]] = {r, p.Rpos[t]};
+    for (int t = p.Kp[r]; t < p.Kp[r + 1]; ++t) {
+      const int col = p.Kj[t];
+      if (col == r) {
+        s.kdst[s.kslot[t]] = (uint16_t)r;
+      } else if (col < r) {
+        if (mark[col].of != r) return false;  // not inside the factor's pattern
+        s.kdst[s.kslot[t]] = (uint16_t)(N + mark[col].at);
       }
     }
   }
@@ -262,16 +276,19 @@ bool sl_build(const Prepared &p, int vgroup, SlicedPlan &s) {
   // d_k), grouped by target, targets in increasing order; the stream is cut
   // into kSlWarps parts of about equal length at segment starts, chunks start
   // anew in each
-  struct Op {
-    uint16_t a, b, k;
-  };
-  thread_local std::vector<Op> lev;
-  thread_local std::vector<int> nodes, cnt, segs, target, rowpos, rowmark;
-  thread_local std::vector<uint32_t> opg[kSlWarps];
-  thread_local std::vector<int> page_of;
-  if ((int)rowpos.size() < N) rowpos.resize(N);
-  rowmark.assign(N, -1);
-  int oskip[kSlWarps] = {};
+  auto &nodes = work.nodes, &cnt = work.cnt, &segs = work.segs, &target = work.target,
+       &page_of = work.page_of;
+  auto &opg = work.opg;
+  size_t nops = p.Rk.size();  // every op of the instance, so of any level
+  for (size_t r = 0; r < p.Rk.size(); ++r) nops += p.Lp[p.Rk[r] + 1] - p.Rpos[r] - 1;
+  if (work.lev.size() < nops) {
+    work.lev.resize(nops);
+    work.found.resize(nops);
+    work.target_of.resize(nops);
+  }
+  Op *lev = work.lev.data(), *found = work.found.data();
+  int *target_of = work.target_of.data();
+  int oskip[kSlWarps] = {}, ends[kSlWarps] = {};
   for (auto &o : opg) o.clear();
   s.nopcarry = 0;
   s.olevels = 0;
@@ -279,7 +296,7 @@ bool sl_build(const Prepared &p, int vgroup, SlicedPlan &s) {
   for (int j = 0; j < N; ++j)
     for (int q = p.Lp[j]; q < p.Lp[j + 1]; ++q) s.ecol[q] = (uint16_t)j;
   s.sign.assign(p.Dsign.begin(), p.Dsign.end());
-  s.leaf.clear();
+  s.leaf.assign(p.lvl_nodes.begin() + p.lvl_ptr[0], p.lvl_nodes.begin() + p.lvl_ptr[1]);
   const int zero = N + nl;
   // one lane of an op page (the fields of sliced.hpp)
   auto encode = [](uint32_t *w, const Op &o0, const Op &o1, uint32_t t, uint32_t ini,
@@ -289,66 +306,66 @@ bool sl_build(const Prepared &p, int vgroup, SlicedPlan &s) {
     w[2] = ((uint32_t)o1.b >> 6) | ((uint32_t)o1.k << 9) | (t << 22);
     w[3] = (t >> 10) | (ini << 5) | (meta << 16);
   };
-  auto none = [&](uint16_t k) { return Op{(uint16_t)zero, (uint16_t)zero, k}; };
+  const Op none_op{(uint16_t)zero, (uint16_t)zero, 0};
   uint32_t padw[4];
-  encode(padw, none(0), none(0), (uint32_t)zero, 0u, 0u);
-  thread_local std::vector<int> page_reach;
-  for (int l = 0; l < nlev; ++l) {
-    const int qa = p.lvl_ptr[l], qb = p.lvl_ptr[l + 1];
-    if (l == 0) {
-      s.leaf.assign(p.lvl_nodes.begin() + qa, p.lvl_nodes.begin() + qb);
-      continue;
-    }
-    nodes.assign(p.lvl_nodes.begin() + qa, p.lvl_nodes.begin() + qb);
+  encode(padw, none_op, none_op, (uint32_t)zero, 0u, 0u);
+  // the level ends a warp's last page has collected, written with its next page
+  auto settle = [&](int w) {
+    if (opg[w].empty() || !ends[w]) return;
+    uint32_t *e = opg[w].data() + opg[w].size() - kSlOpWords;
+    for (int l = 0; l < 32; ++l) e[4 * l + 3] |= (uint32_t)ends[w] << 25;
+    ends[w] = 0;
+  };
+  work.mark.assign(N, {-1, 0});
+  const int *Li = p.Li.data(), *Lp = p.Lp.data();
+  for (int l = 1; l < nlev; ++l) {
+    nodes.assign(p.lvl_nodes.begin() + p.lvl_ptr[l], p.lvl_nodes.begin() + p.lvl_ptr[l + 1]);
     std::sort(nodes.begin(), nodes.end());
-    size_t nop = 0;
-    for (int j : nodes)
-      for (int r = p.Rp[j]; r < p.Rp[j + 1]; ++r) nop += p.Lp[p.Rk[r] + 1] - p.Rpos[r];
-    if (lev.size() < nop) lev.resize(nop);
+    // one sweep lists the diagonals' ops in place and the entries' in the order
+    // they are found, each with its entry's place in the level
     segs.clear();
     target.clear();
-    int f = 0;
+    int nent = 0, nd = 0, nf = 0;
     for (int j : nodes) {
-      if (p.Rp[j + 1] > p.Rp[j]) {
-        segs.push_back(f);
-        target.push_back(j);
-      }
-      for (int r = p.Rp[j]; r < p.Rp[j + 1]; ++r) {
-        const uint16_t e = (uint16_t)(N + p.Rpos[r]);
-        lev[f++] = {e, e, (uint16_t)p.Rk[r]};
-      }
-    }
-    for (int j : nodes) {
-      if (p.Rp[j + 1] == p.Rp[j]) continue;
-      const int q0 = p.Lp[j], len = p.Lp[j + 1] - q0;
-      cnt.assign(len + 1, 0);
-      for (int q = q0; q < q0 + len; ++q) {
-        rowpos[p.Li[q]] = q - q0;
-        rowmark[p.Li[q]] = j;
-      }
-      for (int r = p.Rp[j]; r < p.Rp[j + 1]; ++r) {
-        const int k = p.Rk[r];
-        for (int pp = p.Rpos[r] + 1; pp < p.Lp[k + 1]; ++pp) {
-          if (rowmark[p.Li[pp]] != j) return false;  // fill outside the pattern
-          cnt[rowpos[p.Li[pp]] + 1]++;
+      const int r0 = p.Rp[j], r1 = p.Rp[j + 1], q0 = Lp[j], len = Lp[j + 1] - q0;
+      if (r0 == r1) continue;
+      segs.push_back(nd);
+      target.push_back(j);
+      for (int q = 0; q < len; ++q) mark[Li[q0 + q]] = {j, nent + q};
+      bool inside = true;
+      for (int r = r0; r < r1; ++r) {
+        const int k = p.Rk[r], pjk = p.Rpos[r], pe = Lp[k + 1];
+        const uint16_t b = (uint16_t)(N + pjk), kk = (uint16_t)k;
+        lev[nd++] = {b, b, kk};
+        for (int pp = pjk + 1; pp < pe; ++pp, ++nf) {
+          const Mark m = mark[Li[pp]];
+          inside &= m.of == j;
+          target_of[nf] = m.at;
+          found[nf] = {(uint16_t)(N + pp), b, kk};
         }
       }
-      for (int a = 0; a < len; ++a) {
-        if (cnt[a + 1]) {
-          segs.push_back(f + cnt[a]);
-          target.push_back(N + q0 + a);
-        }
-        cnt[a + 1] += cnt[a];
-      }
-      const int total = cnt[len];
-      for (int r = p.Rp[j]; r < p.Rp[j + 1]; ++r) {
-        const int k = p.Rk[r], pjk = p.Rpos[r];
-        for (int pp = pjk + 1; pp < p.Lp[k + 1]; ++pp)
-          lev[f + cnt[rowpos[p.Li[pp]]]++] = {(uint16_t)(N + pp), (uint16_t)(N + pjk),
-                                              (uint16_t)k};
-      }
-      f += total;
+      if (!inside) return false;  // fill outside the pattern
+      nent += len;
     }
+    // sorted by entry, in the order found (columns of L lie in node order)
+    cnt.assign(nent + 1, 0);
+    for (int t = 0; t < nf; ++t) cnt[target_of[t]]++;
+    const int f = nd + nf;
+    {
+      int at = nd, e = 0;
+      for (int j : nodes) {
+        if (p.Rp[j] == p.Rp[j + 1]) continue;
+        for (int q = Lp[j]; q < Lp[j + 1]; ++q, ++e) {
+          const int n = cnt[e];
+          cnt[e] = at;
+          if (!n) continue;
+          segs.push_back(at);
+          target.push_back(N + q);
+          at += n;
+        }
+      }
+    }
+    for (int t = 0; t < nf; ++t) lev[cnt[target_of[t]]++] = found[t];
     const int nseg = (int)segs.size();
     segs.push_back(f);
     int sb[kSlWarps + 1];
@@ -359,25 +376,17 @@ bool sl_build(const Prepared &p, int vgroup, SlicedPlan &s) {
       const int g = (int)(std::lower_bound(segs.begin(), segs.end(), ideal) - segs.begin());
       sb[w] = std::min(nseg, std::max(sb[w - 1], g));
     }
-    // split: every stream part starts a chunk; positions in the level are kept
-    // by aligning each part's start to a chunk boundary of a common stream
+    // every stream part starts a chunk of the common stream
     split.start();
     constexpr int chunk = 32 * kSlOpRun;
-    int base[kSlWarps], at0 = 0;
-    for (int w = 0; w < kSlWarps; ++w) {
+    for (int w = 0, at = 0; w < kSlWarps; ++w) {
       const int s0 = segs[sb[w]];
-      base[w] = s0 - at0;  // stream position -> level position
       for (int g = sb[w]; g < sb[w + 1]; ++g)
-        split.add(g, segs[g] - base[w], segs[g + 1] - base[w], kSlOpRun);
-      at0 += (segs[sb[w + 1]] - s0 + chunk - 1) / chunk * chunk;
+        split.add<kSlOpRun>(target[g], segs[g], segs[g] - s0 + at, segs[g + 1] - s0 + at);
+      at += (segs[sb[w + 1]] - s0 + chunk - 1) / chunk * chunk;
     }
     s.nopcarry = std::max(s.nopcarry, split.ncarry);
     if (zero + s.nopcarry >= 1 << kSlOpT.width || s.nopcarry >= 1 << kSlOpIni.width) return false;
-    auto part_of = [&](int g) {
-      int w = 0;
-      while (g >= sb[w + 1]) ++w;
-      return w;
-    };
     for (int ph = 0; ph < split.nphase; ++ph) {
       const auto &parts = split.phase[ph];
       packer.pack(parts);
@@ -385,57 +394,58 @@ bool sl_build(const Prepared &p, int vgroup, SlicedPlan &s) {
       for (int w = 0; w < kSlWarps; ++w) rank[w] = w;
       std::stable_sort(rank, rank + kSlWarps,
                        [&](int a, int b) { return opg[a].size() < opg[b].size(); });
-      page_of.resize(packer.npages);
-      for (int i = 0; i < packer.npages; ++i) {
-        auto &O = opg[rank[i % kSlWarps]];
-        page_of[i] = (int)(O.size() / kSlOpWords);
+      const int np = (int)packer.pages.size();
+      page_of.resize(np);
+      for (int i = 0; i < np; ++i) {
+        const int w = rank[i % kSlWarps];
+        settle(w);
+        auto &O = opg[w];
+        page_of[i] = (int)O.size();
         O.resize(O.size() + kSlOpWords);
-        uint32_t *w = O.data() + (size_t)page_of[i] * kSlOpWords;
-        for (int l2 = 0; l2 < kSlOpWords; l2 += 4) std::copy_n(padw, 4, w + l2);
-      }
-      page_reach.assign(packer.npages, 0);
-      for (size_t i = 0; i < parts.size(); ++i) {
-        const Part &q = parts[i];
-        const int pgi = packer.at[i].first, l0 = packer.at[i].second;
-        auto &O = opg[rank[pgi % kSlWarps]];
-        uint32_t *e = O.data() + (size_t)page_of[pgi] * kSlOpWords;
-        const int off = base[part_of(q.seg)];
-        int t = q.first;
-        const int end = q.first + q.len;
-        for (int r = 0; r < q.lanes; ++r) {
-          const Op &o0 = lev[t + off];
-          const bool two = t % kSlOpRun == 0 && t + 1 < end;
-          const Op o1 = two ? lev[t + 1 + off] : none(o0.k);
-          t += two ? 2 : 1;
-          const bool last = r == q.lanes - 1;
-          const bool prev = last && !q.scan_last && r > 0;
-          if (!prev) page_reach[pgi] = std::max(page_reach[pgi], r);
-          const int to = !last ? zero : (q.more ? zero + 1 + q.carry_out : target[q.seg]);
-          const int ini = r == 0 && q.carry_in >= 0 ? 1 + q.carry_in : 0;
-          encode(e + 4 * (l0 + r), o0, o1, (uint32_t)to, (uint32_t)ini,
-                 prev ? 32u : (uint32_t)r);
+        uint32_t *e = O.data() + page_of[i];
+        const Packer::Page &pg = packer.pages[i];
+        for (int l2 = pg.used; l2 < 32; ++l2) {
+          std::copy_n(padw, 4, e + 4 * l2);
+          e[4 * l2 + 3] |= (uint32_t)pg.steps << 22;
         }
       }
-      for (int i = 0; i < packer.npages; ++i) {
-        const uint32_t steps = (uint32_t)scan_steps(page_reach[i]) << 22;
-        uint32_t *w = opg[rank[i % kSlWarps]].data() + (size_t)page_of[i] * kSlOpWords;
-        for (int l2 = 0; steps && l2 < 32; ++l2) w[4 * l2 + 3] |= steps;
+      for (int i : packer.order) {
+        const Part &q = parts[i];
+        const int pgi = packer.at[i].first, l0 = packer.at[i].second;
+        uint32_t *e = opg[rank[pgi % kSlWarps]].data() + page_of[pgi] + 4 * l0;
+        const uint32_t steps = (uint32_t)packer.pages[pgi].steps << 6;
+        const bool prev = adds_previous(q);
+        const uint32_t to = (uint32_t)(q.carry_out >= 0 ? zero + 1 + q.carry_out : q.to);
+        const Op *o = lev + q.src;
+        int t = q.first;
+        const int end = q.first + q.len;
+        for (int r = 0; r < q.lanes; ++r, e += 4) {
+          const bool two = t % kSlOpRun == 0 && t + 1 < end, last = r == q.lanes - 1;
+          Op o1 = o[two ? 1 : 0];
+          if (!two) o1.a = o1.b = (uint16_t)zero;
+          encode(e, o[0], o1, last ? to : (uint32_t)zero,
+                 r == 0 && q.carry_in >= 0 ? 1u + (uint32_t)q.carry_in : 0u,
+                 steps | (last && prev ? 32u : (uint32_t)r));
+          t += two ? 2 : 1;
+          o += two ? 2 : 1;
+        }
       }
       // the phase's end (the last one is the level's)
       ++s.olevels;
       for (int w = 0; w < kSlWarps; ++w) {
-        if (opg[w].empty()) {
+        if (opg[w].empty())
           ++oskip[w];
-          continue;
-        }
-        uint32_t *e = opg[w].data() + opg[w].size() - kSlOpWords;
-        if ((e[3] >> 25) == (uint32_t)kSlOpMaxWait) return false;
-        for (int l2 = 0; l2 < 32; ++l2) e[4 * l2 + 3] += 1u << 25;
+        else if (++ends[w] > kSlOpMaxWait)
+          return false;
       }
     }
   }
   s.ops.clear();
+  size_t nop_words = 0;
+  for (const auto &o : opg) nop_words += o.size();
+  s.ops.reserve(nop_words);
   for (int w = 0; w < kSlWarps; ++w) {
+    settle(w);
     s.op.first[w] = (int)(s.ops.size() / kSlOpWords);
     s.op.count[w] = (int)(opg[w].size() / kSlOpWords);
     s.op.skip[w] = oskip[w];
