@@ -1244,10 +1244,8 @@ extern "C" int clgpu_debug_check_instance(const clgpu_problem *pb, const clgpu_s
               done.insert({t.x, t.y});
             }
           }
-          if ((L.kind == SN_ASSEMBLE || L.kind == SN_FWD_GATHER) &&
-              (t.y < 0 || t.z > ld || t.y >= t.z))
-            return -41;
-          if (L.kind == SN_ASSEMBLE || L.kind == SN_FWD_GATHER) {
+          if (L.kind == SN_ASSEMBLE && (t.y < 0 || t.z > ld || t.y >= t.z)) return -41;
+          if (L.kind == SN_ASSEMBLE) {
             // the chunk's children: entries q of each map inside [t.y, t.z)
             if (t.w < plan.chunk_off[t.x] || t.w >= plan.chunk_off[t.x + 1] ||
                 (t.w - plan.chunk_off[t.x]) * kSnAsmCols != t.y)

@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_sn_small(SnDev d, KKTDev k, L
 // Assembly of columns [ca, cb) of a blocked front: zero (rows c..ld), the
 // original entries (+ static regularisation), unit dummy pivots, then the
 // Schur complements of the children that touch these columns, in child
-// order (the plan lists them per 32-column chunk with their entry ranges).
+// order (the plan lists them per 8-column chunk with their entry ranges).
 template <typename T>
 __global__ void __launch_bounds__(kAsmThreads) k_sn_assemble(SnDev d, KKTDev k, int base,
                                                             const int *run) {
@@ -802,7 +802,7 @@ __global__ void __launch_bounds__(256) k_sn_bwd_small(SnDev d, int base, int cou
 // value is written, so it travels in one store and one polled load; each
 // direction empties the other's vector.  (Two launches per panel and direction,
 // each staging its block after the launch: 24 us a panel.  A pass over 2 000
-// second-order cones' 22 panels in 7 levels: 1.5 ms before, 0.50 ms now.)
+// second-order cones' 22 panels in 7 levels: 1.5 ms before, 0.33 ms now.)
 // Every sum is in an order that does not depend on the split: the children in
 // order; per panel four interleaved column sums forward; per tile and column a
 // balanced tree over the rows, and four interleaved sums over the tiles in

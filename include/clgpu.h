@@ -440,11 +440,6 @@ int clgpu_cones_debug_scaling(const clgpu_cones *h, double *soc_w, double *soc_l
                               double *soc_u, double *soc_v, double *soc_eta, double *soc_d,
                               double *psd_R, double *psd_Rinv, double *psd_lambda,
                               int *psd_nmax);
-/* Host-only replay of the device factorisation on the structures prepared
- * for one instance: validates the ordering, the symbolic factorisation and
- * every index map, then factors a quasi-definite test matrix on the KKT
- * pattern and returns the solve residual.  No reference counterpart
- * (diagnostic); needs no GPU. */
 /* Host-only view of the SOC tiling (diagnostic, no reference counterpart):
  * for n second-order cones with first rows off[k] and dimensions dim[k],
  * writes the tiles the kernels would use for tiles of at most max_cones
@@ -453,6 +448,11 @@ int clgpu_cones_debug_scaling(const clgpu_cones *h, double *soc_w, double *soc_l
  * little room.  Needs no GPU. */
 int clgpu_debug_soc_tiles(const int *off, const int *dim, int n, int max_cones,
                           int max_rows, int *tiles, int cap);
+/* Host-only replay of the device factorisation on the structures prepared
+ * for one instance: validates the ordering, the symbolic factorisation and
+ * every index map, then factors a quasi-definite test matrix on the KKT
+ * pattern and returns the solve residual.  No reference counterpart
+ * (diagnostic); needs no GPU. */
 int clgpu_debug_check_instance(const clgpu_problem *prob,
                                const clgpu_settings *settings, double *resid);
 /* Host-only view of the factorisation path setup picks for one instance
