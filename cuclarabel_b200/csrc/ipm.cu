@@ -2562,8 +2562,10 @@ static int ipm_pass(clgpu_solver *h, Phase &P, cudaStream_t st, double elapsed, 
     if (!ex) {
       cudaGraph_t g = nullptr;
       const long long l0 = h->launches;
-      if (!h->st_cap &&
-          cudaStreamCreateWithFlags(&h->st_cap, cudaStreamNonBlocking) != cudaSuccess)
+      int priority = 0;  // the graph's kernels keep the priority they are captured with
+      cudaStreamGetPriority(st, &priority);
+      if (!h->st_cap && cudaStreamCreateWithPriority(&h->st_cap, cudaStreamNonBlocking,
+                                                     priority) != cudaSuccess)
         h->st_cap = nullptr;
       Phase C{h, h->st_cap, P.dp, P.cp};
       if (h->st_cap &&
