@@ -2000,6 +2000,7 @@ extern "C" int clgpu_debug_launch_groups(const clgpu_problem *pbs, int n, const 
   if (st) {
     opt.equilibrate_enable = st->equilibrate_enable;
     if (st->soc_threshold > 0) opt.soc_threshold = st->soc_threshold;
+    opt.fp32_factor = st->direct_solve_method != CLGPU_METHOD_FP64;
   }
   std::vector<SlNeed> need(n);
   std::vector<int> items;
@@ -2051,6 +2052,7 @@ extern "C" int clgpu_debug_factor_stream(const clgpu_problem *pb, const clgpu_se
   if (st) {
     opt.soc_threshold = st->soc_threshold;
     opt.equilibrate_enable = st->equilibrate_enable;
+    opt.fp32_factor = st->direct_solve_method != CLGPU_METHOD_FP64;
     opt.equilibrate_max_iter = st->equilibrate_max_iter;
   }
   Prepared p;
@@ -2257,6 +2259,7 @@ extern "C" int clgpu_solver_create(const clgpu_problem *probs, int nprob,
   SetupOptions opt;
   opt.soc_threshold = h->st.soc_threshold;
   opt.equilibrate_enable = h->st.equilibrate_enable;
+  opt.fp32_factor = h->mixed;
   opt.equilibrate_max_iter = h->st.equilibrate_max_iter;
   opt.equilibrate_min_scaling = h->st.equilibrate_min_scaling;
   opt.equilibrate_max_scaling = h->st.equilibrate_max_scaling;

@@ -87,6 +87,7 @@ struct SetupOptions {
   // leave the Ruiz equilibration (and so the KKT values) to the device when
   // the caller's P and A columns are sorted without repeated entries
   bool defer_equilibration = false;
+  bool fp32_factor = false;  // the factor is stored, or computed, in FP32
 };
 
 bool prepare_instance(const clgpu_problem &pb, const SetupOptions &opt,

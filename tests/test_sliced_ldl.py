@@ -119,9 +119,9 @@ def test_large_solves_match_the_oracle(cuda_device, name):
     assert all(np.array_equal(one.x, t.x) and np.array_equal(one.z, t.z) for t in two)
 
 
-def _entries(pb):
+def _entries(pb, method="cudss"):
     cp, keep, n, m = _prep_problem(*pb)
-    st = Settings().to_c()
+    st = Settings(direct_solve_method=method).to_c()
     sn, ent = ctypes.c_int(), ctypes.c_longlong()
     assert _lib.load().clgpu_debug_instance_path(ctypes.byref(cp), ctypes.byref(st),
                                                  ctypes.byref(sn), ctypes.byref(ent)) == 0
@@ -165,3 +165,12 @@ def test_launch_groups_of_needs_around_a_threshold(method):
     rc = _lib.load().clgpu_debug_launch_groups(arr, len(base), ctypes.byref(st), counts)
     assert rc == 0 and counts[2] == len(base)
     assert 1 <= counts[0] <= 3 and 1 <= counts[1] <= 3, list(counts)
+
+
+@pytest.mark.parametrize("method", ["cudssmixed", "mixed_f64elim"])
+def test_fp32_factors_keep_dissection_unless_it_is_five_times_denser(method):
+    """Minimum degree takes pivots that cost an FP32 factor digits: it stays for
+    budgets over all assets, not for a few coupled semidefinite blocks."""
+    dense, mild = problems.portfolio(3, 50, 5), problems.psd_lp(8, 3, seed=2)
+    assert _entries(dense, method) == _entries(dense)
+    assert _entries(mild, method)[1] > 1.5 * _entries(mild)[1]
